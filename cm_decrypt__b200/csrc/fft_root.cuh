@@ -53,6 +53,18 @@ template <int S> struct FftDims {
 // through this map.
 __device__ __forceinline__ int fa_word(int w) { return w ^ ((0 - ((w >> 5) & 1)) & 31); }
 
+// Where depth d's twiddle words start: its 2^(m-d-6) words, plane after plane,
+// follow those of the depths before it.  Plane-major, so that a warp's lanes
+// read one plane of consecutive words: one 128-byte line a load.  (A word's
+// planes side by side put the 32 lanes of a load 64 bytes apart, 16 lines a
+// load, 3.3 k line accesses a ciphertext against 0.4 k: 65,536 mceliece6960119
+// ciphertexts took 3.45 ms that way and take 3.14 ms so, 2^20 of 348864 18.6
+// and 16.5 ms.)
+template <int M> __host__ __device__ constexpr int tw_offset(int d)
+{
+    return M * ((1 << (M - 5)) - (1 << (M - 5 - d)));
+}
+
 // Radix conversion of the bitsliced array cv[x * CVS + k] (x < 2^D, k < M),
 // by NT cooperating threads (tid in [0, NT)); `sync` orders the steps.
 template <int S, int CVS, int NT, class Sync>
@@ -232,123 +244,15 @@ __device__ __forceinline__ void store_row_packed(uint8_t *p, const uint32_t *v, 
     }
 }
 
-// One warp: error row (and weight) of locator q from the converted array cv
-// (bitsliced, cv[s * CVS + k]).  fa: this warp's FA_WORDS words of shared
-// memory.  erow: NW words, or null.  epack: null, or the row's n/8 bytes
-// packed (store_row_packed).  prow: null, or t+1 u16 that receive the
-// weight, the flagged positions in ascending order and 0xFFFF in the unused
-// slots (the weight never exceeds t: the reversed locator's leading
-// coefficient is C[0], which the update never zeroes).  Returns the weight
-// (all lanes).
-template <int S, int CVS>
-__device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t *fa, const uint32_t *__restrict__ tw,
-                                            const uint32_t *__restrict__ bctl, uint32_t *erow, uint16_t *prow,
-                                            int lane, uint8_t *epack = nullptr)
+// One warp: the outputs of one ciphertext from its flags in support order
+// (z[j] = word lane + 32j): erow, epack and prow as for fft_root_one below.
+// Returns the weight (all lanes).
+template <int S>
+__device__ __forceinline__ int root_output(const uint32_t *z, uint32_t *erow, uint16_t *prow, uint8_t *epack, int lane)
 {
     using F = FftDims<S>;
-    constexpr int M = F::M, D = F::D, NWD = F::NWD, R = F::R, NW = F::NW;
+    constexpr int R = F::R, NW = F::NW;
     constexpr uint32_t FULL = 0xFFFFFFFFu;
-    // Depth D-1: both operands are depth-D constants, read straight from cv.
-    {
-        constexpr int sbit = M - D - 5, Sw = 1 << sbit;
-        const uint32_t *twd = tw + (size_t)((1 << (M - 5)) - (1 << (M - 5 - (D - 1)))) * 16;
-#pragma unroll 1
-        for (int j = 0; j < R / 2; j++) {
-            const int P2 = lane + 32 * j;
-            const int wa = ((P2 >> sbit) << (sbit + 1)) | (P2 & (Sw - 1));
-            const int sa = (int)(__brev((uint32_t)(wa >> sbit)) >> (32 - D));
-            const int sb = (int)(__brev((uint32_t)((wa + Sw) >> sbit)) >> (32 - D));
-            const uint32_t *g = twd + (P2 & (Sw - 1)) * 16;
-            uint32_t B[M], G[M], p[2 * M - 1];
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                B[k] = 0u - ((cv[sb * CVS + k] >> q) & 1u);
-                G[k] = __ldg(g + k);
-            }
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-            bs_mul_acc<M>(p, G, B);
-            bs_reduce<M>(p);
-            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const uint32_t na = (0u - ((cv[sa * CVS + k] >> q) & 1u)) ^ p[k];
-                fa[k * NWD + pa] = na;
-                fa[k * NWD + pb] = na ^ B[k];
-            }
-        }
-        __syncwarp();
-    }
-#pragma unroll
-    for (int d = D - 2; d >= 1; d--) {
-        const int sbit = M - d - 6, Sw = 1 << sbit;
-        const uint32_t *twd = tw + (size_t)((1 << (M - 5)) - (1 << (M - 5 - d))) * 16;
-#pragma unroll 1
-        for (int j = 0; j < R / 2; j++) {
-            const int P2 = lane + 32 * j;
-            const int wa = ((P2 >> sbit) << (sbit + 1)) | (P2 & (Sw - 1));
-            const uint32_t *g = twd + (P2 & (Sw - 1)) * 16;
-            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
-            uint32_t A[M], B[M], G[M], p[2 * M - 1];
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                A[k] = fa[k * NWD + pa];
-                B[k] = fa[k * NWD + pb];
-                G[k] = __ldg(g + k);
-            }
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-            bs_mul_acc<M>(p, G, B);
-            bs_reduce<M>(p);
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const uint32_t na = A[k] ^ p[k];
-                fa[k * NWD + pa] = na;
-                fa[k * NWD + pb] = na ^ B[k];
-            }
-        }
-        __syncwarp();
-    }
-    // Depth 0 pairs word w = lane + 32j with w + 2^(m-6): exactly the words
-    // z[j] and z[j + R/2] of this lane, so the zero flags come straight from
-    // the butterfly (no store of the evaluations).
-    uint32_t z[R];
-    {
-        constexpr int Sw = 1 << (M - 6);
-#pragma unroll
-        for (int j = 0; j < R / 2; j++) {
-            const int wa = lane + 32 * j;
-            const uint32_t *g = tw + (size_t)wa * 16;  // depth 0: offset 0
-            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
-            uint32_t A[M], B[M], G[M], p[2 * M - 1];
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                A[k] = fa[k * NWD + pa];
-                B[k] = fa[k * NWD + pb];
-                G[k] = __ldg(g + k);
-            }
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-            bs_mul_acc<M>(p, G, B);
-            bs_reduce<M>(p);
-            uint32_t anya = 0, anyb = 0;
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const uint32_t na = A[k] ^ p[k];
-                anya |= na;
-                anyb |= na ^ B[k];
-            }
-            z[j] = ~anya;
-            z[j + R / 2] = ~anyb;
-        }
-    }
-    __syncwarp();  // fa may be refilled right after this call
-#pragma unroll
-    for (int l = 0; l < 2 * M - 1; l++)
-        swap_layer<S>(z, bctl, l, lane);
     uint32_t v[R];
     int cnt = 0;
 #pragma unroll
@@ -398,6 +302,125 @@ __device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t 
             prow[0] = (uint16_t)cnt;
     }
     return cnt;
+}
+
+// One warp: error row (and weight) of locator q from the converted array cv
+// (bitsliced, cv[s * CVS + k]).  fa: this warp's FA_WORDS words of shared
+// memory.  erow: NW words, or null.  epack: null, or the row's n/8 bytes
+// packed (store_row_packed).  prow: null, or t+1 u16 that receive the
+// weight, the flagged positions in ascending order and 0xFFFF in the unused
+// slots (the weight never exceeds t: the reversed locator's leading
+// coefficient is C[0], which the update never zeroes).  Returns the weight
+// (all lanes).
+template <int S, int CVS>
+__device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t *fa, const uint32_t *__restrict__ tw,
+                                            const uint32_t *__restrict__ bctl, uint32_t *erow, uint16_t *prow,
+                                            int lane, uint8_t *epack = nullptr)
+{
+    using F = FftDims<S>;
+    constexpr int M = F::M, D = F::D, NWD = F::NWD, R = F::R;
+    // Depth D-1: both operands are depth-D constants, read straight from cv.
+    {
+        constexpr int sbit = M - D - 5, Sw = 1 << sbit;
+        const uint32_t *twd = tw + tw_offset<M>(D - 1);
+#pragma unroll 1
+        for (int j = 0; j < R / 2; j++) {
+            const int P2 = lane + 32 * j;
+            const int wa = ((P2 >> sbit) << (sbit + 1)) | (P2 & (Sw - 1));
+            const int sa = (int)(__brev((uint32_t)(wa >> sbit)) >> (32 - D));
+            const int sb = (int)(__brev((uint32_t)((wa + Sw) >> sbit)) >> (32 - D));
+            const uint32_t *g = twd + (P2 & (Sw - 1));
+            uint32_t B[M], G[M], p[2 * M - 1];
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                B[k] = 0u - ((cv[sb * CVS + k] >> q) & 1u);
+                G[k] = __ldg(g + k * Sw);
+            }
+#pragma unroll
+            for (int k = 0; k < 2 * M - 1; k++)
+                p[k] = 0;
+            bs_mul_acc<M>(p, G, B);
+            bs_reduce<M>(p);
+            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                const uint32_t na = (0u - ((cv[sa * CVS + k] >> q) & 1u)) ^ p[k];
+                fa[k * NWD + pa] = na;
+                fa[k * NWD + pb] = na ^ B[k];
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int d = D - 2; d >= 1; d--) {
+        const int sbit = M - d - 6, Sw = 1 << sbit;
+        const uint32_t *twd = tw + tw_offset<M>(d);
+#pragma unroll 1
+        for (int j = 0; j < R / 2; j++) {
+            const int P2 = lane + 32 * j;
+            const int wa = ((P2 >> sbit) << (sbit + 1)) | (P2 & (Sw - 1));
+            const uint32_t *g = twd + (P2 & (Sw - 1));
+            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
+            uint32_t A[M], B[M], G[M], p[2 * M - 1];
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                A[k] = fa[k * NWD + pa];
+                B[k] = fa[k * NWD + pb];
+                G[k] = __ldg(g + k * Sw);
+            }
+#pragma unroll
+            for (int k = 0; k < 2 * M - 1; k++)
+                p[k] = 0;
+            bs_mul_acc<M>(p, G, B);
+            bs_reduce<M>(p);
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                const uint32_t na = A[k] ^ p[k];
+                fa[k * NWD + pa] = na;
+                fa[k * NWD + pb] = na ^ B[k];
+            }
+        }
+        __syncwarp();
+    }
+    // Depth 0 pairs word w = lane + 32j with w + 2^(m-6): exactly the words
+    // z[j] and z[j + R/2] of this lane, so the zero flags come straight from
+    // the butterfly (no store of the evaluations).
+    uint32_t z[R];
+    {
+        constexpr int Sw = 1 << (M - 6);
+#pragma unroll
+        for (int j = 0; j < R / 2; j++) {
+            const int wa = lane + 32 * j;
+            const uint32_t *g = tw + wa;  // depth 0: offset 0
+            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
+            uint32_t A[M], B[M], G[M], p[2 * M - 1];
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                A[k] = fa[k * NWD + pa];
+                B[k] = fa[k * NWD + pb];
+                G[k] = __ldg(g + k * Sw);
+            }
+#pragma unroll
+            for (int k = 0; k < 2 * M - 1; k++)
+                p[k] = 0;
+            bs_mul_acc<M>(p, G, B);
+            bs_reduce<M>(p);
+            uint32_t anya = 0, anyb = 0;
+#pragma unroll
+            for (int k = 0; k < M; k++) {
+                const uint32_t na = A[k] ^ p[k];
+                anya |= na;
+                anyb |= na ^ B[k];
+            }
+            z[j] = ~anya;
+            z[j + R / 2] = ~anyb;
+        }
+    }
+    __syncwarp();  // fa may be refilled right after this call
+#pragma unroll
+    for (int l = 0; l < 2 * M - 1; l++)
+        swap_layer<S>(z, bctl, l, lane);
+    return root_output<S>(z, erow, prow, epack, lane);
 }
 
 }  // namespace cmd

@@ -107,13 +107,13 @@ __device__ __forceinline__ void tsynd_one(const LatItem &it, const uint8_t *__re
 #pragma unroll
     for (int j = 0; j < R / 2; j++) {
         const int wa = lane + 32 * j, wb = wa + NWD / 2;
-        const uint32_t *g = tw + (size_t)wa * 16;
+        const uint32_t *g = tw + wa;
         uint32_t A[M], B[M], G[M], p[2 * M - 1];
 #pragma unroll
         for (int k = 0; k < M; k++) {
             B[k] = z[j + R / 2] & __ldg(wf + k * NWD + wb);
             A[k] = (z[j] & __ldg(wf + k * NWD + wa)) ^ B[k];
-            G[k] = __ldg(g + k);
+            G[k] = __ldg(g + k * (NWD / 2));
         }
 #pragma unroll
         for (int k = 0; k < 2 * M - 1; k++)
@@ -132,19 +132,19 @@ __device__ __forceinline__ void tsynd_one(const LatItem &it, const uint8_t *__re
 #pragma unroll 1
     for (int d = 1; d < DS - 1; d++) {
         const int sbit = M - d - 6, Sw = 1 << sbit;
-        const uint32_t *twd = tw + (size_t)(NWD - (NWD >> d)) * 16;
+        const uint32_t *twd = tw + tw_offset<M>(d);
 #pragma unroll 1
         for (int j = 0; j < R / 2; j++) {
             const int P2 = lane + 32 * j;
             const int wa = ((P2 >> sbit) << (sbit + 1)) | (P2 & (Sw - 1));
-            const uint32_t *g = twd + (P2 & (Sw - 1)) * 16;
+            const uint32_t *g = twd + (P2 & (Sw - 1));
             const int pa = fa_word(wa), pb = fa_word(wa + Sw);
             uint32_t A[M], B[M], G[M], p[2 * M - 1];
 #pragma unroll
             for (int k = 0; k < M; k++) {
                 B[k] = fa[k * NWD + pb];
                 A[k] = fa[k * NWD + pa] ^ B[k];
-                G[k] = __ldg(g + k);
+                G[k] = __ldg(g + k * Sw);
             }
 #pragma unroll
             for (int k = 0; k < 2 * M - 1; k++)
@@ -163,7 +163,7 @@ __device__ __forceinline__ void tsynd_one(const LatItem &it, const uint8_t *__re
     //       a group: its parity per plane goes out as the sum of sub-problem
     //       bitrev_D'(word)
     {
-        const uint32_t *g = tw + (size_t)(NWD - (NWD >> (DS - 1))) * 16;
+        const uint32_t *g = tw + tw_offset<M>(DS - 1);  // one word per plane
         uint32_t G[M];
 #pragma unroll
         for (int k = 0; k < M; k++)
