@@ -13,7 +13,7 @@
 
 namespace cmd {
 static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-                    uint16_t *d_weight, uint16_t *d_synd, cudaStream_t s);
+                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s);
 
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
@@ -362,7 +362,7 @@ int cmd_stage_synd_fft(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts
         return CMD_OK;
     cudaSetDevice(eng->device);
     std::lock_guard<std::mutex> lk(eng->mu);
-    return run_tile(eng, key, d_cts, count, nullptr, nullptr, d_synd, stream ? (cudaStream_t)stream : eng->stream);
+    return run_tile(eng, key, d_cts, count, nullptr, nullptr, nullptr, d_synd, stream ? (cudaStream_t)stream : eng->stream);
 }
 
 int cmd_stage_bm(cmd_engine *eng, cmd_set set, const uint16_t *d_synd, size_t count, uint16_t *d_loc, void *stream)
@@ -441,11 +441,13 @@ static int run_plain(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, 
 // word offsets fit the tile items' 32-bit fields.  With d_synd: syndromes
 // only.  Caller holds eng->mu.
 static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-                    uint16_t *d_weight, uint16_t *d_synd, cudaStream_t s)
+                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s)
 {
     const SetInfo si = set_info(key->dev.set);
     const size_t chunk = std::min<size_t>(count, (size_t)1 << 22);
-    int rc = eng->scratch.reserve(eng, tile_single_scratch_words(chunk) * 4);
+    int rc = CMD_OK;
+    if (d_synd || count > CT_ONE_LAUNCH)  // smaller batches keep everything on chip
+        rc = eng->scratch.reserve(eng, tile_single_scratch_words(chunk) * 4);
     if (rc)
         return rc;
     FftPlans plans;
@@ -455,8 +457,8 @@ static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
         const size_t n = std::min(chunk, count - c0);
         const cudaError_t e = launch_tile_single(
             key->dev, d_cts + c0 * si.ct, n, static_cast<uint32_t *>(eng->scratch.ptr),
-            d_err ? d_err + c0 * si.nw : nullptr, d_weight ? d_weight + c0 : nullptr,
-            d_synd ? d_synd + c0 * 2 * si.t : nullptr, plans, s, LaunchCounter{&eng->launches});
+            d_err ? d_err + c0 * si.nw : nullptr, d_weight ? d_weight + c0 : nullptr, d_pos,
+            d_synd ? d_synd + c0 * 2 * si.t : nullptr, plans, eng->num_sms, s, LaunchCounter{&eng->launches});
         if (e != cudaSuccess)
             return cuda_fail(e, "tile path launch");
     }
@@ -471,7 +473,7 @@ int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t
     if (path == CMD_PATH_PLAIN)
         return run_plain(eng, key, d_cts, count, d_err, d_weight, s);
     if (path == CMD_PATH_TILE || (path == CMD_PATH_AUTO && count < eng->fcfg[key->dev.set].tile_below))
-        return run_tile(eng, key, d_cts, count, d_err, d_weight, nullptr, s);
+        return run_tile(eng, key, d_cts, count, d_err, d_weight, nullptr, nullptr, s);
     return run_fused_single(eng, key, d_cts, count, d_err, d_weight, s);
 }
 

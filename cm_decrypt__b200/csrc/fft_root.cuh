@@ -160,23 +160,40 @@ __device__ __forceinline__ void fft_convert_t(uint32_t *cv, const uint16_t *__re
     }
 }
 
-// Layer l of the key's support network over a 2^m-bit array held by one
-// warp (word w = lane + 32j in z[j]): every pair (p, p + 2^e) whose mask bit
-// (the lower element's) is set exchanges its two bits; e = l for l < m, else
-// 2m-2-l.  A layer is its own inverse.
-template <int S>
-__device__ __forceinline__ void swap_layer(uint32_t *z, const uint32_t *__restrict__ bctl, int l, int lane)
+// Barrier of the WPC warps that share one ciphertext: the warp's own, or named
+// barrier 1 + g of group g of the block.
+template <int WPC> __device__ __forceinline__ void group_sync()
+{
+    if constexpr (WPC == 1)
+        __syncwarp();
+    else if constexpr (WPC == 4)  // the block's only group
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / (32 * WPC)), "n"(32 * WPC) : "memory");
+}
+
+// Layer l of the key's support network over a 2^m-bit array held by WPC warps
+// (thread tid < 32 WPC holds word w = tid + 32 WPC j in z[j]): every pair (p,
+// p + 2^e) whose mask bit (the lower element's) is set exchanges its two
+// bits; e = l for l < m, else 2m-2-l.  A layer is its own inverse.  Pairs
+// lie inside a word, across a warp's lanes, across the group's warps (through
+// xb, 2 x 2^(m-5) words of shared memory whose halves alternate with `half`,
+// so one barrier an exchange is enough) or inside a thread.
+template <int S, int WPC = 1>
+__device__ __forceinline__ void swap_layer(uint32_t *z, const uint32_t *__restrict__ bctl, int l, int tid,
+                                           uint32_t *xb = nullptr, int *half = nullptr)
 {
     using F = FftDims<S>;
-    constexpr int M = F::M, NWD = F::NWD, R = F::R;
+    constexpr int M = F::M, NWD = F::NWD, NT = 32 * WPC, R = NWD / NT;
     constexpr uint32_t FULL = 0xFFFFFFFFu;
+    static_assert(R >= 1, "a word per thread");
     const int e = l < M ? l : 2 * M - 2 - l;
     const uint32_t *ml = bctl + l * NWD;
     if (e < 5) {  // pairs inside a word
         const int sh = 1 << e;
 #pragma unroll
         for (int j = 0; j < R; j++) {
-            const uint32_t mk = __ldg(ml + lane + 32 * j);
+            const uint32_t mk = __ldg(ml + tid + NT * j);
             const uint32_t t = ((z[j] >> sh) ^ z[j]) & mk;
             z[j] ^= t ^ (t << sh);
         }
@@ -185,15 +202,29 @@ __device__ __forceinline__ void swap_layer(uint32_t *z, const uint32_t *__restri
 #pragma unroll
         for (int j = 0; j < R; j++) {
             const uint32_t other = __shfl_xor_sync(FULL, z[j], ls);
-            const uint32_t mk = __ldg(ml + ((lane & ~ls) + 32 * j));
+            const uint32_t mk = __ldg(ml + ((tid & ~ls) + NT * j));
             z[j] ^= (z[j] ^ other) & mk;
         }
-    } else {  // pairs inside a lane
-        const int js = 1 << (e - 10);
+    } else if (1 << (e - 5) < NT) {  // pairs across warps
+        const int ws = 1 << (e - 5);
+        uint32_t *x = xb + *half * NWD;
+        *half ^= 1;
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            x[tid + NT * j] = z[j];
+        group_sync<WPC>();
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const uint32_t other = x[(tid ^ ws) + NT * j];
+            const uint32_t mk = __ldg(ml + ((tid & ~ws) + NT * j));
+            z[j] ^= (z[j] ^ other) & mk;
+        }
+    } else {  // pairs inside a thread
+        const int js = (1 << (e - 5)) / NT;
 #pragma unroll
         for (int j = 0; j < R; j++) {
             if (!(j & js)) {
-                const uint32_t mk = __ldg(ml + lane + 32 * j);
+                const uint32_t mk = __ldg(ml + tid + NT * j);
                 const uint32_t t = (z[j] ^ z[j | js]) & mk;
                 z[j] ^= t;
                 z[j | js] ^= t;

@@ -138,16 +138,31 @@ constexpr int TILE_SCRATCH_WORDS = TILE_LOC_WORDS + TILE_SUM_WORDS;
 struct FftPlans {
     FftPlanDev p[NSETS];
 };
-cudaError_t launch_tile_path(const void *d_items, const uint8_t *d_cts, uint32_t ntiles, uint32_t *d_scratch,
-                             uint32_t *d_err, uint16_t *d_weight, const FftPlans &plans, cudaStream_t s,
-                             LaunchCounter lc);
+// live: ciphertexts among the slots; small batches take the per-ciphertext
+// kernels below.
+cudaError_t launch_tile_path(const void *d_items, const uint8_t *d_cts, uint32_t ntiles, uint32_t live,
+                             uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight, const FftPlans &plans,
+                             int num_sms, cudaStream_t s, LaunchCounter lc);
 // The tile path over one key's batch (ciphertexts at the set's ct stride,
 // error rows at its nw stride); with d_synd, only the syndromes (rows of 2t
-// u16).  d_scratch: tile_single_scratch_words(count) words.
+// u16).  d_scratch: tile_single_scratch_words(count) words.  d_pos (positions
+// rows): only for batches of up to CT_PER_SM an SM.
 cudaError_t launch_tile_single(const KeyDev &k, const uint8_t *d_cts, size_t count, uint32_t *d_scratch,
-                               uint32_t *d_err, uint16_t *d_weight, uint16_t *d_synd, const FftPlans &plans,
-                               cudaStream_t s, LaunchCounter lc);
+                               uint32_t *d_err, uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd,
+                               const FftPlans &plans, int num_sms, cudaStream_t s, LaunchCounter lc);
 size_t tile_single_scratch_words(size_t count);
+// The per-ciphertext kernels (single.cu).  Up to CT_ONE_LAUNCH live
+// ciphertexts run in one launch; more, up to CT_PER_SM an SM, in three with
+// d_mid (256 u16 per slot) between them.  launch_ct_items: nslots items (set
+// -1: skipped), `live` of them in use.  launch_ct_one: count <= CT_ONE_LAUNCH
+// ciphertexts of one key at the set's strides.  d_pos: rows of t+1 u16 by slot
+// (FusedArgs::pos), of one set.
+constexpr uint32_t CT_ONE_LAUNCH = 64, CT_PER_SM = 24;
+cudaError_t launch_ct_items(const LatItem *d_items, const uint8_t *d_cts, uint32_t nslots, uint32_t live,
+                            uint16_t *d_mid, uint32_t *d_err, uint16_t *d_weight, uint16_t *d_pos,
+                            const FftPlans &plans, int num_sms, cudaStream_t s, LaunchCounter lc);
+cudaError_t launch_ct_one(const KeyDev &k, const uint8_t *d_cts, uint32_t count, uint32_t *d_err, uint16_t *d_weight,
+                          uint16_t *d_pos, const FftPlans &plans, cudaStream_t s, LaunchCounter lc);
 
 void set_last_error(const std::string &msg);
 

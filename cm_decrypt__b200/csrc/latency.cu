@@ -580,11 +580,13 @@ cudaError_t tile_prepare(int dev, size_t smem, size_t ts_smem, size_t root_smem)
 
 // The tile path over one key's batch (d_scratch: tile_single_scratch_words).
 cudaError_t launch_tile_single(const KeyDev &k, const uint8_t *d_cts, size_t count, uint32_t *d_scratch,
-                               uint32_t *d_err, uint16_t *d_weight, uint16_t *d_synd, const FftPlans &plans,
-                               cudaStream_t s, LaunchCounter lc)
+                               uint32_t *d_err, uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd,
+                               const FftPlans &plans, int num_sms, cudaStream_t s, LaunchCounter lc)
 {
     if (count == 0)
         return cudaSuccess;
+    if (!d_synd && count <= CT_ONE_LAUNCH)
+        return launch_ct_one(k, d_cts, (uint32_t)count, d_err, d_weight, d_pos, plans, s, lc);
     const SetInfo si = set_info(k.set);
     const uint32_t ntiles = (uint32_t)((count + 31) / 32);
     LatItem *items = reinterpret_cast<LatItem *>(d_scratch);
@@ -607,7 +609,12 @@ cudaError_t launch_tile_single(const KeyDev &k, const uint8_t *d_cts, size_t cou
         lc.bump(2);
         return cudaGetLastError();
     }
-    return launch_tile_path(items, d_cts, ntiles, tiles, d_err, d_weight, plans, s, lc);
+    if (d_pos)
+        return count <= (size_t)CT_PER_SM * num_sms
+                   ? launch_ct_items(items, d_cts, ntiles * 32, (uint32_t)count, reinterpret_cast<uint16_t *>(tiles),
+                                     d_err, d_weight, d_pos, plans, num_sms, s, lc)
+                   : cudaErrorInvalidValue;
+    return launch_tile_path(items, d_cts, ntiles, (uint32_t)count, tiles, d_err, d_weight, plans, num_sms, s, lc);
 }
 
 size_t tile_single_scratch_words(size_t count)
@@ -643,12 +650,15 @@ cudaError_t tile_prepare(int dev, size_t smem, size_t ts_smem, size_t root_smem)
 }
 
 // ntiles tiles of 32 item slots; weights are indexed by item slot.
-cudaError_t launch_tile_path(const void *d_items, const uint8_t *d_cts, uint32_t ntiles, uint32_t *d_scratch,
-                             uint32_t *d_err, uint16_t *d_weight, const FftPlans &plans, cudaStream_t s,
-                             LaunchCounter lc)
+cudaError_t launch_tile_path(const void *d_items, const uint8_t *d_cts, uint32_t ntiles, uint32_t live,
+                             uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight, const FftPlans &plans,
+                             int num_sms, cudaStream_t s, LaunchCounter lc)
 {
     if (ntiles == 0)
         return cudaSuccess;
+    if (live <= CT_PER_SM * (uint32_t)num_sms)
+        return launch_ct_items(static_cast<const LatItem *>(d_items), d_cts, ntiles * 32, live,
+                               reinterpret_cast<uint16_t *>(d_scratch), d_err, d_weight, nullptr, plans, num_sms, s, lc);
     int dev = 0;
     cudaGetDevice(&dev);
     const size_t smem = tile_smem_bytes();

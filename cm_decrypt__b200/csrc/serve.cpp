@@ -521,7 +521,8 @@ int cmd_server::launch(Slot &sl)
         FftPlans plans;
         for (int st = 0; st < NSETS; st++)
             plans.p[st] = eng->fft[st];
-        e = launch_tile_path(sl.d_in + lay.items, sl.d_in + lay.cts, ntiles, sl.d_locbs, sl.d_err, sl.d_w, plans, s, lc);
+        e = launch_tile_path(sl.d_in + lay.items, sl.d_in + lay.cts, ntiles, (uint32_t)B, sl.d_locbs, sl.d_err, sl.d_w,
+                             plans, eng->num_sms, s, lc);
         if (e != cudaSuccess)
             return cuda_fail(e, "server tile-path launch");
     } else {
