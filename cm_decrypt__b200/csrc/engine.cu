@@ -465,15 +465,48 @@ static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
     return CMD_OK;
 }
 
+// Batch size below which CMD_PATH_AUTO (and positions and decapsulation, up to
+// the per-ciphertext kernels' limit) leaves the fused kernel: the tuned
+// crossover, or one that holds for every set on a B200 when the engine has
+// not been tuned.  The fused kernel's time is flat up to about four tiles an
+// SM (one 6960119 ciphertext 779 us, 9,472 1,208 us), the small-batch kernels'
+// is 79 us for one, 501 us for 4,736 and 796 us for 9,472 (348864: 458 us
+// against 47, 249 and 377 us).
+static size_t small_below(const FusedConfig &c)
+{
+    return c.tuned || c.tile_below ? c.tile_below : 8192;
+}
+
+size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count)
+{
+    return count < small_below(eng->fcfg[set]) && count > CT_ONE_LAUNCH ? tile_single_scratch_words(count) * 4 : 0;
+}
+
+// The best kernels for the batch size, error rows and weights or positions.
+// Small batches fall back to the fused kernel, which needs no scratch, when
+// their scratch does not fit the budget.
+static int run_auto(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
+                    uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
+{
+    if (count < small_below(eng->fcfg[key->dev.set]) && (!d_pos || count <= (size_t)CT_PER_SM * eng->num_sms)) {
+        if (eng->scratch.reserve(eng, auto_scratch_bytes(eng, key->dev.set, count)) == CMD_OK)
+            return run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s);
+        cudaGetLastError();
+    }
+    return run_fused_single(eng, key, d_cts, count, d_err, d_weight, s, d_pos);
+}
+
 int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t *d_cts, size_t count,
-               uint32_t *d_err, uint16_t *d_weight, cudaStream_t s)
+               uint32_t *d_err, uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos)
 {
     if (count == 0)
         return CMD_OK;
     if (path == CMD_PATH_PLAIN)
         return run_plain(eng, key, d_cts, count, d_err, d_weight, s);
-    if (path == CMD_PATH_TILE || (path == CMD_PATH_AUTO && count < eng->fcfg[key->dev.set].tile_below))
+    if (path == CMD_PATH_TILE)
         return run_tile(eng, key, d_cts, count, d_err, d_weight, nullptr, nullptr, s);
+    if (path == CMD_PATH_AUTO)
+        return run_auto(eng, key, d_cts, count, d_err, d_weight, d_pos, s);
     return run_fused_single(eng, key, d_cts, count, d_err, d_weight, s);
 }
 
@@ -624,8 +657,8 @@ int cmd_decrypt_positions_device(cmd_engine *eng, const cmd_key *key, const uint
         return CMD_OK;
     cudaSetDevice(eng->device);
     std::lock_guard<std::mutex> lk(eng->mu);
-    return run_fused_single(eng, key, d_cts, count, nullptr, nullptr, stream ? (cudaStream_t)stream : eng->stream,
-                            d_pos);
+    return run_device(eng, key, CMD_PATH_AUTO, d_cts, count, nullptr, nullptr,
+                      stream ? (cudaStream_t)stream : eng->stream, d_pos);
 }
 
 int cmd_decrypt_positions(cmd_engine *eng, const cmd_key *key, const uint8_t *h_cts, size_t count, uint16_t *h_pos)
@@ -695,7 +728,7 @@ int cmd_decrypt_positions(cmd_engine *eng, const cmd_key *key, const uint8_t *h_
         cudaError_t e = cudaMemcpyAsync(d_cts, h_cts + c0 * si.ct, n * si.ct, cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaMemcpyAsync(cts H2D)");
-        if ((rc = run_fused_single(eng, key, d_cts, n, nullptr, nullptr, s, d_pos)))
+        if ((rc = run_device(eng, key, CMD_PATH_AUTO, d_cts, n, nullptr, nullptr, s, d_pos)))
             return rc;
         e = cudaMemcpyAsync(h_pos + c0 * row, d_pos, n * row * 2, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess)

@@ -41,7 +41,8 @@ struct FusedConfig {
                               // the tile kernels (five warps per 32-ciphertext
                               // tile for Berlekamp-Massey, one warp per
                               // ciphertext for the FFTs) instead of the fused
-                              // kernel (one warp per tile); 0 = never
+                              // kernel (one warp per tile); 0 = never when
+                              // tuned (untuned: small_below in engine.cu)
 };
 
 int cuda_fail(cudaError_t e, const char *what);
@@ -57,8 +58,12 @@ bool budget_take(cmd_engine *eng, size_t bytes);
 uint8_t *device_view(uint8_t *h, size_t bytes);
 void budget_give(cmd_engine *eng, size_t bytes);
 
+// d_pos: with CMD_PATH_AUTO only, positions rows instead of error rows.
 int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t *d_cts, size_t count,
-               uint32_t *d_err, uint16_t *d_weight, cudaStream_t s);
+               uint32_t *d_err, uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos = nullptr);
+// The eng->scratch bytes (from its start) CMD_PATH_AUTO would use; 0 for the
+// fused kernel, which it also falls back to when they do not fit.
+size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count);
 int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                      uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos = nullptr);
 // Explicit work counter and round schedule (balanced: -1 = the tuned choice,

@@ -42,3 +42,24 @@ def test_small_batch_shapes_match_plain(engine, s):
                 assert np.array_equal(got_w, want_w[first:first + count]), (count, first)
     finally:
         key.free()
+
+
+@pytest.mark.parametrize("s", [348864, 6960119])
+def test_auto_positions_and_decap_small(engine, s):
+    """Small batches of the calls without a path argument: positions against
+    the fused kernel's rows, decapsulation against the keys of a large batch."""
+    key = cmd.Key(engine, s, golden_sk(s))
+    try:
+        info = key.info
+        valid, _, _ = cmd.PubKey(s, golden_sk(s)).ciphertexts(seed=32, count=9000, malformed_permille=60)
+        cts = np.concatenate([degenerate(info), valid])
+        rows, _ = cmd.decrypt(engine, key, cts, path="fused")
+        large_k, large_a = cmd.kem_decap(engine, key, cts)
+        for count in (1, 64, 65, 3552, 3553, 8191, 8192):
+            assert np.array_equal(cmd.decrypt_positions(engine, key, cts[:count]),
+                                  cmd.positions_from_errors(s, rows[:count])), count
+            assert np.array_equal(cmd.decrypt(engine, key, cts[:count])[0], rows[:count]), count
+            k, a = cmd.kem_decap(engine, key, cts[:count])
+            assert np.array_equal(k, large_k[:count]) and np.array_equal(a, large_a[:count]), count
+    finally:
+        key.free()
