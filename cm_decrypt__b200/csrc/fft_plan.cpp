@@ -26,7 +26,7 @@
 //   * the twiddles: the butterfly of depth d pairs positions Y and
 //     Y + 2^(m-d-1); its multiplier a(Y) depends on r = Y mod 2^(m-d-1):
 //     a = sum_j bit(m-d-2-j of r) * G_{j+2}, stored bitsliced, 32 values r
-//     per word, plane-major (all words of plane 0, then of plane 1, ...).
+//     per word, plane-major (plane 0 of all depths, then plane 1, ...).
 #include <cstring>
 #include <vector>
 
@@ -62,7 +62,7 @@ uint32_t finv(uint32_t a, int m)
 struct FftPlanHost {
     int D = 0;
     std::vector<uint16_t> scalpow;  // [8][256]
-    std::vector<uint32_t> tw;       // per depth: [m][words]
+    std::vector<uint32_t> tw;       // [m][2^(m-5)], a plane's depths one after the other
 };
 
 FftPlanHost make_fft_plan(int set)
@@ -72,6 +72,9 @@ FftPlanHost make_fft_plan(int set)
     FftPlanHost p;
     p.D = synd_depth(si.t);
     p.scalpow.assign(8 * 256, 0);
+    const int plane = 1 << (m - 5);  // at least the sum of all depths' words
+    p.tw.assign((size_t)m * plane, 0);
+    int base = 0;
     std::vector<uint32_t> B(m);
     for (int j = 0; j < m; j++)
         B[j] = 1u << j;
@@ -88,16 +91,15 @@ FftPlanHost make_fft_plan(int set)
             G[i] = fmul(B[i], inv, m);
         const int nbits = m - d - 1;
         const int words = 1 << (nbits - 5);
-        const size_t base = p.tw.size();
-        p.tw.resize(base + (size_t)words * m, 0);
         for (int r = 0; r < (1 << nbits); r++) {
             uint32_t a = 0;
             for (int j = 0; j < nbits; j++)
                 if ((r >> (nbits - 1 - j)) & 1)
                     a ^= G[j + 1];
             for (int k = 0; k < m; k++)
-                p.tw[base + (size_t)k * words + (r >> 5)] |= ((a >> k) & 1u) << (r & 31);
+                p.tw[(size_t)k * plane + base + (r >> 5)] |= ((a >> k) & 1u) << (r & 31);
         }
+        base += words;
         std::vector<uint32_t> nb(B.size() - 1);
         for (size_t i = 1; i < B.size(); i++)
             nb[i - 1] = fmul(G[i], G[i], m) ^ G[i];

@@ -43,26 +43,30 @@ template <int S> struct FftDims {
     static_assert(D <= M - 5, "butterflies must pair whole words");
 };
 
-// Where word w of a plane of the per-warp butterfly array is stored: odd
-// 32-word rows keep their words with the bank bits inverted.  The butterfly
-// levels that pair words less than 32 apart put lanes l and l + 16 in rows 2r
-// and 2r + 1 at the same offsets; with the inversion those offsets fall in
-// disjoint halves of the banks (offsets whose bit log2(distance) is 0 map to
-// ones where it is 1), so no level meets a bank conflict.  Whole-row accesses
+// Where word w of a plane of the per-warp butterfly array is stored: rows of 32
+// words, their bank bits XORed with 11111 in odd rows and with 10101 in rows 2
+// and 3 (mod 4).  A butterfly over one level puts a warp's lanes in two rows at
+// offsets that share bank bit log2(distance), one over two levels in four rows
+// at offsets that share two neighbouring bits: the XORs move the rows to
+// different values of those bits (11111 and 10101 are independent on every two
+// neighbouring bits), so no level meets a bank conflict.  Whole-row accesses
 // stay a permutation of the banks.  Every read and write of the array goes
 // through this map.
-__device__ __forceinline__ int fa_word(int w) { return w ^ ((0 - ((w >> 5) & 1)) & 31); }
+__device__ __forceinline__ int fa_word(int w)
+{
+    return w ^ ((0 - ((w >> 5) & 1)) & 31) ^ ((0 - ((w >> 6) & 1)) & 21);
+}
 
-// Where depth d's twiddle words start: its 2^(m-d-6) words, plane after plane,
-// follow those of the depths before it.  Plane-major, so that a warp's lanes
-// read one plane of consecutive words: one 128-byte line a load.  (A word's
-// planes side by side put the 32 lanes of a load 64 bytes apart, 16 lines a
-// load, 3.3 k line accesses a ciphertext against 0.4 k: 65,536 mceliece6960119
-// ciphertexts took 3.45 ms that way and take 3.14 ms so, 2^20 of 348864 18.6
-// and 16.5 ms.)
+// Twiddle word u of depth d, plane k, is tw[k * 2^(m-5) + tw_offset(d) + u]: a
+// plane holds the 2^(m-d-6) words of depth 0, then of depth 1, ...  A warp's
+// lanes read one plane of consecutive words: one 128-byte line a load, at a
+// constant distance from plane to plane.  (A word's planes side by side put the
+// 32 lanes of a load 64 bytes apart, 16 lines a load, 3.3 k line accesses a
+// ciphertext against 0.4 k: 65,536 mceliece6960119 ciphertexts took 3.45 ms that
+// way and 3.14 ms so, 2^20 of 348864 18.6 and 16.5 ms.)
 template <int M> __host__ __device__ constexpr int tw_offset(int d)
 {
-    return M * ((1 << (M - 5)) - (1 << (M - 5 - d)));
+    return (1 << (M - 5)) - (1 << (M - 5 - d));
 }
 
 // Radix conversion of the bitsliced array cv[x * CVS + k] (x < 2^D, k < M),
@@ -335,6 +339,56 @@ __device__ __forceinline__ int root_output(const uint32_t *z, uint32_t *erow, ui
     return cnt;
 }
 
+// The butterfly: its outputs A + G*B and A + G*B + B, in place.  A starts
+// the accumulators, so adding it costs nothing.
+template <int M> __device__ __forceinline__ void butterfly(uint32_t *A, uint32_t *B, const uint32_t *G)
+{
+    uint32_t p[2 * M - 1];
+#pragma unroll
+    for (int k = 0; k < 2 * M - 1; k++)
+        p[k] = k < M ? A[k] : 0u;
+    bs_mul_acc<M>(p, G, B);
+    bs_reduce<M>(p);
+#pragma unroll
+    for (int k = 0; k < M; k++) {
+        A[k] = p[k];
+        B[k] ^= p[k];
+    }
+}
+
+// Depths d and d-1 of the butterflies on four words of one lane: w[0], w[1],
+// w[2], w[3] at word offsets 0, Sw, 2Sw, 3Sw (Sw = 2^(m-d-6)).  Both pairs of
+// depth d take the same twiddle word u; depth d-1 takes words u and u + Sw.
+template <int M>
+__device__ __forceinline__ void butterfly4(uint32_t (*w)[M], const uint32_t *__restrict__ tw, int d, int u)
+{
+    constexpr int NWD = 1 << (M - 5);
+    const int Sw = 1 << (M - d - 6);
+    const uint32_t *g = tw + tw_offset<M>(d) + u;
+    uint32_t G[M];
+#pragma unroll
+    for (int k = 0; k < M; k++)
+        G[k] = __ldg(g + k * NWD);
+    butterfly<M>(w[0], w[1], G);
+    butterfly<M>(w[2], w[3], G);
+    g = tw + tw_offset<M>(d - 1) + u;
+#pragma unroll
+    for (int k = 0; k < M; k++)
+        G[k] = __ldg(g + k * NWD);
+    butterfly<M>(w[0], w[2], G);
+#pragma unroll
+    for (int k = 0; k < M; k++)
+        G[k] = __ldg(g + k * NWD + Sw);
+    butterfly<M>(w[1], w[3], G);
+}
+
+// Bound by the logic pipe (169 AND-XORs and 37 XORs a butterfly word), so A is
+// folded into the product's accumulators and the constants' bits are spread with
+// one shift.  Two depths a pass halve the array's shared-memory traffic, and the
+// rolled loops keep the code small: the same passes unrolled over the depths
+// took 1,821 us for 37,888 mceliece6960119 ciphertexts, rolled 1,643 us; 65,536
+// of them 3,143 us with one depth a pass and 3,119 us so.
+//
 // One warp: error row (and weight) of locator q from the converted array cv
 // (bitsliced, cv[s * CVS + k]).  fa: this warp's FA_WORDS words of shared
 // memory.  erow: NW words, or null.  epack: null, or the row's n/8 bytes
@@ -350,9 +404,12 @@ __device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t 
 {
     using F = FftDims<S>;
     constexpr int M = F::M, D = F::D, NWD = F::NWD, R = F::R;
-    // Depth D-1: both operands are depth-D constants, read straight from cv.
+    // Depth D-1: both operands are depth-D constants, read straight from cv:
+    // bit q of each plane, shifted to the sign by a multiply (off the logic
+    // pipe) and spread.
     {
         constexpr int sbit = M - D - 5, Sw = 1 << sbit;
+        const uint32_t top = 0x80000000u >> q;
         const uint32_t *twd = tw + tw_offset<M>(D - 1);
 #pragma unroll 1
         for (int j = 0; j < R / 2; j++) {
@@ -361,92 +418,90 @@ __device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t 
             const int sa = (int)(__brev((uint32_t)(wa >> sbit)) >> (32 - D));
             const int sb = (int)(__brev((uint32_t)((wa + Sw) >> sbit)) >> (32 - D));
             const uint32_t *g = twd + (P2 & (Sw - 1));
-            uint32_t B[M], G[M], p[2 * M - 1];
+            uint32_t A[M], B[M], G[M];
 #pragma unroll
             for (int k = 0; k < M; k++) {
-                B[k] = 0u - ((cv[sb * CVS + k] >> q) & 1u);
-                G[k] = __ldg(g + k * Sw);
+                A[k] = (uint32_t)((int32_t)(cv[sa * CVS + k] * top) >> 31);
+                B[k] = (uint32_t)((int32_t)(cv[sb * CVS + k] * top) >> 31);
+                G[k] = __ldg(g + k * NWD);
             }
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-            bs_mul_acc<M>(p, G, B);
-            bs_reduce<M>(p);
+            butterfly<M>(A, B, G);
             const int pa = fa_word(wa), pb = fa_word(wa + Sw);
 #pragma unroll
             for (int k = 0; k < M; k++) {
-                const uint32_t na = (0u - ((cv[sa * CVS + k] >> q) & 1u)) ^ p[k];
-                fa[k * NWD + pa] = na;
-                fa[k * NWD + pb] = na ^ B[k];
+                fa[k * NWD + pa] = A[k];
+                fa[k * NWD + pb] = B[k];
             }
         }
         __syncwarp();
     }
-#pragma unroll
-    for (int d = D - 2; d >= 1; d--) {
+    // The other depths two at a time, so that the array is read and written
+    // half as often.  Depths 1 and 0 (D odd), or depth 0 alone (D even), leave
+    // words lane + 32j in the lane that holds word j of the flags, so they store
+    // those, over plane 0, instead of the evaluations.
+#pragma unroll 1
+    for (int d = D - 2; d >= 1; d -= 2) {
         const int sbit = M - d - 6, Sw = 1 << sbit;
-        const uint32_t *twd = tw + tw_offset<M>(d);
+#pragma unroll 1
+        for (int j = 0; j < R / 4; j++) {
+            const int P4 = lane + 32 * j, u = P4 & (Sw - 1);
+            const int w0 = ((P4 >> sbit) << (sbit + 2)) | u;
+            uint32_t w[4][M];
+            int at[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                at[i] = fa_word(w0 + i * Sw);
+#pragma unroll
+                for (int k = 0; k < M; k++)
+                    w[i][k] = fa[k * NWD + at[i]];
+            }
+            butterfly4<M>(w, tw, d, u);
+            if (d > 1) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int k = 0; k < M; k++)
+                        fa[k * NWD + at[i]] = w[i][k];
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    uint32_t any = 0;
+#pragma unroll
+                    for (int k = 0; k < M; k++)
+                        any |= w[i][k];
+                    fa[at[i]] = ~any;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if constexpr (D % 2 == 0) {
 #pragma unroll 1
         for (int j = 0; j < R / 2; j++) {
-            const int P2 = lane + 32 * j;
-            const int wa = ((P2 >> sbit) << (sbit + 1)) | (P2 & (Sw - 1));
-            const uint32_t *g = twd + (P2 & (Sw - 1));
-            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
-            uint32_t A[M], B[M], G[M], p[2 * M - 1];
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                A[k] = fa[k * NWD + pa];
-                B[k] = fa[k * NWD + pb];
-                G[k] = __ldg(g + k * Sw);
-            }
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-            bs_mul_acc<M>(p, G, B);
-            bs_reduce<M>(p);
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const uint32_t na = A[k] ^ p[k];
-                fa[k * NWD + pa] = na;
-                fa[k * NWD + pb] = na ^ B[k];
-            }
-        }
-        __syncwarp();
-    }
-    // Depth 0 pairs word w = lane + 32j with w + 2^(m-6): exactly the words
-    // z[j] and z[j + R/2] of this lane, so the zero flags come straight from
-    // the butterfly (no store of the evaluations).
-    uint32_t z[R];
-    {
-        constexpr int Sw = 1 << (M - 6);
-#pragma unroll
-        for (int j = 0; j < R / 2; j++) {
             const int wa = lane + 32 * j;
-            const uint32_t *g = tw + wa;  // depth 0: offset 0
-            const int pa = fa_word(wa), pb = fa_word(wa + Sw);
-            uint32_t A[M], B[M], G[M], p[2 * M - 1];
+            const int pa = fa_word(wa), pb = fa_word(wa + NWD / 2);
+            uint32_t A[M], B[M], G[M];
 #pragma unroll
             for (int k = 0; k < M; k++) {
                 A[k] = fa[k * NWD + pa];
                 B[k] = fa[k * NWD + pb];
-                G[k] = __ldg(g + k * Sw);
+                G[k] = __ldg(tw + wa + k * NWD);
             }
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-            bs_mul_acc<M>(p, G, B);
-            bs_reduce<M>(p);
+            butterfly<M>(A, B, G);
             uint32_t anya = 0, anyb = 0;
 #pragma unroll
             for (int k = 0; k < M; k++) {
-                const uint32_t na = A[k] ^ p[k];
-                anya |= na;
-                anyb |= na ^ B[k];
+                anya |= A[k];
+                anyb |= B[k];
             }
-            z[j] = ~anya;
-            z[j + R / 2] = ~anyb;
+            fa[pa] = ~anya;
+            fa[pb] = ~anyb;
         }
     }
+    uint32_t z[R];
+#pragma unroll
+    for (int j = 0; j < R; j++)
+        z[j] = fa[fa_word(lane + 32 * j)];
     __syncwarp();  // fa may be refilled right after this call
 #pragma unroll
     for (int l = 0; l < 2 * M - 1; l++)

@@ -84,8 +84,8 @@ struct FusedKeyRef {
 // Additive-FFT evaluation plan of one parameter set (fft_plan.cpp): constant
 // tables shared by every key of the set.
 //   scalpow[d*256 + i]: b_d^i, the radix-conversion scale of depth d;
-//   tw[m*off_d + k*n_d + u]: plane k of twiddle word u of depth d (n_d =
-//   2^(m-d-6) words; off_d = the sum of the word counts of the depths before).
+//   tw[k*2^(m-5) + off_d + u]: plane k of twiddle word u of depth d (off_d =
+//   the sum of the word counts 2^(m-e-6) of the depths e < d).
 struct FftPlanDev {
     const uint16_t *scalpow;
     const uint32_t *tw;

@@ -113,7 +113,7 @@ __device__ __forceinline__ void tsynd_one(const LatItem &it, const uint8_t *__re
         for (int k = 0; k < M; k++) {
             B[k] = z[j + R / 2] & __ldg(wf + k * NWD + wb);
             A[k] = (z[j] & __ldg(wf + k * NWD + wa)) ^ B[k];
-            G[k] = __ldg(g + k * (NWD / 2));
+            G[k] = __ldg(g + k * NWD);
         }
 #pragma unroll
         for (int k = 0; k < 2 * M - 1; k++)
@@ -144,7 +144,7 @@ __device__ __forceinline__ void tsynd_one(const LatItem &it, const uint8_t *__re
             for (int k = 0; k < M; k++) {
                 B[k] = fa[k * NWD + pb];
                 A[k] = fa[k * NWD + pa] ^ B[k];
-                G[k] = __ldg(g + k * Sw);
+                G[k] = __ldg(g + k * NWD);
             }
 #pragma unroll
             for (int k = 0; k < 2 * M - 1; k++)
@@ -167,7 +167,7 @@ __device__ __forceinline__ void tsynd_one(const LatItem &it, const uint8_t *__re
         uint32_t G[M];
 #pragma unroll
         for (int k = 0; k < M; k++)
-            G[k] = __ldg(g + k);
+            G[k] = __ldg(g + k * NWD);
 #pragma unroll 1
         for (int j = 0; j < R / 2; j++) {
             const int wa = 2 * (lane + 32 * j);
@@ -492,7 +492,7 @@ __device__ __forceinline__ void root_tile(const LatItem &it, const uint32_t *cv,
 }
 
 // Four CTAs per tile; warp w of CTA c handles ciphertext 8c + w of the tile.
-__global__ void __launch_bounds__(ROOT_WARPS * 32) k_root_tile(const LatItem *__restrict__ items,
+__global__ void __launch_bounds__(ROOT_WARPS * 32, 2) k_root_tile(const LatItem *__restrict__ items,
                                                                const uint32_t *__restrict__ loc_bs,
                                                                uint32_t *__restrict__ err,
                                                                uint16_t *__restrict__ weight, FftPlans plans)

@@ -377,7 +377,7 @@ __device__ __forceinline__ void synd_phase(const LatItem &it, const uint8_t *__r
         for (int k = 0; k < M; k++) {
             B[k] = zb & __ldg(it.wfft + k * NWD + wb);
             A[k] = (za & __ldg(it.wfft + k * NWD + wa)) ^ B[k];
-            G[k] = __ldg(tw + wa + k * (NWD / 2));
+            G[k] = __ldg(tw + wa + k * NWD);
         }
 #pragma unroll
         for (int k = 0; k < 2 * M - 1; k++)
@@ -406,7 +406,7 @@ __device__ __forceinline__ void synd_phase(const LatItem &it, const uint8_t *__r
             for (int k = 0; k < M; k++) {
                 B[k] = fa[k * NWD + pb];
                 A[k] = fa[k * NWD + pa] ^ B[k];
-                G[k] = __ldg(g + k * Sw);
+                G[k] = __ldg(g + k * NWD);
             }
 #pragma unroll
             for (int k = 0; k < 2 * M - 1; k++)
@@ -500,7 +500,7 @@ __device__ __forceinline__ void root_phase(const LatItem &it, uint32_t *err, uin
             }
 #pragma unroll
             for (int k = 0; k < M; k++)
-                G[k] = __ldg(g + k * Sw);
+                G[k] = __ldg(g + k * NWD);
 #pragma unroll
             for (int k = 0; k < 2 * M - 1; k++)
                 p[k] = 0;
@@ -526,7 +526,7 @@ __device__ __forceinline__ void root_phase(const LatItem &it, uint32_t *err, uin
         for (int k = 0; k < M; k++) {
             A[k] = fa[k * NWD + pa];
             B[k] = fa[k * NWD + pb];
-            G[k] = __ldg(tw + wa + k * (NWD / 2));
+            G[k] = __ldg(tw + wa + k * NWD);
         }
 #pragma unroll
         for (int k = 0; k < 2 * M - 1; k++)
