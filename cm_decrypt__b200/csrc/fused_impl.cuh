@@ -17,18 +17,8 @@
 //     four bits select (a read indexed by public ciphertext bits only);
 //  3. transpose the syndromes to bitsliced form (bit q = ciphertext q) by a
 //     shuffle butterfly;
-//  4. Berlekamp-Massey (bm.c:12-68) bitsliced across the 32 ciphertexts: lane
-//     l owns locator coefficients l, l+32, ... (kept in shared memory, so the
-//     per-step loop over them stays rolled and small), the discrepancy is a
-//     redux XOR reduction, B lives in a shared ring buffer whose rotation
-//     implements the x*B shift.  The update is the scaled form C <- b*C +
-//     d*x*B instead of bm()'s C <- C + (d/b)*x*B: same decisions (d != 0,
-//     N >= 2L), same truncation, and by induction the result is lambda times
-//     bm()'s locator with lambda a product of nonzero b values -- the same
-//     roots, so the same flagged positions, with no inversion chain per step.
-//     deg C <= L for every ciphertext, so only coefficients up to the tile's
-//     largest L enter the discrepancy and the update (about half the slots
-//     of the reference loop bounds for weight-t errors, where L ~ N/2);
+//  4. Berlekamp-Massey (bm.c:12-68) bitsliced across the 32 ciphertexts
+//     (bm_tile.cuh);
 //  5. root search (root_13.c:216-240 evaluates the locator at each support
 //     point): the locator is evaluated at all 2^m field elements by an
 //     additive FFT, then the key's support network (the Benes layers that
@@ -44,6 +34,7 @@
 //        the packed error row and its weight.
 //     The tables of the recursion are per set (fft_plan.cpp).
 #pragma once
+#include "bm_tile.cuh"
 #include "fft_root.cuh"
 #include "gf.cuh"
 #include "internal.h"
@@ -58,16 +49,16 @@ __host__ __device__ constexpr int al16(int x) { return (x + 15) / 16 * 16; }
 
 template <int S> struct Fz {
     using P = Set<S>;
-    static constexpr int M = P::M, T = P::T, NJ = (T + 1 + 31) / 32;
+    static constexpr int M = P::M, T = P::T, SS = BmDims<S>::SS;
     static constexpr int TWD = P::TWD;               // dense table row (words)
-    static constexpr int RING = T + 2;               // B ring slots
     static constexpr int NX = FftDims<S>::NX;        // radix-conversion entries
     static constexpr int RAW_B = 32 * P::CT;
-    static constexpr int RING_B = RING * M * 4;
+    static constexpr int RING_B = BmDims<S>::RING_WORDS * 4;
     static constexpr int FA_B = FftDims<S>::FA_WORDS * 4;  // root-search array
-    static constexpr int CM_B = (T + 1) * M * 4;     // BM locator, after the ring
+    static constexpr int CM_B = BmDims<S>::C_WORDS * 4;  // BM locator, after the ring
     static constexpr int A_B = al16(cmax(cmax(RAW_B + 16, RING_B + CM_B), FA_B));
-    static constexpr int S_B = al16(2 * T * M * 4);  // bitsliced syndromes / locator
+    // bitsliced syndromes / the locator's conversion array
+    static constexpr int S_B = al16(4 * cmax(BmDims<S>::SYN_WORDS, NX * SS));
     static constexpr int WARP_B = A_B + S_B;
     static constexpr int NWU = (2 * T * M + 31) / 32;  // syndrome accumulator words in use
     static constexpr int CS = NWU | 1;  // combination row stride: odd, so the 16 rows lanes pick meet distinct banks
@@ -75,7 +66,6 @@ template <int S> struct Fz {
     // group's 16 XOR combinations
     static constexpr int SYN_B = al16((2 * GROUP_ROWS * TWD + 16 * CS) * 4);
     static_assert(P::SB % GROUP_ROWS == 0, "whole groups of ciphertext bits");
-    static_assert(NX * M * 4 <= S_B, "conversion array must fit the syndrome region");
 };
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src)
@@ -137,7 +127,7 @@ __device__ __forceinline__ void fused_round(const RoundCtx &rc, uint8_t *smem)
 {
     using Z = Fz<S>;
     using P = Set<S>;
-    constexpr int M = Z::M, T = Z::T, TWD = Z::TWD, NW = P::NW;
+    constexpr int M = Z::M, T = Z::T, TWD = Z::TWD, SS = Z::SS;
     const FusedArgs &a = *rc.a;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint32_t wfirst;
@@ -243,7 +233,7 @@ __device__ __forceinline__ void fused_round(const RoundCtx &rc, uint8_t *smem)
     if (ntile == 0)
         return;  // no work for this warp in this round (the CTA-wide part is done)
 
-    // ---- 3. transpose: sS[j*M + k] bit q = bit k of syndrome j of ct q ----
+    // ---- 3. transpose: sS[j*SS + k] bit q = bit k of syndrome j of ct q ----
     // Syndrome bit x = j*M + k is bit x mod 32 of accumulator word x / 32.
     // Each accumulator word is a 32x32 bit matrix (row q = lane q's word),
     // and sS wants its transpose: five butterfly steps, each swapping the
@@ -266,141 +256,36 @@ __device__ __forceinline__ void fused_round(const RoundCtx &rc, uint8_t *smem)
                 const uint32_t t = (lane & j) ? (x >> j) : (x << j);
                 v = (v & keep[st]) | (t & ~keep[st]);
             }
-            if (32 * w + lane < 2 * T * M)
-                sS[32 * w + lane] = v;
+            const int x = 32 * w + lane;
+            if (x < 2 * T * M)
+                sS[SS == M ? x : x / M * SS + x % M] = v;
         }
     }
     __syncwarp();
 
     // ---- 4. Berlekamp-Massey, bitsliced across the 32 ciphertexts --------
-    {
-        constexpr int NJ = Z::NJ, R = Z::RING;
-        uint32_t *sCm = ring + R * M;  // locator coefficients [T+1][M]
-        for (int v = lane; v < (T + 1) * M; v += 32)
-            sCm[v] = (v == 0) ? FULLMASK : 0u;  // C = 1
-        for (int v = lane; v < R * M; v += 32)
-            ring[v] = (v == M) ? FULLMASK : 0u;  // B = x
-        uint32_t bb[M];
-#pragma unroll
-        for (int k = 0; k < M; k++)
-            bb[k] = k == 0 ? FULLMASK : 0u;       // b = 1
-        int Lq = 0;                               // L of ciphertext `lane`
-        int Bd = 1;                               // bound on deg B of ciphertext `lane`
-        int Lmax = 0, Bmax = 1;                   // their maxima over the tile
-        __syncwarp();
-#pragma unroll 1
-        for (int N = 0; N < 2 * T; N++) {
-            // deg C <= L for every ciphertext, so coefficients above the
-            // tile's largest L are zero: they take no part in the discrepancy
-            const int lim = min(N, min(T, Lmax));
-            uint32_t p[2 * M - 1];
-#pragma unroll
-            for (int k = 0; k < 2 * M - 1; k++)
-                p[k] = 0;
-#pragma unroll 1
-            for (int j = 0; 32 * j <= lim; j++) {
-                const int i = lane + 32 * j;
-                if (i <= lim) {
-                    const uint32_t *sv = sS + (N - i) * M;
-                    const uint32_t *cp = sCm + i * M;
-                    uint32_t s[M], c[M];
-#pragma unroll
-                    for (int k = 0; k < M; k++) {
-                        s[k] = sv[k];
-                        c[k] = cp[k];
-                    }
-                    bs_mul_acc<M>(p, c, s);
-                }
-            }
-            bs_reduce<M>(p);
-            uint32_t d[M];
-            uint32_t mne = 0;
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const uint32_t v = __reduce_xor_sync(FULLMASK, p[k]);
-                d[k] = v;
-                mne |= v;
-            }
-            const bool my_mle = ((mne >> lane) & 1u) && (N >= 2 * Lq);
-            const uint32_t mle = __ballot_sync(FULLMASK, my_mle);
-            const int Bdn = min(min(my_mle ? Lq : Bd, T) + 1, T);
-            Lq = my_mle ? N + 1 - Lq : Lq;
-            const int Lb = min((int)__reduce_max_sync(FULLMASK, (unsigned)Lq), T);
-            const int Bm = min(Bmax, T);
-            // Scaled update C <- b*C + d*x*B (see the note at the top of the
-            // file): both products accumulate unreduced, one reduction.
-            // After the step deg C <= L, so coefficients above the tile's
-            // new largest L stay zero; B there only takes the swap (to C_i =
-            // 0) where its degree bound reaches, and is zero above that.
-            int off = (R - (N % R)) % R;  // slot(i) = (i - N) mod R
-            const int hi = Lb > Bm ? Lb : Bm;
-#pragma unroll 1
-            for (int j = 0; j < NJ && 32 * j <= hi; j++) {
-                const int i = lane + 32 * j;
-                if (i > Lb && i <= Bm) {
-                    int slot = i + off;
-                    slot = slot >= R ? slot - R : slot;
-                    uint32_t *bp = ring + slot * M;
-#pragma unroll
-                    for (int k = 0; k < M; k++)
-                        bp[k] &= ~mle;
-                } else if (i <= Lb) {
-                    int slot = i + off;
-                    slot = slot >= R ? slot - R : slot;
-                    uint32_t *bp = ring + slot * M;
-                    uint32_t *cp = sCm + i * M;
-                    uint32_t bv[M], oc[M], q[2 * M - 1];
-#pragma unroll
-                    for (int k = 0; k < M; k++) {
-                        bv[k] = bp[k];
-                        oc[k] = cp[k];
-                    }
-#pragma unroll
-                    for (int k = 0; k < 2 * M - 1; k++)
-                        q[k] = 0;
-                    bs_mul_acc<M>(q, bb, oc);
-                    bs_mul_acc<M>(q, d, bv);
-                    bs_reduce<M>(q);
-#pragma unroll
-                    for (int k = 0; k < M; k++) {
-                        cp[k] = q[k];
-                        bp[k] = (bv[k] & ~mle) | (oc[k] & mle);
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < M; k++)
-                bb[k] = (bb[k] & ~mle) | (d[k] & mle);
-            const int freeslot = (R - ((N + 1) % R)) % R;
-            if (lane < M)
-                ring[freeslot * M + lane] = 0;
-            Bd = Bdn;
-            Lmax = Lb;
-            // (lanes past the tile's count never take the swap: zero syndromes)
-            Bmax = (int)__reduce_max_sync(FULLMASK, lane < ntile ? (unsigned)Bd : 0u);
-            __syncwarp();
-        }
-        // The reference's root search evaluates sum_x C[T-x] a^x
-        // (bm.c:62-65 reverses the locator): entry x of the conversion array
-        // is C[T-x], zero for T < x < 2^D.
-        for (int v = lane; v < (T + 1) * M; v += 32) {
-            const int i = v / M, k = v - i * M;
-            cv[(T - i) * M + k] = sCm[v];
-        }
-        for (int v = lane; v < (Z::NX - T - 1) * M; v += 32)
-            cv[(T + 1) * M + v] = 0u;
-        __syncwarp();
+    uint32_t *cm = ring + BmDims<S>::RING_WORDS;
+    bm_tile_warp<S>(sS, ring, cm, ntile, lane);
+    // The reference's root search evaluates sum_x C[T-x] a^x (bm.c:62-65
+    // reverses the locator): entry x of the conversion array is C[T-x], zero
+    // for T < x < 2^D.
+    for (int v = lane; v < (T + 1) * SS; v += 32) {
+        const int i = v / SS, k = v - i * SS;
+        cv[(T - i) * SS + k] = cm[v];
     }
+    for (int v = lane; v < (Z::NX - T - 1) * SS; v += 32)
+        cv[(T + 1) * SS + v] = 0u;
+    __syncwarp();
 
     // ---- 5. root search (fft_root.cuh) -------------------------------------
     const FftPlanDev pl = a.fft[S];
-    fft_convert<S, M, 32>(cv, pl.scalpow, lane, [] { __syncwarp(); });
+    fft_convert<S, SS, 32>(cv, pl.scalpow, lane, [] { __syncwarp(); });
     for (int q = 0; q < ntile; q++) {
         const uint64_t c = ct_index(rc, wfirst, q);
         uint32_t *erow = a.err ? a.err + (a.err_off ? a.err_off[c] : c * (uint64_t)a.err_stride) : nullptr;
         uint16_t *prow = a.pos ? a.pos + c * (uint64_t)a.pos_stride : nullptr;
         uint8_t *epack = a.err_packed ? a.err_packed + c * (uint64_t)(Set<S>::N / 8) : nullptr;
-        const int cnt = fft_root_one<S, M>(cv, q, fa, pl.tw, rc.key.bctl, erow, prow, lane, epack);
+        const int cnt = fft_root_one<S, SS>(cv, q, fa, pl.tw, rc.key.bctl, erow, prow, lane, epack);
         if (lane == 0 && a.weight)
             a.weight[c] = (uint16_t)cnt;
     }

@@ -146,6 +146,67 @@ template <int M> __device__ __forceinline__ void bs_mul_acc(uint32_t *p, const u
             p[i + j] ^= x[i] & y[j];
 }
 
+// One-level Karatsuba form of the same product, for sums of products that are
+// combined once: x = x0 + X^H x1 with H = ceil(M/2), so
+//   x*y = lo + X^H (mid + lo + hi) + X^2H hi,
+// lo = x0 y0, hi = x1 y1, mid = (x0 + x1)(y0 + y1).  134 AND-XORs instead of 169
+// for M = 13 (108 instead of 144 for M = 12); the sums x0 + x1 (6 XORs an
+// operand) and the combination (19; 16) are worth it where an operand is shared
+// by several products or several products share the combination.
+template <int M> struct KAcc {
+    static constexpr int H = (M + 1) / 2, W = M - H;  // planes of x0 and of x1
+    uint32_t lo[2 * H - 1], hi[2 * W - 1], mid[2 * H - 1];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int k = 0; k < 2 * H - 1; k++)
+            lo[k] = mid[k] = 0;
+#pragma unroll
+        for (int k = 0; k < 2 * W - 1; k++)
+            hi[k] = 0;
+    }
+    // xs, ys: ksum of x and y
+    __device__ __forceinline__ void mac(const uint32_t *x, const uint32_t *xs, const uint32_t *y, const uint32_t *ys)
+    {
+#pragma unroll
+        for (int i = 0; i < H; i++)
+#pragma unroll
+            for (int j = 0; j < H; j++) {
+                lo[i + j] ^= x[i] & y[j];
+                mid[i + j] ^= xs[i] & ys[j];
+                if (i < W && j < W)
+                    hi[i + j] ^= x[H + i] & y[H + j];
+            }
+    }
+    // p[0 .. 2M-2] = the unreduced sum
+    __device__ __forceinline__ void combine(uint32_t *p) const
+    {
+#pragma unroll
+        for (int k = 0; k < H; k++)
+            p[k] = lo[k];
+#pragma unroll
+        for (int k = 0; k < 2 * H - 1; k++)  // plane H + k; the part both neighbours share first
+            p[H + k] = (k < W && H + k < 2 * H - 1 ? lo[H + k] ^ hi[k] : k < 2 * W - 1 ? hi[k] : 0u) ^ mid[k] ^ lo[k];
+#pragma unroll
+        for (int k = 0; k < 2 * W - 1; k++) {  // plane 2H + k
+            if (2 * H + k <= 3 * H - 2) {
+                // lo[H + k] ^ hi[k] again, with hi[H + k]
+                p[2 * H + k] = (H + k < 2 * H - 1 ? lo[H + k] ^ hi[k] : hi[k]) ^ mid[H + k] ^
+                               (H + k < 2 * W - 1 ? hi[H + k] : 0u);
+            } else {
+                p[2 * H + k] = hi[k];
+            }
+        }
+    }
+};
+template <int M> __device__ __forceinline__ void ksum(uint32_t *xs, const uint32_t *x)
+{
+    constexpr int H = (M + 1) / 2, W = M - H;
+#pragma unroll
+    for (int k = 0; k < H; k++)
+        xs[k] = k < W ? x[k] ^ x[H + k] : x[k];
+}
+
 // o = x * y (o may alias x or y).
 template <int M> __device__ __forceinline__ void bs_mul(uint32_t *o, const uint32_t *x, const uint32_t *y)
 {
