@@ -1,7 +1,6 @@
-// Berlekamp-Massey (bm.c:12-68) bitsliced across the 32 ciphertexts of a warp's
-// tile: word bit q belongs to ciphertext q, lane l owns locator coefficients l,
-// l + 32, ...  Coefficients, syndromes and B are rows of SS words in the warp's
-// shared memory (SS = m made odd, so that lanes' rows meet no bank conflict; for
+// Berlekamp-Massey (bm.c:12-68) bitsliced across the 32 ciphertexts of a tile:
+// word bit q belongs to ciphertext q, lane l owns locator coefficients l, l + 32,
+// ...  Coefficients, syndromes and B are rows of SS words in shared memory (SS = m made odd, so that lanes' rows meet no bank conflict; for
 // m = 12 the 12-word rows of neighbouring lanes met four ways).
 //
 // The update is the scaled form C <- b*C + d*x*B instead of bm()'s C <- C +
@@ -31,35 +30,88 @@ template <int S> struct BmDims {
     static constexpr int SYN_WORDS = 2 * T * SS, RING_WORDS = R * SS, C_WORDS = (T + 1) * SS;
 };
 
-// One warp: syndromes syn -> locator coefficients C (both rows of SS words);
-// ntile: ciphertexts of the tile (the others' syndromes are zero).
-template <int S>
-__device__ __forceinline__ void bm_tile_warp(const uint32_t *syn, uint32_t *ring, uint32_t *cm, int ntile, int lane)
+// W warps (thread tid < 32 W of them): syndromes -> locator coefficients C (rows
+// of SS words); ntile: ciphertexts of the tile (the others' syndromes are zero).
+//
+// W = 1: the warp alone.  W > 1: groups of 32 coefficients go round the warps,
+// which meet once a step (named barrier 1) to add their shares of the
+// discrepancy (share: 2 W rows of 16 words); for batches that leave schedulers
+// without a warp.  The first groups are active longest, so warp (W - turn) % W
+// takes the first one: callers vary `turn` between the tiles of an SM.
+//
+// The syndromes are either all in shared memory (syn, gsyn null) or in global
+// memory (gsyn), one row a step coming into syn as a ring of t + 2 rows: step N
+// multiplies rows N + 1 - L .. N + 1 only, and L stops at t.  The ring takes a
+// quarter off a tile's shared memory.
+template <int S, bool GLOBAL_SYN = false, int W = 1>
+__device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t *cm, int ntile, int tid,
+                                        const uint32_t *gsyn = nullptr, uint32_t *share = nullptr, int turn = 0)
 {
     using Z = BmDims<S>;
-    constexpr int M = Z::M, T = Z::T, SS = Z::SS, R = Z::R, H = KAcc<M>::H;
+    constexpr int M = Z::M, T = Z::T, SS = Z::SS, R = Z::R, H = KAcc<M>::H, NT = 32 * W;
     constexpr uint32_t FULL = 0xFFFFFFFFu;
-    for (int v = lane; v < Z::C_WORDS; v += 32)
+    const int lane = tid & 31, warp = tid >> 5;
+    const int first = W == 1 ? tid : (tid + 32 * turn) % NT;  // this lane's first coefficient
+    auto sync = [] {
+        if constexpr (W == 1)
+            __syncwarp();
+        else
+            asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+    };
+    for (int v = tid; v < Z::C_WORDS; v += NT)
         cm[v] = v == 0 ? FULL : 0u;  // C = 1
-    for (int v = lane; v < Z::RING_WORDS; v += 32)
+    for (int v = tid; v < Z::RING_WORDS; v += NT)
         ring[v] = v == SS ? FULL : 0u;  // B = x
+    if constexpr (GLOBAL_SYN) {
+        for (int v = tid; v < 2 * SS; v += NT)
+            syn[v] = gsyn[v];
+        sync();
+    }
     uint32_t b[M], p[2 * M - 1];  // p: this lane's share of the discrepancy
 #pragma unroll
     for (int k = 0; k < M; k++) {
-        b[k] = k == 0 ? FULL : 0u;              // b = 1
-        p[k] = lane == 0 ? syn[k] : 0u;         // d_0 = C_0 S_0
+        b[k] = k == 0 ? FULL : 0u;      // b = 1
+        p[k] = tid == 0 ? syn[k] : 0u;  // d_0 = C_0 S_0 (any one lane)
     }
-    int Lq = 0;              // L of ciphertext `lane`
-    int Bd = 1, Bmax = 1;    // bound on deg B of ciphertext `lane`; the tile's
-    __syncwarp();
+    int Lq = 0;            // L of ciphertext `lane`
+    int Bd = 1, Bmax = 1;  // bound on deg B of ciphertext `lane`; the tile's
+    if (W == 1)
+        sync();
 #pragma unroll 1
     for (int N = 0; N < 2 * T; N++) {
+        uint32_t row = 0;
+        if (GLOBAL_SYN && tid < SS && N + 2 < 2 * T)
+            row = gsyn[(N + 2) * SS + tid];
         uint32_t d[M], mne = 0;
 #pragma unroll
-        for (int k = 0; k < M; k++) {
+        for (int k = 0; k < M; k++)
             d[k] = __reduce_xor_sync(FULL, p[k]);
-            mne |= d[k];
+        if constexpr (W > 1) {
+            uint32_t *sh = share + (N & 1) * W * 16;  // rewritten two barriers later
+            uint32_t mine = 0;
+#pragma unroll
+            for (int k = 0; k < M; k++)
+                mine = lane == k ? d[k] : mine;
+            if (lane < M)
+                sh[warp * 16 + lane] = mine;
+            sync();
+#pragma unroll
+            for (int k = 0; k < M; k++)
+                d[k] = 0;
+#pragma unroll
+            for (int w = 0; w < W; w++)
+#pragma unroll
+                for (int v = 0; v < (M + 3) / 4; v++) {
+                    const uint4 x = reinterpret_cast<const uint4 *>(sh + w * 16)[v];
+                    if (4 * v + 0 < M) d[4 * v + 0] ^= x.x;
+                    if (4 * v + 1 < M) d[4 * v + 1] ^= x.y;
+                    if (4 * v + 2 < M) d[4 * v + 2] ^= x.z;
+                    if (4 * v + 3 < M) d[4 * v + 3] ^= x.w;
+                }
         }
+#pragma unroll
+        for (int k = 0; k < M; k++)
+            mne |= d[k];
         const bool my_mle = ((mne >> lane) & 1u) && (N >= 2 * Lq);
         const uint32_t mle = __ballot_sync(FULL, my_mle);
         const int Bdn = min(min(my_mle ? Lq : Bd, T) + 1, T);
@@ -77,14 +129,16 @@ __device__ __forceinline__ void bm_tile_warp(const uint32_t *syn, uint32_t *ring
         const int off = (R - (N % R)) % R;  // slot(i) = (i - N) mod R
         const int next = min(N + 1, 2 * T - 1);
         const int hi = max(Lb, Bm);
+        const int srow = GLOBAL_SYN ? next % R : next;
 #pragma unroll 1
-        for (int i = lane; (i & ~31) <= hi; i += 32) {
+        for (int i = first; (i & ~31) <= hi; i += NT) {
             int slot = i + off;
             slot = slot >= R ? slot - R : slot;
             uint32_t *bp = ring + slot * SS;
             if (i <= Lb) {
                 uint32_t *cp = cm + i * SS;
-                const uint32_t *sp = syn + (next - i) * SS;
+                const int sr = srow - i;
+                const uint32_t *sp = syn + (GLOBAL_SYN && sr < 0 ? sr + R : sr) * SS;
                 uint32_t bv[M], c[M], s[M], xs[H], ys[H], q[2 * M - 1];
 #pragma unroll
                 for (int k = 0; k < M; k++) {
@@ -119,15 +173,20 @@ __device__ __forceinline__ void bm_tile_warp(const uint32_t *syn, uint32_t *ring
         for (int k = 0; k < M; k++)
             b[k] = (b[k] & ~mle) | (d[k] & mle);
         const int freeslot = (R - ((N + 1) % R)) % R;
-        if (lane < M)
-            ring[freeslot * SS + lane] = 0;
+        if (tid < M)
+            ring[freeslot * SS + tid] = 0;
+        if (GLOBAL_SYN && tid < SS)  // over row N - t, which no later step reads
+            syn[(N + 2) % R * SS + tid] = row;
         Bd = Bdn;
         // (lanes past the tile's count never take the swap: zero syndromes)
         Bmax = (int)__reduce_max_sync(FULL, lane < ntile ? (unsigned)Bd : 0u);
         acc.combine(p);
         bs_reduce<M>(p);
-        __syncwarp();
+        if (W == 1)
+            sync();  // W > 1: the next discrepancy's barrier
     }
+    if (W > 1)
+        sync();
 }
 
 }  // namespace cmd

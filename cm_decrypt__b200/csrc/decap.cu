@@ -272,8 +272,9 @@ int cmd_kem_decap_device(cmd_engine *eng, cmd_key *key, const uint8_t *d_cts, si
         return rc;
     uint32_t *d_err = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(eng->scratch.ptr) + inner);
     uint16_t *d_w = reinterpret_cast<uint16_t *>(d_err + words);
-    rc = inner || count <= CT_ONE_LAUNCH ? run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)
-                                         : run_fused_single(eng, key, d_cts, count, d_err, d_w, s);
+    rc = inner || !auto_scratch_bytes(eng, key->dev.set, count)
+             ? run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)
+             : run_fused_single(eng, key, d_cts, count, d_err, d_w, s);
     if (rc)
         return rc;
     const uint8_t *d_s = key->dev.sk + 40 + 2 * si.t + si.cond;

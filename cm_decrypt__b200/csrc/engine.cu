@@ -197,6 +197,7 @@ void cmd_engine_destroy(cmd_engine *eng)
     eng->scratch.release(eng);
     eng->io.release(eng);
     eng->fused.release(eng);
+    eng->staged.release(eng);
     eng->keygen.release(eng);
     eng->host_scratch.release();
     release_fft_plans(eng);
@@ -205,6 +206,12 @@ void cmd_engine_destroy(cmd_engine *eng)
             cudaStreamSynchronize(eng->piece_stream[i]);
             cudaStreamDestroy(eng->piece_stream[i]);
         }
+    for (cudaEvent_t ev : {eng->staged_fork, eng->staged_done})
+        if (ev)
+            cudaEventDestroy(ev);
+    for (cudaEvent_t ev : eng->staged_join)
+        if (ev)
+            cudaEventDestroy(ev);
     if (eng->tile_counter)
         cudaFree(eng->tile_counter);
     cudaStreamDestroy(eng->stream);
@@ -465,34 +472,117 @@ static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
     return CMD_OK;
 }
 
-// Batch size below which CMD_PATH_AUTO (and positions and decapsulation, up to
-// the per-ciphertext kernels' limit) leaves the fused kernel: the tuned
-// crossover, or one that holds for every set on a B200 when the engine has
-// not been tuned.  The fused kernel's time is flat up to about four tiles an
-// SM (one 6960119 ciphertext 779 us, 9,472 1,208 us), the small-batch kernels'
-// is 79 us for one, 501 us for 4,736 and 796 us for 9,472 (348864: 458 us
-// against 47, 249 and 377 us).
-static size_t small_below(const FusedConfig &c)
+int ensure_piece_streams(cmd_engine *eng)
 {
-    return c.tuned || c.tile_below ? c.tile_below : 8192;
+    for (int i = 0; i < BATCH_STREAMS; i++)
+        if (!eng->piece_stream[i]) {
+            const cudaError_t e = cudaStreamCreateWithFlags(&eng->piece_stream[i], cudaStreamNonBlocking);
+            if (e != cudaSuccess)
+                return cuda_fail(e, "cudaStreamCreate(piece)");
+        }
+    return CMD_OK;
+}
+
+// Parts of a staged batch: one up to 45,000 ciphertexts (about a wave of
+// Berlekamp-Massey warps), two equal ones up to 131,072, then parts of about
+// 65,536.  Parts run on their own streams, STAGED_STREAMS in flight, so that one
+// part's syndromes (shared-memory bound) and ends of waves run beside another's
+// Berlekamp-Massey and FFT (logic bound): 65,536 mceliece6960119 ciphertexts
+// 2,709 us in one part, 2,537 us in two; 262,144 10,527 us in one stream's
+// parts of 131,072, 9,642 us in four of 65,536.
+static size_t staged_part(size_t count)
+{
+    const size_t parts = count <= 45000 ? 1 : count <= 131072 ? 2 : (count + 65535) / 65536;
+    return ((count + parts - 1) / parts + 31) / 32 * 32;
+}
+
+int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
+               uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
+{
+    const SetInfo si = set_info(key->dev.set);
+    const size_t part = staged_part(count), nparts = (count + part - 1) / part;
+    const size_t ns = std::min<size_t>(nparts, STAGED_STREAMS), words = staged_scratch_words(key->dev.set, part);
+    int rc = eng->staged.reserve(eng, ns * words * 4);
+    if (rc || (rc = ensure_piece_streams(eng)))
+        return rc;
+    cudaError_t e = cudaSuccess;
+    if (!eng->staged_done) {
+        auto make = [&](cudaEvent_t *ev) {
+            if (e == cudaSuccess)
+                e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        };
+        make(&eng->staged_fork);
+        for (cudaEvent_t &ev : eng->staged_join)
+            make(&ev);
+        make(&eng->staged_done);
+    } else if (eng->staged_last != s) {
+        // the scratch may still be in use by a batch on another stream
+        e = cudaStreamWaitEvent(s, eng->staged_done);
+    }
+    if (e == cudaSuccess && ns > 1) {
+        e = cudaEventRecord(eng->staged_fork, s);
+        for (size_t i = 0; i < ns && e == cudaSuccess; i++)
+            e = cudaStreamWaitEvent(eng->piece_stream[i], eng->staged_fork);
+    }
+    for (size_t p = 0; p < nparts && e == cudaSuccess; p++) {
+        const size_t c0 = p * part, n = std::min(part, count - c0), i = p % ns;
+        e = launch_staged(key->dev, d_cts + c0 * si.ct, (uint32_t)n,
+                          static_cast<uint32_t *>(eng->staged.ptr) + i * words, d_err ? d_err + c0 * si.nw : nullptr,
+                          d_weight ? d_weight + c0 : nullptr, d_pos ? d_pos + c0 * (si.t + 1) : nullptr, nullptr,
+                          eng->fft[key->dev.set], eng->num_sms, ns > 1 ? eng->piece_stream[i] : s,
+                          LaunchCounter{&eng->launches});
+    }
+    for (size_t i = 0; i < ns && ns > 1; i++) {  // joined even after an error
+        cudaError_t e2 = cudaEventRecord(eng->staged_join[i], eng->piece_stream[i]);
+        if (e2 == cudaSuccess)
+            e2 = cudaStreamWaitEvent(s, eng->staged_join[i]);
+        if (e == cudaSuccess)
+            e = e2;
+    }
+    if (e == cudaSuccess)
+        e = cudaEventRecord(eng->staged_done, s);
+    eng->staged_last = s;
+    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "staged batch");
+}
+
+// Whether CMD_PATH_AUTO takes the small-batch kernels: batches within the
+// per-ciphertext kernels' reach, or below the tuned crossover.  At 24 ciphertexts
+// an SM (3,552) the per-ciphertext kernels and the staged ones take the same time
+// (6960119 442 and 447 us, 348864 202 and 235 us), at half of that 206 against
+// 415 us; the fused kernel takes 1,037 us for any number up to 18,944.
+static bool takes_small(const cmd_engine *eng, int set, size_t count)
+{
+    return count <= (size_t)CT_PER_SM * eng->num_sms || count < eng->fcfg[set].tile_below;
 }
 
 size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count)
 {
-    return count < small_below(eng->fcfg[set]) && count > CT_ONE_LAUNCH ? tile_single_scratch_words(count) * 4 : 0;
+    return takes_small(eng, set, count) && count > CT_ONE_LAUNCH ? tile_single_scratch_words(count) * 4 : 0;
 }
 
-// The best kernels for the batch size, error rows and weights or positions.
-// Small batches fall back to the fused kernel, which needs no scratch, when
-// their scratch does not fit the budget.
+// The best kernels for the batch size, error rows and weights or positions:
+// small-batch kernels, else the staged ones.  The fused kernel takes batches of
+// six to eight tiles an SM, one nearly full round of its warps (37,888
+// mceliece6960119 ciphertexts 1,505 us, staged 1,534 us); needing no scratch, it
+// also runs when theirs does not fit the budget, and under stream capture, where
+// nothing may be allocated and a graph would keep the address of scratch that can
+// grow.
 static int run_auto(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                     uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
 {
-    if (count < small_below(eng->fcfg[key->dev.set]) && (!d_pos || count <= (size_t)CT_PER_SM * eng->num_sms)) {
-        if (eng->scratch.reserve(eng, auto_scratch_bytes(eng, key->dev.set, count)) == CMD_OK)
-            return run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s);
-        cudaGetLastError();
+    const int set = key->dev.set;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        if (takes_small(eng, set, count) && (!d_pos || count <= (size_t)CT_PER_SM * eng->num_sms)) {
+            if (eng->scratch.reserve(eng, auto_scratch_bytes(eng, set, count)) == CMD_OK)
+                return run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s);
+        } else if (count <= 192 * (size_t)eng->num_sms || count > 256 * (size_t)eng->num_sms) {
+            const int rc = run_staged(eng, key, d_cts, count, d_err, d_weight, d_pos, s);
+            if (rc != CMD_E_BUDGET)
+                return rc;
+        }
     }
+    cudaGetLastError();
     return run_fused_single(eng, key, d_cts, count, d_err, d_weight, s, d_pos);
 }
 
@@ -570,9 +660,12 @@ int cmd_decrypt_batch(cmd_engine *eng, const cmd_key *key, cmd_path path, const 
     uint32_t *d_err = cv.take<uint32_t>(chunk * si.nw);
     uint16_t *d_w = cv.take<uint16_t>(chunk);
     cudaStream_t s = eng->stream;
-    // Large fused batches go as BATCH_STREAMS pieces on their own streams
-    // (each with its own work counter, full rounds): one piece's copies run
-    // while the others compute, and the pieces' kernels share the SMs.
+    // Large batches go as BATCH_STREAMS fused pieces on their own streams (each
+    // with its own work counter, full rounds): one piece's copies run while the
+    // others compute, and the pieces' kernels share the SMs.  The fused kernel
+    // rather than the staged ones, because its rows come out evenly over its run:
+    // staged pieces that fill the GPU end together, and their copies out follow
+    // (100,003 mceliece6960119 ciphertexts 5.2 to 6.2 ms against 4.9 ms).
     const bool pieces = path != CMD_PATH_PLAIN && path != CMD_PATH_TILE && chunk >= (size_t)BATCH_STREAMS * 8192;
     // With host error rows the GPU can write, the pieces' kernels store the
     // packed rows there directly: the rows cross PCIe while the kernels run,
@@ -581,12 +674,8 @@ int cmd_decrypt_batch(cmd_engine *eng, const cmd_key *key, cmd_path path, const 
     if (pieces) {
         if ((rc = ensure_counter(eng)))
             return rc;
-        for (int i = 0; i < BATCH_STREAMS; i++)
-            if (!eng->piece_stream[i]) {
-                cudaError_t e = cudaStreamCreateWithFlags(&eng->piece_stream[i], cudaStreamNonBlocking);
-                if (e != cudaSuccess)
-                    return cuda_fail(e, "cudaStreamCreate(piece)");
-            }
+        if ((rc = ensure_piece_streams(eng)))
+            return rc;
     }
     for (size_t c0 = 0; c0 < count; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
@@ -684,12 +773,8 @@ int cmd_decrypt_positions(cmd_engine *eng, const cmd_key *key, const uint8_t *h_
     if (pieces) {
         if ((rc = ensure_counter(eng)))
             return rc;
-        for (int i = 0; i < BATCH_STREAMS; i++)
-            if (!eng->piece_stream[i]) {
-                cudaError_t e = cudaStreamCreateWithFlags(&eng->piece_stream[i], cudaStreamNonBlocking);
-                if (e != cudaSuccess)
-                    return cuda_fail(e, "cudaStreamCreate(piece)");
-            }
+        if ((rc = ensure_piece_streams(eng)))
+            return rc;
     }
     for (size_t c0 = 0; c0 < count; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);

@@ -66,6 +66,10 @@ int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t
 size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count);
 int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                      uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos = nullptr);
+// The staged kernels over one key's device batch (see engine.cu): err/weight or
+// pos, each or null.  CMD_E_BUDGET when their scratch does not fit.
+int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
+               uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s);
 // Explicit work counter and round schedule (balanced: -1 = the tuned choice,
 // 0 = full rounds, 1 = equal shares; round_cts > 0 overrides all three with
 // rounds of that many ciphertexts, a multiple of 32 from fused_round).
@@ -79,6 +83,8 @@ int run_fused_counter(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts,
 uint32_t fused_round(cmd_engine *eng, int set, size_t count);
 int ensure_counter(cmd_engine *eng);  // eng->tile_counter: 64 u32 work counters
 constexpr int BATCH_STREAMS = 8;      // pieces of a host-buffer batch in flight
+constexpr int STAGED_STREAMS = 4;     // parts of a staged device batch in flight
+int ensure_piece_streams(cmd_engine *eng);
 size_t fused_smem(int set, int wpb);
 size_t smem_limit_bytes();
 int fused_blocks_per_sm(int single_set, int wpb, size_t smem);
@@ -108,6 +114,10 @@ struct cmd_engine {
     cmd::Scratch scratch;          // plain-path intermediates
     cmd::Scratch io;               // device staging for host-buffer calls
     cmd::Scratch fused;            // fused-kernel work lists
+    cmd::Scratch staged;           // staged kernels' intermediates, one part per piece stream
+    cudaEvent_t staged_fork = nullptr, staged_join[cmd::STAGED_STREAMS] = {};  // created on first use
+    cudaEvent_t staged_done = nullptr;      // recorded after each staged batch, on staged_last
+    cudaStream_t staged_last = nullptr;
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
     cmd::HostScratch host_scratch; // pinned staging
     uint32_t *tile_counter = nullptr;

@@ -237,6 +237,44 @@ __device__ __forceinline__ void swap_layer(uint32_t *z, const uint32_t *__restri
     }
 }
 
+// The whole network, layer 0 first, over NC arrays of one warp (word lane + 32j of
+// array i in z[i][j]); each layer's mask words are loaded once for all of them.
+template <int S, int NC>
+__device__ __forceinline__ void swap_network(uint32_t (*z)[FftDims<S>::R], const uint32_t *__restrict__ bctl, int lane)
+{
+    using F = FftDims<S>;
+    constexpr int M = F::M, NWD = F::NWD, R = F::R;
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+#pragma unroll
+    for (int l = 0; l < 2 * M - 1; l++) {
+        const int e = l < M ? l : 2 * M - 2 - l;
+        const uint32_t *ml = bctl + l * NWD;
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int js = e < 10 ? 0 : 1 << (e - 10);
+            if (j & js)
+                continue;
+            const int ls = e < 5 || e >= 10 ? 0 : 1 << (e - 5);
+            const uint32_t mk = __ldg(ml + (lane & ~ls) + 32 * j);
+#pragma unroll
+            for (int i = 0; i < NC; i++) {
+                uint32_t *w = z[i];
+                if (e < 5) {  // pairs inside a word
+                    const uint32_t t = ((w[j] >> (1 << e)) ^ w[j]) & mk;
+                    w[j] ^= t ^ (t << (1 << e));
+                } else if (e < 10) {  // pairs across lanes
+                    const uint32_t other = __shfl_xor_sync(FULL, w[j], ls);
+                    w[j] ^= (w[j] ^ other) & mk;
+                } else {  // pairs inside a lane
+                    const uint32_t t = (w[j] ^ w[j | js]) & mk;
+                    w[j] ^= t;
+                    w[j | js] ^= t;
+                }
+            }
+        }
+    }
+}
+
 // Error row of n/8 bytes at byte address p (2-byte aligned), from the words
 // v[j] = row word lane + 32j: 32-bit stores to 4-byte aligned addresses (a
 // warp's store covers whole 128-byte lines), the row's odd 16-bit ends as
@@ -389,18 +427,12 @@ __device__ __forceinline__ void butterfly4(uint32_t (*w)[M], const uint32_t *__r
 // took 1,821 us for 37,888 mceliece6960119 ciphertexts, rolled 1,643 us; 65,536
 // of them 3,143 us with one depth a pass and 3,119 us so.
 //
-// One warp: error row (and weight) of locator q from the converted array cv
-// (bitsliced, cv[s * CVS + k]).  fa: this warp's FA_WORDS words of shared
-// memory.  erow: NW words, or null.  epack: null, or the row's n/8 bytes
-// packed (store_row_packed).  prow: null, or t+1 u16 that receive the
-// weight, the flagged positions in ascending order and 0xFFFF in the unused
-// slots (the weight never exceeds t: the reversed locator's leading
-// coefficient is C[0], which the update never zeroes).  Returns the weight
-// (all lanes).
+// One warp: the zero flags of locator q at all 2^m elements, FFT position order
+// (z[j] = word lane + 32j), from the converted array cv (bitsliced, cv[s * CVS +
+// k]).  fa: this warp's FA_WORDS words of shared memory.
 template <int S, int CVS>
-__device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t *fa, const uint32_t *__restrict__ tw,
-                                            const uint32_t *__restrict__ bctl, uint32_t *erow, uint16_t *prow,
-                                            int lane, uint8_t *epack = nullptr)
+__device__ __forceinline__ void fft_eval_one(const uint32_t *cv, int q, uint32_t *fa, const uint32_t *__restrict__ tw,
+                                             int lane, uint32_t *z)
 {
     using F = FftDims<S>;
     constexpr int M = F::M, D = F::D, NWD = F::NWD, R = F::R;
@@ -498,11 +530,27 @@ __device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t 
             fa[pb] = ~anyb;
         }
     }
-    uint32_t z[R];
 #pragma unroll
     for (int j = 0; j < R; j++)
         z[j] = fa[fa_word(lane + 32 * j)];
     __syncwarp();  // fa may be refilled right after this call
+}
+
+// One warp: error row (and weight) of locator q from the converted array cv (as
+// for fft_eval_one).  erow: NW words, or null.  epack: null, or the row's n/8
+// bytes packed (store_row_packed).  prow: null, or t+1 u16 that receive the
+// weight, the flagged positions in ascending order and 0xFFFF in the unused
+// slots (the weight never exceeds t: the reversed locator's leading
+// coefficient is C[0], which the update never zeroes).  Returns the weight
+// (all lanes).
+template <int S, int CVS>
+__device__ __forceinline__ int fft_root_one(const uint32_t *cv, int q, uint32_t *fa, const uint32_t *__restrict__ tw,
+                                            const uint32_t *__restrict__ bctl, uint32_t *erow, uint16_t *prow,
+                                            int lane, uint8_t *epack = nullptr)
+{
+    constexpr int M = Set<S>::M;
+    uint32_t z[FftDims<S>::R];
+    fft_eval_one<S, CVS>(cv, q, fa, tw, lane, z);
 #pragma unroll
     for (int l = 0; l < 2 * M - 1; l++)
         swap_layer<S>(z, bctl, l, lane);

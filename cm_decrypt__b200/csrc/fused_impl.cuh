@@ -265,7 +265,7 @@ __device__ __forceinline__ void fused_round(const RoundCtx &rc, uint8_t *smem)
 
     // ---- 4. Berlekamp-Massey, bitsliced across the 32 ciphertexts --------
     uint32_t *cm = ring + BmDims<S>::RING_WORDS;
-    bm_tile_warp<S>(sS, ring, cm, ntile, lane);
+    bm_tile<S>(sS, ring, cm, ntile, lane);
     // The reference's root search evaluates sum_x C[T-x] a^x (bm.c:62-65
     // reverses the locator): entry x of the conversion array is C[T-x], zero
     // for T < x < 2^D.

@@ -118,6 +118,14 @@ struct FusedArgs {
 cudaError_t launch_fused(const FusedArgs &a, int grid, int warps_per_block, cudaStream_t s,
                          LaunchCounter lc);
 
+// One key's batch in four kernels (staged.cu): error rows at the set's nw stride,
+// weights, positions rows (FusedArgs::pos), packed rows (FusedArgs::err_packed),
+// each or null.  d_scratch: staged_scratch_words(set, count) words.
+cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count, uint32_t *d_scratch, uint32_t *d_err,
+                          uint16_t *d_weight, uint16_t *d_pos, uint8_t *err_packed, const FftPlanDev &plan,
+                          int num_sms, cudaStream_t s, LaunchCounter lc);
+size_t staged_scratch_words(int set, size_t count);
+
 // Latency path (serving loop; latency.cu): one work item per ciphertext.
 struct LatItem {
     const uint32_t *wfft; // key's syndrome weights in FFT order (KeyDev::wfft)

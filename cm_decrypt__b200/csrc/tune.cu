@@ -2,12 +2,11 @@
 //
 // Tuner: for one parameter set on one GPU it times the candidate launch
 // configurations (warps per CTA x round schedule) on a device batch and keeps
-// the fastest; then it times the fastest against the tile kernels (five warps
-// per 32-ciphertext tile for Berlekamp-Massey instead of one) at growing batch
-// sizes and records the size from which the fused kernel wins, below which
-// CMD_PATH_AUTO takes the tile kernels.  The decrypt kernels' instruction stream does not depend on
-// the ciphertext contents, so the sample is a constant byte pattern.  Choices
-// are cached per engine and persisted as JSON keyed by (GPU name, set) in
+// the fastest; then it times the small-batch kernels against the staged ones at
+// growing batch sizes and records the size from which the staged ones win, below
+// which CMD_PATH_AUTO takes the small-batch kernels.  The decrypt kernels'
+// instruction stream does not depend on the ciphertext contents, so the sample is
+// a constant byte pattern.  Choices are cached per engine and persisted as JSON keyed by (GPU name, set) in
 // $CMD_TUNE_CACHE (default ~/.cache/cmd_b200/tune.json).
 //
 // Graphs: a decrypt over fixed device buffers is captured once and replayed,
@@ -249,10 +248,8 @@ int cmd_tune(cmd_engine *eng, const cmd_key *key, size_t sample_count, int force
         return CMD_E_CUDA;
     }
     eng->fcfg[set] = best;
-    // Fused kernel (one warp per tile) against the tile kernels at growing
-    // batch sizes: the tile kernels finish small batches sooner (their
-    // Berlekamp-Massey runs on five warps, their FFTs on a warp per
-    // ciphertext), the fused kernel does less work per ciphertext.
+    // The staged kernels, which CMD_PATH_AUTO runs otherwise, against the
+    // small-batch kernels at growing batch sizes.
     best.tile_below = 0;
     const size_t sizes[] = {256, 1024, 4096, 16384, 65536};
     for (size_t n : sizes) {
@@ -262,9 +259,10 @@ int cmd_tune(cmd_engine *eng, const cmd_key *key, size_t sample_count, int force
             float total = 0;
             for (int rep = 0; rep < 3; rep++) {
                 cudaEventRecord(e0, s);
-                const int r = tile ? run_device(eng, key, CMD_PATH_TILE, d_cts, n, d_err, nullptr, s)
-                                   : run_fused_counter(eng, key, d_cts, n, d_err, nullptr, s, eng->tile_counter,
-                                                       nullptr, -1);
+                int r = tile ? run_device(eng, key, CMD_PATH_TILE, d_cts, n, d_err, nullptr, s)
+                             : run_staged(eng, key, d_cts, n, d_err, nullptr, nullptr, s);
+                if (r == CMD_E_BUDGET && !tile)  // what CMD_PATH_AUTO falls back to
+                    r = run_fused_counter(eng, key, d_cts, n, d_err, nullptr, s, eng->tile_counter, nullptr, -1);
                 cudaEventRecord(e1, s);
                 if (r != CMD_OK || cudaEventSynchronize(e1) != cudaSuccess)
                     return 1e30;
@@ -277,7 +275,7 @@ int cmd_tune(cmd_engine *eng, const cmd_key *key, size_t sample_count, int force
         };
         const double tf = timed(false), tt = timed(true);
         if (tt < tf)
-            best.tile_below = (uint32_t)(2 * n);  // the tile kernels still win here
+            best.tile_below = (uint32_t)(2 * n);  // the small-batch kernels still win here
         else
             break;
     }
