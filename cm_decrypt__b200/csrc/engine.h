@@ -46,11 +46,11 @@ struct FusedConfig {
 };
 
 int cuda_fail(cudaError_t e, const char *what);
-// T of the public key [I | T] of a key, from its device support d_L (n
-// entries) and Goppa polynomial d_g (t + 1 coefficients): column c at
-// d_cols[c * cwp ..], cwp >= ceil(mt / 32) words.  CMD_E_ARG when the key's
-// parity-check matrix has no systematic form.  Takes eng->mu.
-int kg_pubkey_columns(cmd_engine *eng, int set, const uint16_t *d_L, const uint16_t *d_g, uint32_t *d_cols, int cwp);
+// T of the public key [I | T] of a key, from its device support d_L (n entries) and
+// Goppa polynomial d_g (t + 1 coefficients): bit i of d_rows[j * rp + r] is column
+// 30 j + i of row r, rp >= mt.  CMD_E_ARG when the key's parity-check matrix has no
+// systematic form.  Takes eng->mu.
+int kg_pubkey_rows(cmd_engine *eng, int set, const uint16_t *d_L, const uint16_t *d_g, uint32_t *d_rows, int rp);
 bool valid_set(int set);
 bool budget_take(cmd_engine *eng, size_t bytes);
 // Device address of GPU-mapped host memory [h, h + bytes) (2-byte aligned,
@@ -143,7 +143,7 @@ struct cmd_key {
     cmd::KeyDev dev;
     void *block = nullptr;
     size_t bytes = 0;
-    uint32_t *pk = nullptr;  // decapsulation: T block of the public key, column-major
+    uint32_t *pk = nullptr;  // decapsulation: T block of the public key (kg_pubkey_rows)
     size_t pk_bytes = 0;
     std::mutex prep_mu;      // cmd_key_prepare_decap, per key (before eng->mu)
 };

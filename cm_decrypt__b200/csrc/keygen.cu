@@ -37,9 +37,8 @@
 // reference's loop does, so a seed yields the reference's key pair.
 //
 // The same parity-check matrix (from an existing key's support and Goppa
-// polynomial, k_kg_support_key), elimination and a column transpose
-// (k_kg_pk_columns) give the public-key columns that decapsulation checks
-// re-encodings against: kg_pubkey_columns.
+// polynomial, k_kg_support_key) and elimination give the public-key rows that
+// decapsulation checks re-encodings against (k_kg_pk_rows): kg_pubkey_rows.
 //
 // Not all constant-time.  All field arithmetic is table-free: the Goppa
 // polynomial uses a multiply by integer multiplies on operands with holes and
@@ -1063,39 +1062,26 @@ __global__ void k_kg_collect(const uint8_t *__restrict__ work, KgDims d, int K, 
     }
 }
 
-// T's columns from the reduced matrix of slot 0: column c (< n - mt) is bit
-// mt + c of the reduced pivot rows 0 .. mt - 1, word w of it (rows 32w ..
-// 32w + 31) at cols[c * cwp + w]; words from the last row on are zero.  Warp
-// (chunk, w): lane b takes 32 bits of pivot row 32w + b from column mt +
-// 32 chunk on, and 32 ballots turn the 32 x 32 block around.
-__global__ void __launch_bounds__(256) k_kg_pk_columns(const uint8_t *__restrict__ work, KgDims d,
-                                                      uint32_t *__restrict__ cols, int cwp)
+// T's rows from the reduced matrix of slot 0, 30 columns a word: bit i of
+// rows[j * rp + r] is column 30 j + i (< n - mt) of row r; zero past the last
+// column and row.  Thread per word, rows fastest.
+__global__ void __launch_bounds__(256) k_kg_pk_rows(const uint8_t *__restrict__ work, KgDims d,
+                                                   uint32_t *__restrict__ rows, int rp, int nj)
 {
     const PanelInfo *pinfo = reinterpret_cast<const PanelInfo *>(work + d.off_panel);
-    const int xc = d.n - d.mt, chunks = (xc + 31) / 32;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (pinfo->status != KG_OK || warp >= chunks * cwp)
+    const int v = blockIdx.x * blockDim.x + threadIdx.x, j = v / rp, r = v - j * rp;
+    if (pinfo->status != KG_OK || j >= nj)
         return;
-    const int chunk = warp / cwp, w = warp - chunk * cwp, r = 32 * w + lane;
     const uint32_t *mat = reinterpret_cast<const uint32_t *>(work + d.off_mat);
     const uint32_t *prow = reinterpret_cast<const uint32_t *>(work + d.off_prow);
     uint32_t bits = 0;
     if (r < d.mt) {
         const uint32_t *row = mat + (size_t)prow[r] * d.rw;
-        const int b0 = d.mt + 32 * chunk, w0 = b0 >> 5, sh = b0 & 31;
+        const int b0 = d.mt + 30 * j, w0 = b0 >> 5, left = d.n - b0;
         const uint32_t lo = row[w0], hi = w0 + 1 < d.rw ? row[w0 + 1] : 0u;
-        bits = __funnelshift_r(lo, hi, sh);
+        bits = __funnelshift_r(lo, hi, b0 & 31) & ((1u << (left < 30 ? left : 30)) - 1u);
     }
-    uint32_t mine = 0;
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, (bits >> k) & 1u);
-        if (lane == k)
-            mine = bal;
-    }
-    const int c = 32 * chunk + lane;
-    if (c < xc)
-        cols[(size_t)c * cwp + w] = mine;
+    rows[v] = bits;
 }
 
 int set_smem_attr(const void *fn, size_t bytes)
@@ -1106,7 +1092,7 @@ int set_smem_attr(const void *fn, size_t bytes)
 
 }  // namespace
 
-int kg_pubkey_columns(cmd_engine *eng, int set, const uint16_t *d_L, const uint16_t *d_g, uint32_t *d_cols, int cwp)
+int kg_pubkey_rows(cmd_engine *eng, int set, const uint16_t *d_L, const uint16_t *d_g, uint32_t *d_rows, int rp)
 {
     std::lock_guard<std::mutex> lk(eng->mu);
     cudaSetDevice(eng->device);
@@ -1128,8 +1114,8 @@ int kg_pubkey_columns(cmd_engine *eng, int set, const uint16_t *d_L, const uint1
         k_ge_panel<<<1, PANEL_THREADS, 0, s>>>(work, d, p);
         k_ge_apply<<<dim3(1, gy), APPLY_THREADS, apply_smem(d.rw - (p & ~3)), s>>>(work, d, p, rows);
     }
-    const int warps = (d.n - d.mt + 31) / 32 * cwp;
-    k_kg_pk_columns<<<(warps + 7) / 8, 256, 0, s>>>(work, d, d_cols, cwp);
+    const int nj = (d.n - d.mt + 29) / 30;
+    k_kg_pk_rows<<<(nj * rp + 255) / 256, 256, 0, s>>>(work, d, d_rows, rp, nj);
     lc.bump(2 + 2 * (uint64_t)npanels);
     int status = KG_SINGULAR;
     cudaError_t e = cudaGetLastError();
