@@ -200,14 +200,16 @@ struct WarpKeccak {
 constexpr int SPEC = 4;  // attempts of one key expanded ahead (its chain)
 
 // Warp k expands the next SPEC attempts of key keys[k] into its chain:
-// attempt 0 from seeds[k] when given, else from the last 32 bytes of the
-// key's previous chain entry Dprev - 1 (the seed the reference's loop moves
+// attempt 0 from seeds[k] when given, else from the last 32 bytes of entry Dprev
+// - 1 of the key's previous chain, in `from` (the seed the reference's loop moves
 // on to after a rejected attempt); attempt j + 1 from attempt j's last 32
 // bytes.  Chain entry j of key `out` is chain + (out * SPEC + j) * r_stride,
-// its seed chain_seed + (out * SPEC + j) * 32.
+// its seed chain_seed + (out * SPEC + j) * 32.  A set *stop ends it early: every
+// key is finished and the chain will not be read.
 __global__ void __launch_bounds__(32) k_kg_expand(const uint8_t *__restrict__ seeds, const int *__restrict__ keys,
-                                                  uint8_t *__restrict__ chain, uint8_t *__restrict__ chain_seed,
-                                                  KgDims d, int K, int Dprev, size_t r_stride)
+                                                  const uint8_t *from, uint8_t *chain,
+                                                  uint8_t *__restrict__ chain_seed, KgDims d, int K, int Dprev,
+                                                  size_t r_stride, const volatile int *stop)
 {
     const int k = blockIdx.x, lane = threadIdx.x;
     if (k >= K)
@@ -217,7 +219,8 @@ __global__ void __launch_bounds__(32) k_kg_expand(const uint8_t *__restrict__ se
     const int out = keys[k];
     uint8_t *base = chain + (size_t)out * SPEC * r_stride;
     // this lane's byte of the first seed, read before the chain is rewritten
-    uint8_t sb = seeds ? seeds[(size_t)k * 32 + lane] : base[(size_t)(Dprev - 1) * r_stride + d.rlen - 32 + lane];
+    uint8_t sb = seeds ? seeds[(size_t)k * 32 + lane]
+                       : from[((size_t)out * SPEC + Dprev - 1) * r_stride + d.rlen - 32 + lane];
     __syncwarp();
     for (int j = 0; j < SPEC; j++) {
         uint8_t *r = base + (size_t)j * r_stride;
@@ -245,7 +248,10 @@ __global__ void __launch_bounds__(32) k_kg_expand(const uint8_t *__restrict__ se
             a = 0;
 #pragma unroll 1
         for (int off = 0; off < d.rlen; off += RATE) {
+            const int ended = *stop;  // back by the end of the permutation
             a = kc.permute(a);
+            if (__any_sync(0xFFFFFFFFu, ended))
+                return;
             const int len = min(RATE, d.rlen - off);
             if (lane < RATE / 8) {
                 if (8 * lane + 8 <= len) {
@@ -443,9 +449,11 @@ __device__ void genpoly_body(uint8_t *eb, uint8_t *smem, const KgDims &d, size_t
 }
 
 __global__ void __launch_bounds__(GP_THREADS) k_kg_genpoly(uint8_t *__restrict__ chain, const int *__restrict__ keys,
-                                                           KgDims d, size_t r_stride)
+                                                           KgDims d, size_t r_stride, const volatile int *stop)
 {
     extern __shared__ __align__(16) uint8_t sm_gp[];
+    if (__syncthreads_or(*stop))
+        return;
     uint8_t *eb = chain + ((size_t)keys[blockIdx.x / SPEC] * SPEC + blockIdx.x % SPEC) * r_stride;
     const size_t r_al = (d.rlen + 255) / 256 * 256;
     if (d.m == 12)
@@ -1162,9 +1170,13 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
     const size_t fixed = 2048 + chain_bytes;
     // per slot: workspace, seed, collect record, list entry, one pk and sk
     auto need = [&](size_t c) { return fixed + c * (d.stride + 32 + 36 + 4 + pk_bytes + d.sk); };
-    while (cap > 1 && eng->keygen.reserve(eng, need(cap)) != CMD_OK)
+    // Few keys (every round takes all SPEC attempts of each): two sets of chains,
+    // so that the expansions, the longest serial part, never wait for a round: a
+    // chain takes 2.5 ms and its polynomials 0.9 ms, a round of 32 slots 2.2 ms.
+    const bool ahead = count * SPEC <= cap && eng->keygen.reserve(eng, need(cap) + 512 + chain_bytes) == CMD_OK;
+    while (!ahead && cap > 1 && eng->keygen.reserve(eng, need(cap)) != CMD_OK)
         cap /= 2;
-    if (cap == 1 && eng->keygen.reserve(eng, need(1)) != CMD_OK)
+    if (!ahead && cap == 1 && eng->keygen.reserve(eng, need(1)) != CMD_OK)
         return CMD_E_BUDGET;
     uint8_t *mem = static_cast<uint8_t *>(eng->keygen.ptr);
     uint8_t *d_work = mem;
@@ -1177,6 +1189,13 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
     int *d_list = reinterpret_cast<int *>(d_col + cap * 9);
     uint8_t *d_pk = reinterpret_cast<uint8_t *>(d_list + cap);
     uint8_t *d_sk = d_pk + cap * pk_bytes;
+    // set when all keys are done
+    int *d_stop = reinterpret_cast<int *>(mem + (static_cast<size_t>(d_sk + cap * d.sk - mem) + 255) / 256 * 256);
+    // the other set of chains (entries start on 256-byte boundaries) and key list
+    uint8_t *d_more = reinterpret_cast<uint8_t *>(d_stop) + 256;
+    uint8_t *chains[2] = {d_chain, ahead ? d_more : d_chain};
+    uint8_t *chain_seeds[2] = {d_chain_seed, ahead ? d_more + count * SPEC * r_stride : d_chain_seed};
+    int *key_lists[2] = {d_keys, ahead ? reinterpret_cast<int *>(chain_seeds[1] + count * SPEC * 32) : d_keys};
     cudaStream_t s = eng->stream;
     LaunchCounter lc{&eng->launches};
     int rc = CMD_OK;
@@ -1188,14 +1207,32 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
         return rc;
     // s2: the next chains (expansion, Goppa polynomial); s3: the copies of
     // finished key pairs to the host, overlapping the next round on s
-    cudaStream_t s2 = nullptr, s3 = nullptr;
-    cudaEvent_t ev_fill = nullptr, ev_exp = nullptr, ev_out = nullptr, ev_copied = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking);
-    if (e == cudaSuccess)
-        e = cudaStreamCreateWithFlags(&s3, cudaStreamNonBlocking);
-    for (cudaEvent_t *ev : {&ev_fill, &ev_exp, &ev_out, &ev_copied})
+    // (s4: with two sets of chains, the Goppa polynomials, beside the next expansion)
+    cudaStream_t s2 = nullptr, s3 = nullptr, s4 = nullptr;
+    cudaEvent_t ev_fill = nullptr, ev_chain = nullptr, ev_exp[2] = {}, ev_out = nullptr, ev_copied = nullptr;
+    cudaError_t e = cudaSuccess;
+    for (cudaStream_t *st : {&s2, &s3, &s4})
+        if (e == cudaSuccess)
+            e = cudaStreamCreateWithFlags(st, cudaStreamNonBlocking);
+    for (cudaEvent_t *ev : {&ev_fill, &ev_chain, &ev_exp[0], &ev_exp[1], &ev_out, &ev_copied})
         if (e == cudaSuccess)
             e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    // Chain set b: the next attempts of K keys, after entry Dprev - 1 of set b0
+    // (or from the seeds); ev_exp[b] marks it complete.
+    auto next_chain = [&](int b, int b0, const uint8_t *from_seeds, const int *kd, int K, int Dprev) {
+        k_kg_expand<<<K, 32, 0, s2>>>(from_seeds, kd, chains[b0], chains[b], chain_seeds[b], d, K, Dprev, r_stride,
+                                      d_stop);
+        cudaStream_t sg = s2;
+        cudaError_t err = cudaSuccess;
+        if (ahead) {
+            sg = s4;
+            if ((err = cudaEventRecord(ev_chain, s2)) == cudaSuccess)
+                err = cudaStreamWaitEvent(s4, ev_chain);
+        }
+        k_kg_genpoly<<<K * SPEC, GP_THREADS, smem_gp, sg>>>(chains[b], kd, d, r_stride, d_stop);
+        lc.bump(2);
+        return err == cudaSuccess ? cudaEventRecord(ev_exp[b], sg) : err;
+    };
     // every key's first chain, from its seed
     std::vector<int> keys(count);
     for (size_t i = 0; i < count; i++)
@@ -1203,13 +1240,15 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_seeds, h_seeds, count * 32, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_keys, keys.data(), count * 4, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) {
-        k_kg_expand<<<(int)count, 32, 0, s>>>(d_seeds, d_keys, d_chain, d_chain_seed, d, (int)count, 0, r_stride);
-        k_kg_genpoly<<<(int)(count * SPEC), GP_THREADS, smem_gp, s>>>(d_chain, d_keys, d, r_stride);
-        lc.bump(2);
-        e = cudaEventRecord(ev_exp, s);
-    }
+        e = cudaMemcpyAsync(key_lists[1], keys.data(), count * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(d_stop, 0, 4, s);
+    if (e == cudaSuccess && (e = cudaEventRecord(ev_fill, s)) == cudaSuccess)
+        e = cudaStreamWaitEvent(s2, ev_fill);
+    if (e == cudaSuccess)
+        e = next_chain(0, 0, d_seeds, key_lists[1], (int)count, 0);
+    if (e == cudaSuccess && ahead)
+        e = next_chain(1, 0, nullptr, key_lists[1], (int)count, SPEC);
     // keys still to finish, by output index
     std::vector<int> pend(count);
     std::vector<uint32_t> tries(count, 0);
@@ -1217,28 +1256,29 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
         pend[i] = (int)i;
     std::vector<uint32_t> col;
     std::vector<int> list, list_out;
-    while (!pend.empty() && e == cudaSuccess && rc == CMD_OK) {
+    for (int round = 0; !pend.empty() && e == cudaSuccess && rc == CMD_OK; round++) {
+        const int b = ahead ? round & 1 : 0;
         std::vector<int> still;
         const size_t keys_per_chunk = std::min(pend.size(), cap);
         const int D = (int)std::max<size_t>(1, std::min<size_t>(SPEC, cap / keys_per_chunk));
         for (size_t base = 0; base < pend.size() && e == cudaSuccess && rc == CMD_OK; base += keys_per_chunk) {
             const int K = (int)std::min(keys_per_chunk, pend.size() - base), S = K * D;
-            // the chains this chunk reads are complete (every expansion so far
-            // is on s2 before ev_exp); the key list goes to a free region
-            int *kd = d_keys + base;
-            if ((e = cudaStreamWaitEvent(s, ev_exp, 0)) != cudaSuccess ||
+            // the chains this chunk reads are complete (with one set, every
+            // expansion so far is on s2 before ev_exp); the key list goes to a
+            // free region
+            int *kd = key_lists[b] + base;
+            if ((e = cudaStreamWaitEvent(s, ev_exp[b], 0)) != cudaSuccess ||
                 (e = cudaMemcpyAsync(kd, pend.data() + base, (size_t)K * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
                 break;
-            k_kg_fill<<<S, 256, 0, s>>>(d_chain, d_chain_seed, kd, d_work, d_slot_seed, d, D, r_stride);
-            // next chains of these keys (attempts D .. D + SPEC - 1 from now),
-            // overlapping the stages below
+            k_kg_fill<<<S, 256, 0, s>>>(chains[b], chain_seeds[b], kd, d_work, d_slot_seed, d, D, r_stride);
+            lc.bump();
+            // next chains of these keys (attempts D .. D + SPEC - 1 from now; with
+            // two sets, the SPEC after those of the other set), overlapping the
+            // stages below
             if ((e = cudaEventRecord(ev_fill, s)) != cudaSuccess || (e = cudaStreamWaitEvent(s2, ev_fill, 0)) != cudaSuccess)
                 break;
-            k_kg_expand<<<K, 32, 0, s2>>>(nullptr, kd, d_chain, d_chain_seed, d, K, D, r_stride);
-            k_kg_genpoly<<<K * SPEC, GP_THREADS, smem_gp, s2>>>(d_chain, kd, d, r_stride);
-            if ((e = cudaEventRecord(ev_exp, s2)) != cudaSuccess)
+            if ((e = next_chain(b, ahead ? 1 - b : 0, nullptr, kd, K, D)) != cudaSuccess)
                 break;
-            lc.bump(3);
             k_kg_support<<<S, SUP_THREADS, smem_sup, s>>>(d_work, d);
             const int npanels = (d.mt + PANEL - 1) / PANEL;
             // rows per update block: about two blocks per SM over the round's slots
@@ -1311,16 +1351,19 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
     if (h_attempts)
         for (size_t i = 0; i < count; i++)
             h_attempts[i] = tries[i];
-    // the last speculative chains may still run on s2, the last copies on s3
-    for (cudaStream_t st : {s3, s2}) {
+    // the last speculative chains may still run on s2 and s4 (they stop at their
+    // next permutation), the last copies on s3
+    if (s2 && d_stop)
+        cudaMemsetAsync(d_stop, 1, 4, s);
+    for (cudaStream_t st : {s3, s2, s4}) {
         const cudaError_t e2 = st ? cudaStreamSynchronize(st) : cudaSuccess;
         if (e == cudaSuccess)
             e = e2;
     }
-    for (cudaEvent_t ev : {ev_fill, ev_exp, ev_out, ev_copied})
+    for (cudaEvent_t ev : {ev_fill, ev_chain, ev_exp[0], ev_exp[1], ev_out, ev_copied})
         if (ev)
             cudaEventDestroy(ev);
-    for (cudaStream_t st : {s2, s3})
+    for (cudaStream_t st : {s2, s3, s4})
         if (st)
             cudaStreamDestroy(st);
     if (e != cudaSuccess)
