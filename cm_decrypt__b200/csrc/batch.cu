@@ -179,6 +179,129 @@ void plan_mixed(const int *key_set, size_t nkeys, const uint32_t *key_idx, size_
                      [&](const FusedTile &x, const FusedTile &y) { return cost(x) > cost(y); });
 }
 
+// A mixed batch on the staged kernels, set by set: slots grouped by key, each key's
+// run cut into tiles and syndrome blocks.
+struct StagedPlan {
+    std::vector<uint32_t> order;
+    std::vector<StagedPiece> blocks, tiles;  // of all sets, set by set
+    uint32_t block0[NSETS + 1] = {}, tile0[NSETS + 1] = {};
+};
+
+static void plan_staged(const int *key_set, size_t nkeys, const uint32_t *key_idx, size_t count, StagedPlan &p)
+{
+    std::vector<uint32_t> cnt(nkeys + 1, 0);
+    for (size_t c = 0; c < count; c++)
+        cnt[key_idx[c] + 1]++;
+    for (size_t k = 0; k < nkeys; k++)
+        cnt[k + 1] += cnt[k];
+    p.order.resize(count);
+    std::vector<uint32_t> fill(cnt.begin(), cnt.end() - 1);
+    for (size_t c = 0; c < count; c++)
+        p.order[fill[key_idx[c]]++] = (uint32_t)c;
+    constexpr uint32_t bs = 32 * staged_block_tiles;
+    for (int st = 0; st < NSETS; st++) {
+        for (size_t k = 0; k < nkeys; k++) {
+            if (key_set[k] != st)
+                continue;
+            for (uint32_t r = cnt[k]; r < cnt[k + 1]; r += 32) {
+                const uint32_t left = cnt[k + 1] - r, tile = (uint32_t)p.tiles.size() - p.tile0[st];
+                if ((r - cnt[k]) % bs == 0)
+                    p.blocks.push_back(StagedPiece{(uint32_t)k, std::min(left, bs), r, tile});
+                p.tiles.push_back(StagedPiece{(uint32_t)k, std::min(left, 32u), r, 0});
+            }
+        }
+        p.block0[st + 1] = (uint32_t)p.blocks.size();
+        p.tile0[st + 1] = (uint32_t)p.tiles.size();
+    }
+}
+
+static size_t al256(size_t x) { return (x + 255) / 256 * 256; }
+
+// CMD_E_BUDGET: nothing ran, the fused kernel has to.  Caller holds eng->mu.
+static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t nkeys, const int *key_set,
+                            const uint32_t *h_key_idx, const uint8_t *d_cts, const uint64_t *h_ct_off, size_t count,
+                            uint32_t *d_err, const uint64_t *h_err_off, uint16_t *d_weight, cudaStream_t s)
+{
+    StagedPlan p;
+    plan_staged(key_set, nkeys, h_key_idx, count, p);
+    std::vector<FusedKeyRef> krefs(nkeys);
+    for (size_t k = 0; k < nkeys; k++)
+        krefs[k] = key_ref(keys[k]->dev);
+    const size_t b_order = al256(count * 4), b_off = al256(count * 8), b_blk = al256(p.blocks.size() * sizeof(StagedPiece)),
+                 b_tile = al256(p.tiles.size() * sizeof(StagedPiece)), b_keys = al256(nkeys * sizeof(FusedKeyRef));
+    size_t words[NSETS + 1] = {};
+    for (int st = 0; st < NSETS; st++)
+        words[st + 1] = words[st] + staged_scratch_words(st, 32 * (size_t)(p.tile0[st + 1] - p.tile0[st]));
+    if (eng->fused.reserve(eng, b_order + 2 * b_off + b_blk + b_tile + b_keys) != CMD_OK)
+        return CMD_E_BUDGET;
+    int rc = staged_begin(eng, words[NSETS] * 4, 1, s);  // the lists follow the previous batch's reads, too
+    if (rc)
+        return rc;
+    uint8_t *at = static_cast<uint8_t *>(eng->fused.ptr);
+    cudaError_t e = cudaSuccess;
+    auto put = [&](const void *src, size_t bytes, size_t room) {
+        uint8_t *dst = at;
+        at += room;
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+        return dst;
+    };
+    StagedMixed mx;
+    mx.order = reinterpret_cast<const uint32_t *>(put(p.order.data(), count * 4, b_order));
+    mx.ct_off = reinterpret_cast<const uint64_t *>(put(h_ct_off, count * 8, b_off));
+    mx.err_off = reinterpret_cast<const uint64_t *>(put(h_err_off, count * 8, b_off));
+    mx.blocks = reinterpret_cast<const StagedPiece *>(put(p.blocks.data(), p.blocks.size() * sizeof(StagedPiece), b_blk));
+    mx.tiles = reinterpret_cast<const StagedPiece *>(put(p.tiles.data(), p.tiles.size() * sizeof(StagedPiece), b_tile));
+    mx.keys = reinterpret_cast<const FusedKeyRef *>(put(krefs.data(), nkeys * sizeof(FusedKeyRef), b_keys));
+    if (e != cudaSuccess)
+        return staged_end(eng, 1, s, e);
+    // the sets beside one another, as the parts of a single-key batch
+    const int ns = STAGED_STREAMS;
+    if ((rc = staged_begin(eng, words[NSETS] * 4, ns, s)))
+        return rc;
+    for (int st = NSETS - 1, i = 0; st >= 0 && e == cudaSuccess; st--) {  // the costlier sets first
+        const uint32_t nb = p.block0[st + 1] - p.block0[st], nt = p.tile0[st + 1] - p.tile0[st];
+        if (nt == 0)
+            continue;
+        StagedMixed m = mx;
+        m.blocks += p.block0[st];
+        m.tiles += p.tile0[st];
+        e = launch_staged_mixed(st, m, nb, nt, d_cts, static_cast<uint32_t *>(eng->staged.ptr) + words[st], d_err,
+                                d_weight, eng->fft[st], eng->num_sms, eng->piece_stream[i++ % ns],
+                                LaunchCounter{&eng->launches});
+    }
+    return staged_end(eng, ns, s, e);
+}
+
+// A small mixed batch on the per-ciphertext kernels.  CMD_E_BUDGET as above, also
+// when an offset does not fit an item.
+static int run_mixed_small(cmd_engine *eng, const cmd_key *const *keys, const uint32_t *h_key_idx, const uint8_t *d_cts,
+                           const uint64_t *h_ct_off, size_t count, uint32_t *d_err, const uint64_t *h_err_off,
+                           uint16_t *d_weight, cudaStream_t s)
+{
+    std::vector<LatItem> items(count);
+    for (size_t c = 0; c < count; c++) {
+        if ((h_ct_off[c] | h_err_off[c]) >> 32)
+            return CMD_E_BUDGET;
+        const KeyDev &k = keys[h_key_idx[c]]->dev;
+        items[c] = LatItem{k.wfft, k.bctl, (uint32_t)h_ct_off[c], (uint32_t)h_err_off[c], k.set, 0, nullptr};
+    }
+    const size_t b_items = al256(count * sizeof(LatItem)), b_mid = count > CT_ONE_LAUNCH ? count * 512 : 0;
+    int rc = staged_begin(eng, b_items + b_mid, 1, s);
+    if (rc)
+        return rc;
+    uint8_t *base = static_cast<uint8_t *>(eng->staged.ptr);
+    cudaError_t e = cudaMemcpyAsync(base, items.data(), count * sizeof(LatItem), cudaMemcpyHostToDevice, s);
+    FftPlans plans;
+    for (int st = 0; st < NSETS; st++)
+        plans.p[st] = eng->fft[st];
+    if (e == cudaSuccess)
+        e = launch_ct_items(reinterpret_cast<const LatItem *>(base), d_cts, (uint32_t)count, (uint32_t)count,
+                            reinterpret_cast<uint16_t *>(base + b_items), d_err, d_weight, nullptr, plans, eng->num_sms,
+                            s, LaunchCounter{&eng->launches});
+    return staged_end(eng, 1, s, e);
+}
+
 int fused_grid(cmd_engine *eng, int single_set, int wpb, size_t smem, uint64_t rounds)
 {
     return grid_for(eng, single_set, wpb, smem, rounds);
@@ -218,6 +341,25 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
     std::vector<int> kset(nkeys);
     for (size_t k = 0; k < nkeys; k++)
         kset[k] = keys[k]->dev.set;
+    // As run_auto (engine.cu): per-ciphertext kernels up to 24 an SM, then the staged
+    // ones; the fused kernel for about one round of its warps, when their scratch
+    // does not fit and under stream capture.  64 keys on a B200, fused -> taken:
+    // 300 ciphertexts 985 -> 145 us, 1,000 1,271 -> 231 us, 10,000 1,797 -> 1,272 us,
+    // 20,000 1,843 -> 1,653 us, 100,000 4,088 -> 3,829 us; 40,000 1,910 us (staged
+    // 2,023 us).
+    std::lock_guard<std::mutex> lk(eng->mu);
+    const size_t sms = (size_t)eng->num_sms;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!(count > 192 * sms && count <= 320 * sms) && cudaStreamIsCapturing(s, &cap) == cudaSuccess &&
+        cap == cudaStreamCaptureStatusNone) {
+        const int r = count <= CT_PER_SM * sms
+                          ? run_mixed_small(eng, keys, h_key_idx, d_cts, h_ct_off, count, d_err, h_err_off, d_weight, s)
+                          : run_mixed_staged(eng, keys, nkeys, kset.data(), h_key_idx, d_cts, h_ct_off, count, d_err,
+                                             h_err_off, d_weight, s);
+        if (r != CMD_E_BUDGET)
+            return r;
+    }
+    cudaGetLastError();
     int single = mixed_single_set(kset.data(), h_key_idx, count);
     const int wpb = single >= 0 ? eng->fcfg[single].wpb : eng->fcfg_mixed.wpb;
     std::vector<uint32_t> order;
@@ -227,7 +369,6 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
     for (size_t k = 0; k < nkeys; k++)
         krefs[k] = key_ref(keys[k]->dev);
 
-    std::lock_guard<std::mutex> lk(eng->mu);
     int rc = 0;
     if ((rc = [&] {
             if (eng->tile_counter)

@@ -496,13 +496,9 @@ static size_t staged_part(size_t count)
     return ((count + parts - 1) / parts + 31) / 32 * 32;
 }
 
-int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-               uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
+int staged_begin(cmd_engine *eng, size_t bytes, int ns, cudaStream_t s)
 {
-    const SetInfo si = set_info(key->dev.set);
-    const size_t part = staged_part(count), nparts = (count + part - 1) / part;
-    const size_t ns = std::min<size_t>(nparts, STAGED_STREAMS), words = staged_scratch_words(key->dev.set, part);
-    int rc = eng->staged.reserve(eng, ns * words * 4);
+    int rc = eng->staged.reserve(eng, bytes);
     if (rc || (rc = ensure_piece_streams(eng)))
         return rc;
     cudaError_t e = cudaSuccess;
@@ -519,20 +515,16 @@ int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t
         // the scratch may still be in use by a batch on another stream
         e = cudaStreamWaitEvent(s, eng->staged_done);
     }
-    if (e == cudaSuccess && ns > 1) {
+    if (e == cudaSuccess && ns > 1)
         e = cudaEventRecord(eng->staged_fork, s);
-        for (size_t i = 0; i < ns && e == cudaSuccess; i++)
-            e = cudaStreamWaitEvent(eng->piece_stream[i], eng->staged_fork);
-    }
-    for (size_t p = 0; p < nparts && e == cudaSuccess; p++) {
-        const size_t c0 = p * part, n = std::min(part, count - c0), i = p % ns;
-        e = launch_staged(key->dev, d_cts + c0 * si.ct, (uint32_t)n,
-                          static_cast<uint32_t *>(eng->staged.ptr) + i * words, d_err ? d_err + c0 * si.nw : nullptr,
-                          d_weight ? d_weight + c0 : nullptr, d_pos ? d_pos + c0 * (si.t + 1) : nullptr, nullptr,
-                          eng->fft[key->dev.set], eng->num_sms, ns > 1 ? eng->piece_stream[i] : s,
-                          LaunchCounter{&eng->launches});
-    }
-    for (size_t i = 0; i < ns && ns > 1; i++) {  // joined even after an error
+    for (int i = 0; i < ns && ns > 1 && e == cudaSuccess; i++)
+        e = cudaStreamWaitEvent(eng->piece_stream[i], eng->staged_fork);
+    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "staged batch");
+}
+
+int staged_end(cmd_engine *eng, int ns, cudaStream_t s, cudaError_t e)
+{
+    for (int i = 0; i < ns && ns > 1; i++) {  // joined even after an error
         cudaError_t e2 = cudaEventRecord(eng->staged_join[i], eng->piece_stream[i]);
         if (e2 == cudaSuccess)
             e2 = cudaStreamWaitEvent(s, eng->staged_join[i]);
@@ -543,6 +535,26 @@ int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t
         e = cudaEventRecord(eng->staged_done, s);
     eng->staged_last = s;
     return e == cudaSuccess ? CMD_OK : cuda_fail(e, "staged batch");
+}
+
+int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
+               uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
+{
+    const SetInfo si = set_info(key->dev.set);
+    const size_t part = staged_part(count), nparts = (count + part - 1) / part;
+    const size_t ns = std::min<size_t>(nparts, STAGED_STREAMS), words = staged_scratch_words(key->dev.set, part);
+    if (const int rc = staged_begin(eng, ns * words * 4, (int)ns, s))
+        return rc;
+    cudaError_t e = cudaSuccess;
+    for (size_t p = 0; p < nparts && e == cudaSuccess; p++) {
+        const size_t c0 = p * part, n = std::min(part, count - c0), i = p % ns;
+        e = launch_staged(key->dev, d_cts + c0 * si.ct, (uint32_t)n,
+                          static_cast<uint32_t *>(eng->staged.ptr) + i * words, d_err ? d_err + c0 * si.nw : nullptr,
+                          d_weight ? d_weight + c0 : nullptr, d_pos ? d_pos + c0 * (si.t + 1) : nullptr, nullptr,
+                          eng->fft[key->dev.set], eng->num_sms, ns > 1 ? eng->piece_stream[i] : s,
+                          LaunchCounter{&eng->launches});
+    }
+    return staged_end(eng, (int)ns, s, e);
 }
 
 // Whether CMD_PATH_AUTO takes the small-batch kernels: batches within the

@@ -70,6 +70,11 @@ int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, 
 // pos, each or null.  CMD_E_BUDGET when their scratch does not fit.
 int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s);
+// Around staged launches on s (ns = 1) or on the first ns piece streams: reserves
+// the scratch, orders it after its last use on another stream, forks; joins (also
+// after an error e) and marks the scratch's use.
+int staged_begin(cmd_engine *eng, size_t bytes, int ns, cudaStream_t s);
+int staged_end(cmd_engine *eng, int ns, cudaStream_t s, cudaError_t e);
 // Explicit work counter and round schedule (balanced: -1 = the tuned choice,
 // 0 = full rounds, 1 = equal shares; round_cts > 0 overrides all three with
 // rounds of that many ciphertexts, a multiple of 32 from fused_round).

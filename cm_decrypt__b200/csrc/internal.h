@@ -125,6 +125,26 @@ cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count,
                           uint16_t *d_weight, uint16_t *d_pos, uint8_t *err_packed, const FftPlanDev &plan,
                           int num_sms, cudaStream_t s, LaunchCounter lc);
 size_t staged_scratch_words(int set, size_t count);
+// The same for the ciphertexts of one set in a mixed batch: `blocks` and `tiles`
+// cut the slots of `order` (a key's slots contiguous) into syndrome blocks of up
+// to staged_block_tiles tiles and tiles of up to 32 slots, each of one key.
+struct StagedPiece {
+    uint32_t key;    // index into keys
+    uint32_t count;  // slots
+    uint32_t first;  // first slot
+    uint32_t tile0;  // blocks: their first tile
+};
+struct StagedMixed {
+    const StagedPiece *blocks = nullptr, *tiles = nullptr;
+    const FusedKeyRef *keys = nullptr;
+    const uint32_t *order = nullptr;    // ciphertext index of a slot
+    const uint64_t *ct_off = nullptr;   // by ciphertext: bytes
+    const uint64_t *err_off = nullptr;  // words
+};
+constexpr uint32_t staged_block_tiles = 8;
+cudaError_t launch_staged_mixed(int set, const StagedMixed &mx, uint32_t nblocks, uint32_t ntiles,
+                                const uint8_t *d_cts, uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight,
+                                const FftPlanDev &plan, int num_sms, cudaStream_t s, LaunchCounter lc);
 
 // Latency path (serving loop; latency.cu): one work item per ciphertext.
 struct LatItem {

@@ -1,4 +1,5 @@
-// Staged decrypt of one key's batch: the fused kernel's phases as four kernels,
+// Staged decrypt of one key's batch, or of a mixed batch set by set (MIX below:
+// the slots of a tile belong to one key): the fused kernel's phases as four kernels,
 // each with the block shape, shared memory and code size that its phase wants.
 //
 //   k_synd_table  the 2t syndromes (util.c:102-114) from the key's dense table,
@@ -74,10 +75,10 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src)
 // blockDim.x = 32 * SPLIT * (tiles per block): SPLIT warps share the syndrome
 // words of a tile: 8 up to two tiles an SM, 4 up to four, where a warp's time per
 // group counts (4,736 ciphertexts: 452 us with one warp a tile, 137 us with four).
-template <int S, int SPLIT>
+template <int S, int SPLIT, bool MIX = false>
 __global__ void __launch_bounds__(SYND_WARPS * 32, 1) k_synd_table(const uint32_t *__restrict__ tab,
                                                                    const uint8_t *__restrict__ cts, uint32_t count,
-                                                                   uint32_t *__restrict__ tiles)
+                                                                   uint32_t *__restrict__ tiles, StagedMixed mx)
 {
     using Z = SgDims<S>;
     using P = Set<S>;
@@ -89,8 +90,15 @@ __global__ void __launch_bounds__(SYND_WARPS * 32, 1) k_synd_table(const uint32_
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
     const int part = (tid >> 5) % SPLIT, mine = (tid >> 5) / SPLIT * 32 + lane;  // ciphertext in the block
     const int nct = nt / SPLIT;                                                  // ciphertexts of a block
-    const uint64_t first = (uint64_t)blockIdx.x * nct;
-    const int live = (int)(count - first < (uint64_t)nct ? count - first : nct);
+    uint64_t first = (uint64_t)blockIdx.x * nct, tile0 = first / 32;
+    int live = (int)(count - first < (uint64_t)nct ? count - first : nct);
+    if constexpr (MIX) {
+        const StagedPiece blk = mx.blocks[blockIdx.x];
+        tab = mx.keys[blk.key].tab;
+        first = blk.first;
+        tile0 = blk.tile0;
+        live = (int)blk.count;
+    }
 
     constexpr int AHEAD = Z::ROW_BUFS - 2;  // group g's additions, g + 1's combinations, the rest in flight
     auto stage = [&](int g) {  // rows of group g, zero past the last one
@@ -128,9 +136,18 @@ __global__ void __launch_bounds__(SYND_WARPS * 32, 1) k_synd_table(const uint32_
 
     for (int g = 0; g < AHEAD; g++)
         stage(g);
-    {   // the block's ciphertexts: 16-bit loads (every set's length is even)
+    uint16_t *dst16 = reinterpret_cast<uint16_t *>(raw);
+    if constexpr (MIX) {  // a ciphertext starts at any byte
+        for (int q = tid >> 5; q < live; q += nt >> 5) {
+            const uint8_t *src = cts + mx.ct_off[mx.order[first + q]];
+            for (int v = lane; v < P::CT; v += 32)
+                raw[q * P::CT + v] = __ldg(src + v);
+        }
+        for (int v = live * P::CT / 2 + tid; v < nct * P::CT / 2 + 4; v += nt)
+            dst16[v] = 0;
+    } else {  // the block's ciphertexts: 16-bit loads (every set's length is even)
         const uint16_t *src = reinterpret_cast<const uint16_t *>(cts + first * P::CT);
-        uint16_t *dst = reinterpret_cast<uint16_t *>(raw);
+        uint16_t *dst = dst16;
         if (((uintptr_t)src & 15) == 0) {
             const int n = live * P::CT / 16;
             for (int v = tid; v < n; v += nt)
@@ -175,8 +192,9 @@ __global__ void __launch_bounds__(SYND_WARPS * 32, 1) k_synd_table(const uint32_
     }
     // transpose to bitsliced syndromes (bit q = ciphertext q of the tile), as in
     // the fused kernel: word x = j*m + k goes to row j
-    const uint64_t tile = first / 32 + (tid >> 5) / SPLIT;
-    if (tile * 32 >= count)
+    const int ltile = (tid >> 5) / SPLIT;
+    const uint64_t tile = tile0 + ltile;
+    if (32 * ltile >= live)
         return;
     uint32_t *out = tiles + tile * Z::TILE_WORDS;
     constexpr uint32_t M0[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
@@ -204,7 +222,8 @@ __global__ void __launch_bounds__(SYND_WARPS * 32, 1) k_synd_table(const uint32_
 // latency with fewer; 19 KB of shared memory a tile.
 template <int S, int W>
 __global__ void __launch_bounds__(32 * W) k_bm_tile(uint32_t *__restrict__ tiles, uint32_t count,
-                                                    const uint16_t *__restrict__ scalpow, uint32_t turn_after)
+                                                    const uint16_t *__restrict__ scalpow, uint32_t turn_after,
+                                                    const StagedPiece *__restrict__ pieces)
 {
     using Z = SgDims<S>;
     using B = BmDims<S>;
@@ -214,7 +233,7 @@ __global__ void __launch_bounds__(32 * W) k_bm_tile(uint32_t *__restrict__ tiles
     uint32_t *share = smem_sg, *ring = share + 2 * W * 16, *cm = ring + B::RING_WORDS, *syn = cm + B::C_WORDS;
     uint32_t *cv = ring;  // conversion array: the ring, C and the syndromes are free by then
     uint32_t *io = tiles + (size_t)blockIdx.x * Z::TILE_WORDS;
-    const uint32_t left = count - 32 * blockIdx.x;
+    const uint32_t left = pieces ? pieces[blockIdx.x].count : count - 32 * blockIdx.x;
     bm_tile<S, true, W>(syn, ring, cm, left < 32 ? (int)left : 32, tid, io, share,
                         W == 1 ? 0 : blockIdx.x / turn_after % W);
     // entry x of the conversion array is C[T-x] (bm.c:62-65 reverses the
@@ -240,7 +259,8 @@ __global__ void __launch_bounds__(32 * W) k_bm_tile(uint32_t *__restrict__ tiles
 template <int S>
 __global__ void __launch_bounds__(FFT_WARPS * 32, 3) k_fft_tile(const uint32_t *__restrict__ tiles, uint32_t count,
                                                                 const uint32_t *__restrict__ tw,
-                                                                uint32_t *__restrict__ flags)
+                                                                uint32_t *__restrict__ flags,
+                                                                const StagedPiece *__restrict__ pieces)
 {
     using Z = SgDims<S>;
     constexpr int SS = Z::SS, NX = Z::NX, NWD = Z::NWD, R = FftDims<S>::R;
@@ -252,9 +272,9 @@ __global__ void __launch_bounds__(FFT_WARPS * 32, 3) k_fft_tile(const uint32_t *
     for (int v = threadIdx.x; v < NX * SS; v += FFT_WARPS * 32)
         cv[v] = src[v];
     __syncthreads();
-    const uint32_t c0 = 32 * blockIdx.x;
+    const uint32_t c0 = 32 * blockIdx.x, n = pieces ? pieces[blockIdx.x].count : min(count - c0, 32u);
 #pragma unroll 1
-    for (int q = blockIdx.y * FFT_WARPS + warp; q < 32 && c0 + q < count; q += FFT_WARPS * gridDim.y) {
+    for (int q = blockIdx.y * FFT_WARPS + warp; q < (int)n; q += FFT_WARPS * gridDim.y) {
         uint32_t z[R];
         fft_eval_one<S, SS>(cv, q, fa, tw, lane, z);
 #pragma unroll
@@ -271,11 +291,12 @@ struct NetArgs {
     uint16_t *weight;     // or null
     uint16_t *pos;        // rows of t + 1, or null
     uint8_t *err_packed;  // rows of n/8 bytes, or null
+    StagedMixed mx;       // MIX: count is 32 * tiles, err / weight by ciphertext
 };
 
 // The support network of NC ciphertexts a warp: each layer's mask words are loaded
 // once for all of them (they wait on memory, 25 layers in a row).
-template <int S, int NC> __global__ void __launch_bounds__(NET_WARPS * 32) k_net_rows(NetArgs a)
+template <int S, int NC, bool MIX = false> __global__ void __launch_bounds__(NET_WARPS * 32) k_net_rows(NetArgs a)
 {
     using F = FftDims<S>;
     constexpr int M = F::M, NWD = F::NWD, R = F::R;
@@ -284,7 +305,17 @@ template <int S, int NC> __global__ void __launch_bounds__(NET_WARPS * 32) k_net
     const uint64_t c0 = ((uint64_t)blockIdx.x * NET_WARPS + warp) * NC;
     if (c0 >= a.count)
         return;
-    const int n = (int)(a.count - c0 < NC ? a.count - c0 : NC);
+    int n = (int)(a.count - c0 < NC ? a.count - c0 : NC);
+    const uint32_t *order = nullptr;
+    if constexpr (MIX) {
+        const StagedPiece t = a.mx.tiles[c0 / 32];
+        const int left = (int)t.count - (int)(c0 % 32);
+        n = left < NC ? left : NC;
+        if (n <= 0)
+            return;
+        a.bctl = a.mx.keys[t.key].bctl;
+        order = a.mx.order + t.first + c0 % 32;
+    }
     uint32_t z[NC][R];
 #pragma unroll
     for (int i = 0; i < NC; i++)
@@ -303,8 +334,8 @@ template <int S, int NC> __global__ void __launch_bounds__(NET_WARPS * 32) k_net
 #pragma unroll
         for (int j = 0; j < R; j++)
             v[j] = rows[warp][i * NWD + lane + 32 * j];  // this lane's own words
-        const uint64_t c = c0 + i;
-        const int cnt = root_output<S>(v, a.err ? a.err + c * F::NW : nullptr,
+        const uint64_t c = MIX ? order[i] : c0 + i;
+        const int cnt = root_output<S>(v, a.err ? a.err + (MIX ? a.mx.err_off[c] : c * F::NW) : nullptr,
                                        a.pos ? a.pos + c * (F::T + 1) : nullptr,
                                        a.err_packed ? a.err_packed + c * (F::N / 8) : nullptr, lane);
         if (lane == 0 && a.weight)
@@ -363,11 +394,11 @@ cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count,
             return e;
         const uint32_t threads = bt * 32 * split;
         if (split == 8)
-            k_synd_table<S, 8><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles);
+            k_synd_table<S, 8><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles, {});
         else if (split == 4)
-            k_synd_table<S, 4><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles);
+            k_synd_table<S, 4><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles, {});
         else
-            k_synd_table<S, 1><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles);
+            k_synd_table<S, 1><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles, {});
         // Warps a tile, by tiles an SM: enough that every scheduler has a warp (one
         // tile: four warps 255 us, one 467 us for t = 119), and two to even out the
         // schedulers when they would hold one or two (25,000 ciphertexts in all:
@@ -376,22 +407,59 @@ cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count,
         const int bw = ntiles <= sms ? 4 : ntiles <= 2 * sms ? 2 : ntiles <= 4 * sms ? 1 : ntiles <= 6 * sms ? 2 : 1;
         const size_t bm_smem = 4 * (size_t)(Z::BM_WORDS + 2 * bw * 16);
         if (bw == 4)
-            k_bm_tile<S, 4><<<ntiles, 128, bm_smem, s>>>(tiles, count, plan.scalpow, sms);
+            k_bm_tile<S, 4><<<ntiles, 128, bm_smem, s>>>(tiles, count, plan.scalpow, sms, nullptr);
         else if (bw == 2)
-            k_bm_tile<S, 2><<<ntiles, 64, bm_smem, s>>>(tiles, count, plan.scalpow, 2 * sms);
+            k_bm_tile<S, 2><<<ntiles, 64, bm_smem, s>>>(tiles, count, plan.scalpow, 2 * sms, nullptr);
         else
-            k_bm_tile<S, 1><<<ntiles, 32, bm_smem, s>>>(tiles, count, plan.scalpow, 1);
+            k_bm_tile<S, 1><<<ntiles, 32, bm_smem, s>>>(tiles, count, plan.scalpow, 1, nullptr);
         // enough blocks for three an SM, up to a ciphertext a warp
         uint32_t parts = 1;
         while (parts < 32 / FFT_WARPS && ntiles * parts < 3 * sms)
             parts *= 2;
-        k_fft_tile<S><<<dim3(ntiles, parts), FFT_WARPS * 32, fft_smem, s>>>(tiles, count, plan.tw, flags);
-        const NetArgs na{flags, k.bctl, count, d_err, d_weight, d_pos, err_packed};
+        k_fft_tile<S><<<dim3(ntiles, parts), FFT_WARPS * 32, fft_smem, s>>>(tiles, count, plan.tw, flags, nullptr);
+        const NetArgs na{flags, k.bctl, count, d_err, d_weight, d_pos, err_packed, {}};
         const uint32_t nc = count <= 64 * sms ? 1 : 4, per = NET_WARPS * nc;
         if (nc == 1)
             k_net_rows<S, 1><<<(count + per - 1) / per, NET_WARPS * 32, 0, s>>>(na);
         else
             k_net_rows<S, 4><<<(count + per - 1) / per, NET_WARPS * 32, 0, s>>>(na);
+        lc.bump(4);
+        return cudaGetLastError();
+    });
+}
+
+cudaError_t launch_staged_mixed(int set, const StagedMixed &mx, uint32_t nblocks, uint32_t ntiles,
+                                const uint8_t *d_cts, uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight,
+                                const FftPlanDev &plan, int num_sms, cudaStream_t s, LaunchCounter lc)
+{
+    if (ntiles == 0)
+        return cudaSuccess;
+    return dispatch_set(set, [&]<int S>() -> cudaError_t {
+        using Z = SgDims<S>;
+        constexpr uint32_t bt = staged_block_tiles;
+        const uint32_t sms = (uint32_t)num_sms;
+        uint32_t *tiles = d_scratch, *flags = tiles + (size_t)ntiles * Z::TILE_WORDS;
+        constexpr size_t synd_smem = 4 * (Z::ROW_WORDS + Z::COMB_WORDS) + (size_t)bt * 32 * Set<S>::CT + 16;
+        const size_t bm_smem = 4 * (size_t)(Z::BM_WORDS + 2 * 16);
+        const size_t fft_smem = 4 * (size_t)(Z::NX * Z::SS + FFT_WARPS * FftDims<S>::FA_WORDS);
+        static bool g0[64] = {}, g1[64] = {}, g2[64] = {};
+        const bool split = nblocks < sms;  // more warps a tile, as for one key
+        cudaError_t e;
+        if ((e = allow_smem(k_synd_table<S, 1, true>, synd_smem, g0)) != cudaSuccess ||
+            (e = allow_smem(k_synd_table<S, 2, true>, synd_smem, g1)) != cudaSuccess ||
+            (e = allow_smem(k_fft_tile<S>, fft_smem, g2)) != cudaSuccess)
+            return e;
+        if (split)
+            k_synd_table<S, 2, true><<<nblocks, bt * 64, synd_smem, s>>>(nullptr, d_cts, 0, tiles, mx);
+        else
+            k_synd_table<S, 1, true><<<nblocks, bt * 32, synd_smem, s>>>(nullptr, d_cts, 0, tiles, mx);
+        k_bm_tile<S, 1><<<ntiles, 32, bm_smem, s>>>(tiles, 0, plan.scalpow, 1, mx.tiles);
+        uint32_t parts = 1;
+        while (parts < 32 / FFT_WARPS && ntiles * parts < 3 * sms)
+            parts *= 2;
+        k_fft_tile<S><<<dim3(ntiles, parts), FFT_WARPS * 32, fft_smem, s>>>(tiles, 0, plan.tw, flags, mx.tiles);
+        const NetArgs na{flags, nullptr, 32 * ntiles, d_err, d_weight, nullptr, nullptr, mx};
+        k_net_rows<S, 4, true><<<(ntiles + NET_WARPS / 8 - 1) / (NET_WARPS / 8), NET_WARPS * 32, 0, s>>>(na);
         lc.bump(4);
         return cudaGetLastError();
     });

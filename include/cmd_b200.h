@@ -129,10 +129,10 @@ int cmd_decrypt_device(cmd_engine *eng, const cmd_key *key, cmd_path path,
                        const uint8_t *d_cts, size_t count, uint32_t *d_err,
                        uint16_t *d_weight, void *stream);
 
-/* Mixed batch in one launch: ciphertext c belongs to keys[h_key_idx[c]]; its
+/* Mixed batch in one call: ciphertext c belongs to keys[h_key_idx[c]]; its
  * bytes start at d_cts + h_ct_off[c] and its error row at
  * d_err + h_err_off[c] (in 32-bit words).  Keys may be of different sets.
- * Always runs the fused kernel.  Asynchronous on `stream`. */
+ * Asynchronous on `stream`. */
 int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *keys,
                              size_t nkeys, const uint32_t *h_key_idx,
                              const uint8_t *d_cts, const uint64_t *h_ct_off,

@@ -87,3 +87,43 @@ def test_staged_streams_and_capture(engine):
         assert torch.equal(err, want[:5000])
     finally:
         key.free()
+
+
+def test_mixed_sizes_match_plain(engine):
+    """Mixed batches at the sizes where the kernels change (one launch, three
+    launches, staged), keys of all sets, ciphertexts at odd offsets, against the
+    plain path key by key."""
+    sets = [348864, 460896, 6688128, 6960119, 8192128, 348864, 6960119]
+    keys, pool, want = [], [], []
+    rng = np.random.default_rng(5)
+    try:
+        for i, s in enumerate(sets):
+            sk = cmd.synth_key(s, golden_sk(s), 1000 + i)
+            keys.append(cmd.Key(engine, s, sk))
+            cts, _, _ = cmd.PubKey(s, sk).ciphertexts(seed=50 + i, count=300, malformed_permille=100)
+            pool.append(np.concatenate([degenerate(keys[-1].info), cts]))
+            want.append(cmd.decrypt(engine, keys[-1], pool[-1], path="plain"))
+        for count in (1, 64, 65, 1000, 3552, 3553, 20011):
+            ki = rng.integers(0, len(sets) if count != 65 else 1, count).astype(np.uint32)
+            which = np.array([rng.integers(0, len(pool[k])) for k in ki])
+            sizes = np.array([pool[k].shape[1] for k in ki])
+            off = np.concatenate([[3], 3 + np.cumsum(sizes + 1)]).astype(np.uint64)  # a byte between them
+            buf = np.zeros(int(off[-1]), np.uint8)
+            for c, (k, j) in enumerate(zip(ki, which)):
+                buf[int(off[c]):int(off[c]) + sizes[c]] = pool[k][j]
+            words = np.array([keys[k].info.err_words for k in ki])
+            eoff = np.concatenate([[0], np.cumsum(words)]).astype(np.uint64)
+            d, err = torch.from_numpy(buf).cuda(), torch.full((int(eoff[-1]),), -1, dtype=torch.int32, device="cuda")
+            w = torch.full((count,), -1, dtype=torch.int16, device="cuda")
+            torch.cuda.synchronize()
+            cmd.decrypt_mixed_device(engine, keys, ki, d.data_ptr(), off[:-1], err.data_ptr(), eoff[:-1], w.data_ptr())
+            torch.cuda.synchronize()
+            got, got_w = err.cpu().numpy().view(np.uint8), w.cpu().numpy().view(np.uint16)
+            for c, (k, j) in enumerate(zip(ki, which)):
+                row = got[4 * int(eoff[c]):4 * int(eoff[c + 1])]
+                nb = keys[k].info.err_bytes
+                assert np.array_equal(row[:nb], want[k][0][j]) and not row[nb:].any(), (count, c)
+                assert got_w[c] == want[k][1][j], (count, c)
+    finally:
+        for k in keys:
+            k.free()
