@@ -26,7 +26,8 @@
 //   * the twiddles: the butterfly of depth d pairs positions Y and
 //     Y + 2^(m-d-1); its multiplier a(Y) depends on r = Y mod 2^(m-d-1):
 //     a = sum_j bit(m-d-2-j of r) * G_{j+2}, stored bitsliced, 32 values r
-//     per word, plane-major (plane 0 of all depths, then plane 1, ...).
+//     per word, plane-major (plane 0 of all depths, then plane 1, ...), then the
+//     half sums of the butterflies' Karatsuba products: plane k + plane k + (m+1)/2.
 #include <cstring>
 #include <vector>
 
@@ -62,7 +63,7 @@ uint32_t finv(uint32_t a, int m)
 struct FftPlanHost {
     int D = 0;
     std::vector<uint16_t> scalpow;  // [8][256]
-    std::vector<uint32_t> tw;       // [m][2^(m-5)], a plane's depths one after the other
+    std::vector<uint32_t> tw;       // [m + m/2][2^(m-5)], a plane's depths one after the other
 };
 
 FftPlanHost make_fft_plan(int set)
@@ -73,7 +74,8 @@ FftPlanHost make_fft_plan(int set)
     p.D = synd_depth(si.t);
     p.scalpow.assign(8 * 256, 0);
     const int plane = 1 << (m - 5);  // at least the sum of all depths' words
-    p.tw.assign((size_t)m * plane, 0);
+    const int half = (m + 1) / 2, sums = m - half;  // planes k + half added to planes k < sums
+    p.tw.assign((size_t)(m + sums) * plane, 0);
     int base = 0;
     std::vector<uint32_t> B(m);
     for (int j = 0; j < m; j++)
@@ -105,6 +107,8 @@ FftPlanHost make_fft_plan(int set)
             nb[i - 1] = fmul(G[i], G[i], m) ^ G[i];
         B.swap(nb);
     }
+    for (size_t i = 0; i < (size_t)sums * plane; i++)
+        p.tw[(size_t)m * plane + i] = p.tw[i] ^ p.tw[(size_t)half * plane + i];
     return p;
 }
 

@@ -194,6 +194,19 @@ template <int M> struct KAcc {
         for (int k = 0; k < 2 * W - 1; k++)
             hi[k] = 0;
     }
+    // starts from a (it cancels out of the middle part; for M = 12 plane 11 is
+    // beyond lo and comes in through the middle alone)
+    __device__ __forceinline__ void start(const uint32_t *a)
+    {
+#pragma unroll
+        for (int k = 0; k < 2 * H - 1; k++)
+            lo[k] = mid[k] = a[k];
+        if (2 * H - 1 < M)
+            mid[H - 1] ^= a[2 * H - 1];
+#pragma unroll
+        for (int k = 0; k < 2 * W - 1; k++)
+            hi[k] = 0;
+    }
     // xs, ys: ksum of x and y
     __device__ __forceinline__ void mac(const uint32_t *x, const uint32_t *xs, const uint32_t *y, const uint32_t *ys)
     {

@@ -85,7 +85,8 @@ struct FusedKeyRef {
 // tables shared by every key of the set.
 //   scalpow[d*256 + i]: b_d^i, the radix-conversion scale of depth d;
 //   tw[k*2^(m-5) + off_d + u]: plane k of twiddle word u of depth d (off_d =
-//   the sum of the word counts 2^(m-e-6) of the depths e < d).
+//   the sum of the word counts 2^(m-e-6) of the depths e < d); planes m, m + 1,
+//   ... are the half sums plane k ^ plane k + (m+1)/2.
 struct FftPlanDev {
     const uint16_t *scalpow;
     const uint32_t *tw;
