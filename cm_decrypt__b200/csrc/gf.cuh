@@ -22,10 +22,12 @@ namespace cmd {
 template <int M> __device__ __forceinline__ uint32_t gf_reduce(uint32_t p)
 {
     if constexpr (M == 13) {
-        uint32_t h = p >> 13;
-        p = (p & 0x1FFFu) ^ h ^ (h << 1) ^ (h << 3) ^ (h << 4);
+        uint32_t h = p >> 13;  // x^4 + x^3 + x + 1 = (x + 1)(x^3 + 1)
+        h ^= h << 1;
+        p = (p & 0x1FFFu) ^ h ^ (h << 3);
         h = p >> 13;
-        p = (p & 0x1FFFu) ^ h ^ (h << 1) ^ (h << 3) ^ (h << 4);
+        h ^= h << 1;
+        p = (p & 0x1FFFu) ^ h ^ (h << 3);
     } else {
         uint32_t h = p >> 12;
         p = (p & 0xFFFu) ^ h ^ (h << 3);

@@ -44,8 +44,8 @@ constexpr int CT_CV_WORDS = 256 / 2;     // u16 group sums, then locator constan
 constexpr int CT_XB_WORDS = 2 * 256;     // cross-warp exchange of the network (WPC > 1)
 // inside the FFT array while it is free (conversions and Berlekamp-Massey)
 constexpr int CT_SS = 256;               // u32 sx[256] at 0, then uint4 split syndromes [2t]
-constexpr int CT_RING = CT_SS + 4 * 256; // then the B ring [t + 2]
-constexpr int CT_SHARE = CT_RING + 132;  // then the warps' shares, 2 x WPC uint2
+constexpr int CT_RING = CT_SS + 4 * 256; // then the B ring [t + 2] (uint4 split values, or u32)
+constexpr int CT_SHARE = CT_RING + 4 * 132;  // then the warps' shares, 2 x WPC uint2
 static_assert(CT_SHARE + 2 * 2 * CT_WARPS <= CT_FA_WORDS, "Berlekamp-Massey data inside the FFT array");
 
 enum Phase { ALL, SYND, BM, ROOT };
@@ -62,6 +62,14 @@ struct Split {
 };
 constexpr uint32_t K0 = 0x11111111u, K1 = K0 << 1, K2 = K0 << 2, K3 = K0 << 3;
 
+// r | (p & k) as one lop3 (grouped otherwise by the compiler, seven for four).
+__device__ __forceinline__ uint32_t pick(uint32_t r, uint32_t p, uint32_t k)
+{
+    uint32_t o;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(o) : "r"(p), "r"(k), "r"(r));
+    return o;
+}
+
 __device__ __forceinline__ Split split4(uint32_t a) { return {a & K0, a & K1, a & K2, a & K3}; }
 
 // Unreduced carry-less product (bits 0 .. 2m-2).
@@ -71,7 +79,7 @@ __device__ __forceinline__ uint32_t clmul_split(const Split &a, const Split &b)
     const uint32_t p1 = a.c0 * b.c1 + a.c1 * b.c0 + a.c2 * b.c3 + a.c3 * b.c2;
     const uint32_t p2 = a.c0 * b.c2 + a.c1 * b.c1 + a.c2 * b.c0 + a.c3 * b.c3;
     const uint32_t p3 = a.c0 * b.c3 + a.c1 * b.c2 + a.c2 * b.c1 + a.c3 * b.c0;
-    return (p0 & K0) | (p1 & K1) | (p2 & K2) | (p3 & K3);
+    return pick(pick(pick(p0 & K0, p1, K1), p2, K2), p3, K3);
 }
 
 // The Taylor steps of one radix-conversion depth d on scalar entries sx[x],
@@ -156,21 +164,23 @@ __device__ __forceinline__ void convert_scalar(uint32_t *sx, const uint16_t *__r
 // One step of the one-warp Berlekamp-Massey with the first NA groups of 32
 // coefficients active (straight-line code, so the groups' products overlap).
 template <int S, int NA, int NJ>
-__device__ __forceinline__ void bm_step(const uint4 *ss, uint32_t *ring, uint32_t (&C)[NJ], Split &b, int &L, int &off,
+__device__ __forceinline__ void bm_step(const uint4 *ss, uint4 *ring, uint32_t (&C)[NJ], Split &b, int &L, int &off,
                                         int N, int lane)
 {
     constexpr int M = Set<S>::M, T = Set<S>::T, R = T + 2;
-    uint32_t q[NA], bv[NA], pd = 0;
+    uint32_t q[NA], pd = 0;
+    uint4 bv[NA];
+    Split c[NA];
 #pragma unroll
     for (int j = 0; j < NA; j++) {
         const int i = lane + 32 * j;
         int slot = i + off;
         slot = slot >= R ? slot - R : slot;
-        bv[j] = i <= T ? ring[slot] : 0u;
+        bv[j] = i <= T ? ring[slot] : make_uint4(0, 0, 0, 0);
         const uint4 s = ss[max(N - i, 0)];  // C_i = 0 where N < i
-        const Split c = split4(C[j]);
-        pd ^= clmul_split(c, Split{s.x, s.y, s.z, s.w});
-        q[j] = clmul_split(c, b);
+        c[j] = split4(C[j]);
+        pd ^= clmul_split(c[j], Split{s.x, s.y, s.z, s.w});
+        q[j] = clmul_split(c[j], b);
     }
     const uint32_t d = __reduce_xor_sync(FULL, gf_reduce<M>(pd));
     const bool swap = d != 0 && N >= 2 * L;
@@ -183,12 +193,14 @@ __device__ __forceinline__ void bm_step(const uint4 *ss, uint32_t *ring, uint32_
             int slot = i + off;
             slot = slot >= R ? slot - R : slot;
             if (i <= T)
-                ring[slot] = C[j];
+                ring[slot] = j < NA ? make_uint4(c[j < NA ? j : 0].c0, c[j < NA ? j : 0].c1, c[j < NA ? j : 0].c2,
+                                                 c[j < NA ? j : 0].c3)
+                                    : make_uint4(0, 0, 0, 0);
         }
     }
 #pragma unroll
     for (int j = 0; j < NA; j++)
-        C[j] = gf_reduce<M>(q[j] ^ clmul_split(split4(bv[j]), ds));
+        C[j] = gf_reduce<M>(q[j] ^ clmul_split(Split{bv[j].x, bv[j].y, bv[j].z, bv[j].w}, ds));
     if (swap) {
         L = N + 1 - L;
         b = ds;
@@ -196,18 +208,18 @@ __device__ __forceinline__ void bm_step(const uint4 *ss, uint32_t *ring, uint32_
     // the slot that becomes coefficient 0 of x*B
     off = off == 0 ? R - 1 : off - 1;
     if (lane == 0)
-        ring[off] = 0;
+        ring[off] = make_uint4(0, 0, 0, 0);
     __syncwarp();
 }
 
 // One warp: scaled Berlekamp-Massey on the syndromes ss[0 .. 2t) (split);
 // leaves sx[t - i] = C_i, zero above t.
-template <int S> __device__ __forceinline__ void bm_warp(const uint4 *ss, uint32_t *ring, uint32_t *sx, int lane)
+template <int S> __device__ __forceinline__ void bm_warp(const uint4 *ss, uint4 *ring, uint32_t *sx, int lane)
 {
     using F = FftDims<S>;
     constexpr int T = F::T, NX = F::NX, NJ = (T + 32) / 32, R = T + 2;
     for (int v = lane; v < R; v += 32)
-        ring[v] = v == 1;  // B = x
+        ring[v] = make_uint4(v == 1, 0, 0, 0);  // B = x, split
     uint32_t C[NJ];
 #pragma unroll
     for (int j = 0; j < NJ; j++)
@@ -450,7 +462,7 @@ template <int S, int WPC> __device__ __forceinline__ void bm_phase(uint32_t *sme
     }
     group_sync<WPC>();
     if constexpr (WPC == 1)
-        bm_warp<S>(ss, smem + CT_RING, sx, tid);
+        bm_warp<S>(ss, reinterpret_cast<uint4 *>(smem + CT_RING), sx, tid);
     else
         bm_group<S, WPC>(ss, smem + CT_RING, reinterpret_cast<uint2 *>(smem + CT_SHARE), sx, tid);
     group_sync<WPC>();
