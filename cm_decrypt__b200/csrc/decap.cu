@@ -3,7 +3,7 @@
 // computes C = [I | T] e and K = SHAKE256(1 || e || C) (32 bytes).  The
 // Classic McEliece decapsulation inverts that with implicit rejection:
 //
-//   e = decrypt(C)                       (the engine's fused kernel)
+//   e = decrypt(C)                       (CMD_PATH_AUTO's kernels)
 //   accept = padding bits mt..8*ct-1 of C are zero  &&  wt(e) == t
 //            &&  C == [I | T] e          (e re-encodes to C)
 //   K = SHAKE256(b || v || C),  b = accept,  v = accept ? e : s

@@ -38,11 +38,10 @@ struct FusedConfig {
     bool tuned = false;
     double ns_per_ct = 0; // measured by the tuner
     uint32_t tile_below = 0;  // CMD_PATH_AUTO: batches smaller than this take
-                              // the tile kernels (five warps per 32-ciphertext
-                              // tile for Berlekamp-Massey, one warp per
-                              // ciphertext for the FFTs) instead of the fused
-                              // kernel (one warp per tile); 0 = never when
-                              // tuned (untuned: small_below in engine.cu)
+                              // the small-batch kernels (launch_tile_single)
+                              // instead of the staged ones; batches within
+                              // the per-ciphertext kernels' reach take them
+                              // at any value (takes_small in engine.cu)
 };
 
 int cuda_fail(cudaError_t e, const char *what);

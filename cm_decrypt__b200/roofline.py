@@ -3,7 +3,9 @@
 A GF(2^m) multiply is counted as m^2 fused AND-XOR bit operations plus R_m
 reduction XORs (R_12 = 22 for the trinomial x^12+x^3+1, R_13 = 48 for the
 pentanomial x^13+x^4+x^3+x+1); one 32-bit lop3 performs 32 bit operations,
-so every figure below is bit operations / 32 ("lane-ops").
+so every figure below is bit operations / 32 ("lane-ops").  (The kernels' FFT
+and Berlekamp-Massey products split their operands once, Karatsuba's way, and
+execute fewer operations than the m^2 counted here.)
 
 Work of the algorithm the fused kernel executes, per decryption:
 

@@ -102,10 +102,15 @@ int cmd_key_synd_table(const cmd_key *key, uint16_t *h_tab, size_t entries);
 /* Path selector: CMD_PATH_PLAIN runs the three per-stage kernels (syndrome,
  * Berlekamp-Massey, root search + pack); CMD_PATH_FUSED runs the fused
  * bitsliced kernel; CMD_PATH_TILE runs the serving loop's latency kernels
- * (syndromes by the transposed additive FFT, a CTA per 32-ciphertext tile
+ * (one warp or CTA per ciphertext up to 24 ciphertexts an SM; above that
+ * syndromes by the transposed additive FFT, a CTA per 32-ciphertext tile
  * for Berlekamp-Massey, a warp per ciphertext for the root search);
- * CMD_PATH_AUTO lets the engine's tuner choose.  Graph capture takes AUTO,
- * PLAIN and FUSED. */
+ * CMD_PATH_AUTO takes the latency kernels for small batches (up to 24 an SM,
+ * or below the tuned size), the staged kernels (one per phase, with scratch of
+ * about 1.4 KB a ciphertext charged to the engine's budget and kept by the
+ * engine) for larger ones, and the fused kernel for about one round of its
+ * warps (192 to 256 ciphertexts an SM), when the scratch does not fit and
+ * under stream capture.  Graph capture takes AUTO, PLAIN and FUSED. */
 typedef enum { CMD_PATH_AUTO = 0, CMD_PATH_PLAIN = 1, CMD_PATH_FUSED = 2, CMD_PATH_TILE = 3 } cmd_path;
 
 /* Replaces the per-ciphertext loop memcpy -> synd -> bm -> root ->
@@ -201,8 +206,8 @@ int cmd_errorstream_write(cmd_set set, const uint8_t *h_err, size_t count,
 /* The decrypt result as error positions: row c of the output holds t+1 u16,
  * the weight w, then the w flagged positions in ascending order (the numbers
  * write_error_positions prints for that ciphertext), then 0xFFFF.  The
- * weight never exceeds t (the reversed locator has degree exactly t).  Runs
- * the fused kernel, which writes the rows directly: 2(t+1) bytes per
+ * weight never exceeds t (the reversed locator has degree exactly t).  The
+ * kernels (CMD_PATH_AUTO's) write the rows directly: 2(t+1) bytes per
  * ciphertext instead of n/8 (240 vs 870 bytes for 6960119).
  * cmd_decrypt_positions takes host buffers (like cmd_decrypt_batch),
  * cmd_decrypt_positions_device device buffers, asynchronous on `stream`. */
@@ -231,9 +236,9 @@ int cmd_positions_to_errorstream(const char *binary_path, const char *text_path)
  * implicit rejection: e = the decrypt of C (as cmd_decrypt_*); accept iff the
  * padding bits of C above mt are zero, wt(e) == t and C == [I | T] e; then
  * K = SHAKE256(b || v || C) with b = accept and v = e, or v = the secret
- * key's n/8-byte string s when rejected.  The re-encoding check reads every
- * column of T for every ciphertext, and v is selected with masks, so the
- * work does not depend on e.  The first call for a key derives T on the
+ * key's n/8-byte string s when rejected.  The re-encoding check reads all of
+ * T for every ciphertext at addresses that are T's bits, and v is selected
+ * with masks, so the work does not depend on e.  The first call for a key derives T on the
  * device from the key's support and Goppa polynomial (the key generation's
  * elimination) and keeps it there, charged to the engine's budget (1.1 MB for
  * 6960119); cmd_key_prepare_decap does that step ahead of time.  CMD_E_ARG
@@ -380,16 +385,17 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
  * sample_count ciphertexts (0 = about three waves; pass the batch size the
  * caller runs: the winner depends on how that size fills whole rounds of the
  * resident warps, and each size is cached apart), then the batch size below
- * which CMD_PATH_AUTO takes the tile kernels instead (five warps per
- * 32-ciphertext tile for Berlekamp-Massey rather than the fused kernel's
- * one), from timings of both at 256 .. 65,536 ciphertexts.  Results are
+ * which CMD_PATH_AUTO takes the latency kernels (CMD_PATH_TILE) rather than
+ * the staged ones, from timings of both at 256 .. 65,536 ciphertexts; up to 24
+ * ciphertexts an SM AUTO takes them in any case.  Results are
  * cached in the engine and in $CMD_TUNE_CACHE (JSON keyed by GPU name and
  * set); a cached entry is reused unless force != 0. */
 int cmd_tune(cmd_engine *eng, const cmd_key *key, size_t sample_count, int force);
 int cmd_engine_fused_config(cmd_engine *eng, cmd_set set, int *wpb, int *balanced,
                             double *ns_per_ct);
-/* The tuned batch size below which CMD_PATH_AUTO runs the tile kernels (0:
- * never). */
+/* The tuned batch size below which CMD_PATH_AUTO runs the latency kernels (0:
+ * not tuned, or they won at no size; up to 24 ciphertexts an SM it runs them
+ * in any case). */
 int cmd_engine_tile_below(cmd_engine *eng, cmd_set set, uint32_t *tile_below);
 int cmd_engine_set_fused_config(cmd_engine *eng, cmd_set set, int wpb, int balanced);
 
