@@ -39,18 +39,32 @@ template <int S> struct BmDims {
 // without a warp.  The first groups are active longest, so warp (W - turn) % W
 // takes the first one: callers vary `turn` between the tiles of an SM.
 //
+// PAIR: a warp for two tiles, 16 lanes each, groups of 16 coefficients (syn, ring,
+// cm, gsyn and ntile are then those of the lane's own tile; both tiles' arrays are
+// the same distance apart, 16 mod 32 words, so that the halves' rows meet no bank
+// conflict).  The loops are bounded by the larger L of the two, nearly always
+// the same.  L grows from 0 to t, so that a tile takes 1.3 passes of 32 lanes a step
+// instead of 1.5 (t = 64; t = 119: 2.2 instead of 2.5), and the work of a step
+// outside the loop serves both tiles; but half the warps are left to hide its
+// latency.
+//
 // The syndromes are either all in shared memory (syn, gsyn null) or in global
 // memory (gsyn), one row a step coming into syn as a ring of t + 2 rows: step N
 // multiplies rows N + 1 - L .. N + 1 only, and L stops at t.  The ring takes a
 // quarter off a tile's shared memory.
-template <int S, bool GLOBAL_SYN = false, int W = 1>
+template <int S, bool GLOBAL_SYN = false, int W = 1, bool PAIR = false>
 __device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t *cm, int ntile, int tid,
                                         const uint32_t *gsyn = nullptr, uint32_t *share = nullptr, int turn = 0)
 {
     using Z = BmDims<S>;
-    constexpr int M = Z::M, T = Z::T, SS = Z::SS, R = Z::R, H = KAcc<M>::H, NT = 32 * W;
+    static_assert(W == 1 || !PAIR, "a pair of tiles: one warp");
+    constexpr int M = Z::M, T = Z::T, SS = Z::SS, R = Z::R, H = KAcc<M>::H, NT = PAIR ? 16 : 32 * W;
+    constexpr int NQ = PAIR ? 2 : 1;  // ciphertexts whose L a lane keeps: lane, lane + 16 of its tile
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const int lane = tid & 31, warp = tid >> 5;
+    const bool upper = PAIR && lane >= 16;
+    if (PAIR)
+        tid &= 15;
     const int first = W == 1 ? tid : (tid + 32 * turn) % NT;  // this lane's first coefficient
     auto sync = [] {
         if constexpr (W == 1)
@@ -73,8 +87,10 @@ __device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t 
         b[k] = k == 0 ? FULL : 0u;      // b = 1
         p[k] = tid == 0 ? syn[k] : 0u;  // d_0 = C_0 S_0 (any one lane)
     }
-    int Lq = 0;            // L of ciphertext `lane`
-    int Bd = 1, Bmax = 1;  // bound on deg B of ciphertext `lane`; the tile's
+    int Lq[NQ] = {}, Bd[NQ], Bmax = 1;  // L and a bound on deg B of the lane's ciphertexts; the latter's largest
+#pragma unroll
+    for (int h = 0; h < NQ; h++)
+        Bd[h] = 1;
     if (W == 1)
         sync();
 #pragma unroll 1
@@ -83,9 +99,17 @@ __device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t 
         if (GLOBAL_SYN && tid < SS && N + 2 < 2 * T)
             row = gsyn[(N + 2) * SS + tid];
         uint32_t d[M], mne = 0;
+        if (PAIR && upper) {
 #pragma unroll
-        for (int k = 0; k < M; k++)
-            d[k] = __reduce_xor_sync(FULL, p[k]);
+            for (int k = 0; k < M; k++)
+                d[k] = __reduce_xor_sync(0xFFFF0000u, p[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < M; k++)
+                d[k] = __reduce_xor_sync(PAIR ? 0xFFFFu : FULL, p[k]);
+        }
+        if constexpr (PAIR)
+            __syncwarp();
         if constexpr (W > 1) {
             uint32_t *sh = share + (N & 1) * W * 16;  // rewritten two barriers later
             uint32_t mine = 0;
@@ -112,11 +136,19 @@ __device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t 
 #pragma unroll
         for (int k = 0; k < M; k++)
             mne |= d[k];
-        const bool my_mle = ((mne >> lane) & 1u) && (N >= 2 * Lq);
-        const uint32_t mle = __ballot_sync(FULL, my_mle);
-        const int Bdn = min(min(my_mle ? Lq : Bd, T) + 1, T);
-        Lq = my_mle ? N + 1 - Lq : Lq;
-        const int Lb = min((int)__reduce_max_sync(FULL, (unsigned)Lq), T);
+        uint32_t ball[NQ];
+        int Lmax = 0;
+#pragma unroll
+        for (int h = 0; h < NQ; h++) {
+            const bool my_mle = ((mne >> (PAIR ? tid + 16 * h : lane)) & 1u) && (N >= 2 * Lq[h]);
+            ball[h] = __ballot_sync(FULL, my_mle);
+            Bd[h] = min(min(my_mle ? Lq[h] : Bd[h], T) + 1, T);
+            Lq[h] = my_mle ? N + 1 - Lq[h] : Lq[h];
+            Lmax = max(Lmax, Lq[h]);
+        }
+        // of a pair, each ballot has 16 bits of either tile
+        const uint32_t mle = PAIR ? __byte_perm(ball[0], ball[NQ - 1], upper ? 0x7632 : 0x5410) : ball[0];
+        const int Lb = min((int)__reduce_max_sync(FULL, (unsigned)Lmax), T);
         const int Bm = min(Bmax, T);
         uint32_t bs[H], ds[H];
         ksum<M>(bs, b);
@@ -131,7 +163,7 @@ __device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t 
         const int hi = max(Lb, Bm);
         const int srow = GLOBAL_SYN ? next % R : next;
 #pragma unroll 1
-        for (int i = first; (i & ~31) <= hi; i += NT) {
+        for (int i = first; (i & ~(PAIR ? 15 : 31)) <= hi; i += NT) {
             int slot = i + off;
             slot = slot >= R ? slot - R : slot;
             uint32_t *bp = ring + slot * SS;
@@ -177,9 +209,12 @@ __device__ __forceinline__ void bm_tile(uint32_t *syn, uint32_t *ring, uint32_t 
             ring[freeslot * SS + tid] = 0;
         if (GLOBAL_SYN && tid < SS)  // over row N - t, which no later step reads
             syn[(N + 2) % R * SS + tid] = row;
-        Bd = Bdn;
-        // (lanes past the tile's count never take the swap: zero syndromes)
-        Bmax = (int)__reduce_max_sync(FULL, lane < ntile ? (unsigned)Bd : 0u);
+        // (ciphertexts past the tile's count never take the swap: zero syndromes)
+        unsigned Bm1 = 0;
+#pragma unroll
+        for (int h = 0; h < NQ; h++)
+            Bm1 = max(Bm1, (PAIR ? tid + 16 * h : lane) < ntile ? (unsigned)Bd[h] : 0u);
+        Bmax = (int)__reduce_max_sync(FULL, Bm1);
         acc.combine(p);
         bs_reduce<M>(p);
         if (W == 1)

@@ -5,7 +5,8 @@
 //   k_synd_table  the 2t syndromes (util.c:102-114) from the key's dense table,
 //                 lane = ciphertext, rows five at a time;
 //   k_bm_tile     Berlekamp-Massey (bm.c:12-68), a warp and block per tile of 32
-//                 ciphertexts, and the locators' radix conversion;
+//                 ciphertexts, and the locators' radix conversion (k_bm_pair: per
+//                 two tiles);
 //   k_fft_tile    the locators at all field elements (additive FFT), a warp per
 //                 ciphertext: zero flags;
 //   k_net_rows    the key's support network (root_13.c:95-177) over the flags of
@@ -47,6 +48,10 @@ template <int S> struct SgDims {
     static constexpr int TILE_WORDS = BmDims<S>::SYN_WORDS > NX * SS ? BmDims<S>::SYN_WORDS : NX * SS;
     static constexpr int BM_WORDS = 2 * BmDims<S>::RING_WORDS + BmDims<S>::C_WORDS;  // shared, per tile
     static_assert(NX * SS <= BM_WORDS && 4 * (BM_WORDS + 128) <= 48 * 1024, "conversion array in the same memory");
+    static constexpr int PAIR_WORDS = (BM_WORDS + 15) / 32 * 32 + 16;  // a tile of a pair: 16 mod 32 (bm_tile)
+    // two pairs a scheduler fit the SM's shared memory
+    static constexpr bool PAIRS = 8 * (8 * PAIR_WORDS + 1024) <= 228 * 1024;
+    static_assert(!PAIRS || 8 * PAIR_WORDS <= 48 * 1024, "no opt-in for shared memory");
     static constexpr int NWU = (2 * T * M + 31) / 32;  // syndrome words of a ciphertext
     // syndrome kernel: rows per group, combination rows an odd stride apart
     static constexpr int G = 5, NG = (P::SB + G - 1) / G, CS = NWU | 1, COMBS = 1 << G;
@@ -252,6 +257,43 @@ __global__ void __launch_bounds__(32 * W) k_bm_tile(uint32_t *__restrict__ tiles
         io[v] = cv[v];
 }
 
+// The same for two tiles by one warp (bm_tile's PAIR), for large batches of a set
+// with room for ten pairs an SM: 2^20 mceliece348864 ciphertexts 13,397 -> 12,687
+// us, 200,000 2,557 -> 2,463 us.
+template <int S>
+__global__ void __launch_bounds__(32) k_bm_pair(uint32_t *__restrict__ tiles, uint32_t ntiles, uint32_t count,
+                                                const uint16_t *__restrict__ scalpow)
+{
+    using Z = SgDims<S>;
+    using B = BmDims<S>;
+    constexpr int T = Z::T, SS = Z::SS, NX = Z::NX, HW = Z::PAIR_WORDS;
+    extern __shared__ __align__(16) uint32_t smem_sg[];
+    const int lane = threadIdx.x;
+    const uint32_t tile0 = 2 * blockIdx.x;
+    const int nt = ntiles - tile0 < 2 ? 1 : 2;  // for an absent second tile, the first's again, not stored
+    const uint32_t tile = tile0 + (nt == 2 ? lane >> 4 : 0);
+    uint32_t *ring = smem_sg + (lane >> 4) * HW, *cm = ring + B::RING_WORDS, *syn = cm + B::C_WORDS;
+    const uint32_t left = count - 32 * tile;
+    bm_tile<S, true, 1, true>(syn, ring, cm, left < 32 ? (int)left : 32, lane,
+                              tiles + (size_t)tile * Z::TILE_WORDS);
+    __syncwarp();
+#pragma unroll 1
+    for (int j = 0; j < nt; j++) {
+        uint32_t *cv = smem_sg + j * HW, *c = cv + B::RING_WORDS, *io = tiles + (size_t)(tile0 + j) * Z::TILE_WORDS;
+        for (int v = lane; v < (T + 1) * SS; v += 32) {
+            const int i = v / SS, k = v - i * SS;
+            io[(T - i) * SS + k] = c[v];
+        }
+        __syncwarp();
+        for (int v = lane; v < NX * SS; v += 32)
+            cv[v] = v < (T + 1) * SS ? io[v] : 0u;
+        __syncwarp();
+        fft_convert<S, SS, 32>(cv, scalpow, lane, [] { __syncwarp(); });
+        for (int v = lane; v < NX * SS; v += 32)
+            io[v] = cv[v];
+    }
+}
+
 // The additive FFT of a tile's locators, a warp per ciphertext in turn, gridDim.y
 // blocks a tile: flags
 // flags[c * 2^(m-5) + w] = the zero test of elements 32w .. 32w + 31 in FFT
@@ -369,7 +411,7 @@ size_t staged_scratch_words(int set, size_t count)
 
 cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count, uint32_t *d_scratch, uint32_t *d_err,
                           uint16_t *d_weight, uint16_t *d_pos, uint8_t *err_packed, const FftPlanDev &plan,
-                          int num_sms, cudaStream_t s, LaunchCounter lc)
+                          int num_sms, bool many_parts, cudaStream_t s, LaunchCounter lc)
 {
     if (count == 0)
         return cudaSuccess;
@@ -406,7 +448,20 @@ cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count,
         // 878 against 953 us, 37,888: 1,534 against 1,693 us).
         const int bw = ntiles <= sms ? 4 : ntiles <= 2 * sms ? 2 : ntiles <= 4 * sms ? 1 : ntiles <= 6 * sms ? 2 : 1;
         const size_t bm_smem = 4 * (size_t)(Z::BM_WORDS + 2 * bw * 16);
-        if (bw == 4)
+        // Two tiles a warp where the SM holds at least two such warps a scheduler
+        // (t = 64; with five or six of them an SM, t >= 119, 2^20 ciphertexts are
+        // 0.5 to 6 % slower, with seven, t = 96, 1 %) and other parts fill the ends
+        // of the coarser waves (100,000 ciphertexts in two parts 3 % slower,
+        // 131,073 in three the same, 200,000 4 % faster, 2^20 5.6 %).
+        bool pairs = false;
+        if constexpr (Z::PAIRS) {
+            pairs = many_parts;
+            if (pairs)
+                k_bm_pair<S><<<(ntiles + 1) / 2, 32, 8 * Z::PAIR_WORDS, s>>>(tiles, ntiles, count, plan.scalpow);
+        }
+        if (pairs)
+            ;
+        else if (bw == 4)
             k_bm_tile<S, 4><<<ntiles, 128, bm_smem, s>>>(tiles, count, plan.scalpow, sms, nullptr);
         else if (bw == 2)
             k_bm_tile<S, 2><<<ntiles, 64, bm_smem, s>>>(tiles, count, plan.scalpow, 2 * sms, nullptr);
