@@ -1,7 +1,8 @@
 // Berlekamp-Massey (bm.c:12-68) bitsliced across the 32 ciphertexts of a tile:
 // word bit q belongs to ciphertext q, lane l owns locator coefficients l, l + 32,
-// ...  Coefficients, syndromes and B are rows of SS words in shared memory (SS = m made odd, so that lanes' rows meet no bank conflict; for
-// m = 12 the 12-word rows of neighbouring lanes met four ways).
+// ...  Coefficients, syndromes and B are rows of SS words in shared memory (SS = m
+// made odd, so that lanes' rows meet no bank conflict; for m = 12 the 12-word rows
+// of neighbouring lanes met four ways).
 //
 // The update is the scaled form C <- b*C + d*x*B instead of bm()'s C <- C +
 // (d/b)*x*B: same decisions (d != 0, N >= 2L), same truncation, and by induction

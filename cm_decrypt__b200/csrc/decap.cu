@@ -23,10 +23,11 @@
 //     a lane a ciphertext and every column of T (52 words) masked by its bit;
 //  3. row i must equal e_i + C_i; padding and weight checks.
 // k_session_keys: SHAKE256 of the 1 + n/8 + ct byte preimage, one lane per
-// ciphertext, the next block's words loaded during a permutation (110 us for the
-// same batch; 175 us with the loads before each block) (Keccak-f[1600] as defined in FIPS 202; round constants and rotation
-// offsets derived from the standard's definitions at compile time); the
-// preimage's v bytes are selected with masks.
+// ciphertext (Keccak-f[1600] as defined in FIPS 202; round constants and rotation
+// offsets derived from the standard's definitions at compile time), the next
+// block's words loaded during a permutation (110 us for the same batch; 175 us
+// with the loads before each block); the preimage's v bytes are selected with
+// masks.
 // Every column of T and every word of e is read for every ciphertext, so the work
 // and the addresses do not depend on e.
 #include <cstring>

@@ -560,7 +560,7 @@ int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t
 // Whether CMD_PATH_AUTO takes the small-batch kernels: batches within the
 // per-ciphertext kernels' reach, or below the tuned crossover.  At 24 ciphertexts
 // an SM (3,552) the per-ciphertext kernels and the staged ones take the same time
-// (6960119 442 and 447 us, 348864 202 and 235 us), at half of that 206 against
+// (6960119 438 and 447 us, 348864 205 and 235 us), at half of that 279 against
 // 415 us; the fused kernel takes 1,037 us for any number up to 18,944.
 static bool takes_small(const cmd_engine *eng, int set, size_t count)
 {
@@ -575,7 +575,7 @@ size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count)
 // The best kernels for the batch size, error rows and weights or positions:
 // small-batch kernels, else the staged ones.  The fused kernel takes batches of
 // six to eight tiles an SM, one nearly full round of its warps (37,888
-// mceliece6960119 ciphertexts 1,505 us, staged 1,534 us); needing no scratch, it
+// mceliece6960119 ciphertexts 1,485 us, staged 1,534 us); needing no scratch, it
 // also runs when theirs does not fit the budget, and under stream capture, where
 // nothing may be allocated and a graph would keep the address of scratch that can
 // grow.

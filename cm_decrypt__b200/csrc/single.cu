@@ -20,9 +20,9 @@
 //     support network (fft_root.cuh), outputs.
 //
 // WPC warps share a ciphertext in a step.  Measured on a B200 (tile kernels ->
-// these): one ciphertext of mceliece6960119 368 -> 79 us, 37 of 348864 187 ->
-// 47 us, 1,184 of 6960119 388 -> 178 us; above about 24 ciphertexts an SM the
-// tile kernels' bitsliced Berlekamp-Massey wins (4,736: 501 against 580 us).
+// these): one ciphertext of mceliece6960119 368 -> 78 us, 37 of 348864 187 ->
+// 46 us, 1,184 of 6960119 388 -> 180 us; above about 24 ciphertexts an SM the
+// tile kernels' bitsliced Berlekamp-Massey wins (4,736: 496 against 580 us).
 // Bound by the latency of the serial Berlekamp-Massey chain up to one
 // ciphertext an SM, by the multiply and logic pipes above.  Constant time as
 // the other paths: no address or branch depends on the key or the error

@@ -21,10 +21,10 @@
 // ciphertext (syndromes, then the converted locator) and 1 KB of flags.
 //
 // Measured on a B200 against the fused kernel: 65,536 mceliece6960119 ciphertexts
-// 2,879 -> 2,559 us, 50,000 of 8192128 3,082 -> 2,585 us, 2^20 of 348864 14.93 ->
-// 13.57 ms, 12,345 of 460896 879 -> 647 us, 4,736 of 6960119 1,037 -> 440 us.  Of
+// 2,830 -> 2,522 us, 50,000 of 8192128 3,036 -> 2,558 us, 2^20 of 348864 14.68 ->
+// 12.69 ms, 12,345 of 460896 879 -> 642 us, 4,736 of 6960119 1,037 -> 440 us.  Of
 // 37,888 ciphertexts of 6960119 in one part: syndromes 244 us (shared-memory
-// bound), Berlekamp-Massey 820 us (logic pipe 85 % busy), FFT 477 us (91 %),
+// bound), Berlekamp-Massey 820 us (logic pipe 85 % busy), FFT 467 us (89 %),
 // network 43 us.
 #include <algorithm>
 
