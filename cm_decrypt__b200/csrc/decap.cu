@@ -371,19 +371,12 @@ int cmd_kem_decap_device(cmd_engine *eng, cmd_key *key, const uint8_t *d_cts, si
     cudaSetDevice(eng->device);
     std::lock_guard<std::mutex> lk(eng->mu);
     cudaStream_t s = stream ? (cudaStream_t)stream : eng->stream;
-    // error rows and weights after what the decrypt keeps in the same scratch
-    const size_t words = count * si.nw, rows = words * 4 + count * 2 + 256;
-    size_t inner = (auto_scratch_bytes(eng, key->dev.set, count) + 255) / 256 * 256;
-    if (inner && eng->scratch.reserve(eng, inner + rows))
-        inner = 0;
-    if ((rc = eng->scratch.reserve(eng, inner + rows)))
+    const size_t words = count * si.nw;
+    if ((rc = eng->scratch.reserve(eng, words * 4 + count * 2 + 256)))
         return rc;
-    uint32_t *d_err = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(eng->scratch.ptr) + inner);
+    uint32_t *d_err = static_cast<uint32_t *>(eng->scratch.ptr);
     uint16_t *d_w = reinterpret_cast<uint16_t *>(d_err + words);
-    rc = inner || !auto_scratch_bytes(eng, key->dev.set, count)
-             ? run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)
-             : run_fused_single(eng, key, d_cts, count, d_err, d_w, s);
-    if (rc)
+    if ((rc = run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)))
         return rc;
     const uint8_t *d_s = key->dev.sk + 40 + 2 * si.t + si.cond;
     cudaError_t e = launch_decap(key->dev.set, d_cts, d_err, d_w, key->pk, d_s, d_keys, d_accept, count, s,

@@ -13,7 +13,7 @@
 
 namespace cmd {
 static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s);
+                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s, bool ordered = false);
 
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
@@ -446,30 +446,42 @@ static int run_plain(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, 
 
 // The serving tile kernels over one key's batch, in chunks whose byte and
 // word offsets fit the tile items' 32-bit fields.  With d_synd: syndromes
-// only.  Caller holds eng->mu.
+// only.  Scratch: the engine's, or (ordered) that of the staged batches, which is
+// safe with batches in flight on other streams.  Caller holds eng->mu.
 static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s)
+                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s, bool ordered)
 {
     const SetInfo si = set_info(key->dev.set);
     const size_t chunk = std::min<size_t>(count, (size_t)1 << 22);
     int rc = CMD_OK;
-    if (d_synd || count > CT_ONE_LAUNCH)  // smaller batches keep everything on chip
+    if (!d_synd && count <= CT_ONE_LAUNCH)  // everything stays on chip
+        ordered = false;
+    else if (ordered)
+        rc = staged_begin(eng, tile_single_scratch_words(chunk) * 4, 1, s);
+    else
         rc = eng->scratch.reserve(eng, tile_single_scratch_words(chunk) * 4);
     if (rc)
         return rc;
+    uint32_t *scratch = static_cast<uint32_t *>(ordered ? eng->staged.ptr : eng->scratch.ptr);
     FftPlans plans;
     for (int st = 0; st < NSETS; st++)
         plans.p[st] = eng->fft[st];
     for (size_t c0 = 0; c0 < count; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
         const cudaError_t e = launch_tile_single(
-            key->dev, d_cts + c0 * si.ct, n, static_cast<uint32_t *>(eng->scratch.ptr),
-            d_err ? d_err + c0 * si.nw : nullptr, d_weight ? d_weight + c0 : nullptr, d_pos,
+            key->dev, d_cts + c0 * si.ct, n, scratch, d_err ? d_err + c0 * si.nw : nullptr,
+            d_weight ? d_weight + c0 : nullptr, d_pos,
             d_synd ? d_synd + c0 * 2 * si.t : nullptr, plans, eng->num_sms, s, LaunchCounter{&eng->launches});
-        if (e != cudaSuccess)
-            return cuda_fail(e, "tile path launch");
+        if (e != cudaSuccess) {
+            rc = cuda_fail(e, "tile path launch");
+            break;
+        }
     }
-    return CMD_OK;
+    if (ordered) {  // also after an error
+        const int r = staged_end(eng, 1, s, cudaSuccess);
+        return rc ? rc : r;
+    }
+    return rc;
 }
 
 int ensure_piece_streams(cmd_engine *eng)
@@ -499,7 +511,7 @@ static size_t staged_part(size_t count)
 int staged_begin(cmd_engine *eng, size_t bytes, int ns, cudaStream_t s)
 {
     int rc = eng->staged.reserve(eng, bytes);
-    if (rc || (rc = ensure_piece_streams(eng)))
+    if (rc || (ns > 1 && (rc = ensure_piece_streams(eng))))
         return rc;
     cudaError_t e = cudaSuccess;
     if (!eng->staged_done) {
@@ -511,7 +523,7 @@ int staged_begin(cmd_engine *eng, size_t bytes, int ns, cudaStream_t s)
         for (cudaEvent_t &ev : eng->staged_join)
             make(&ev);
         make(&eng->staged_done);
-    } else if (eng->staged_last != s) {
+    } else {
         // the scratch may still be in use by a batch on another stream
         e = cudaStreamWaitEvent(s, eng->staged_done);
     }
@@ -533,7 +545,6 @@ int staged_end(cmd_engine *eng, int ns, cudaStream_t s, cudaError_t e)
     }
     if (e == cudaSuccess)
         e = cudaEventRecord(eng->staged_done, s);
-    eng->staged_last = s;
     return e == cudaSuccess ? CMD_OK : cuda_fail(e, "staged batch");
 }
 
@@ -567,11 +578,6 @@ static bool takes_small(const cmd_engine *eng, int set, size_t count)
     return count <= (size_t)CT_PER_SM * eng->num_sms || count < eng->fcfg[set].tile_below;
 }
 
-size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count)
-{
-    return takes_small(eng, set, count) && count > CT_ONE_LAUNCH ? tile_single_scratch_words(count) * 4 : 0;
-}
-
 // The best kernels for the batch size, error rows and weights or positions:
 // small-batch kernels, else the staged ones.  The fused kernel takes batches of
 // six to eight tiles an SM, one nearly full round of its warps (37,888
@@ -586,8 +592,9 @@ static int run_auto(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
         if (takes_small(eng, set, count) && (!d_pos || count <= (size_t)CT_PER_SM * eng->num_sms)) {
-            if (eng->scratch.reserve(eng, auto_scratch_bytes(eng, set, count)) == CMD_OK)
-                return run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s);
+            const int rc = run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s, true);
+            if (rc != CMD_E_BUDGET)
+                return rc;
         } else if (count <= 192 * (size_t)eng->num_sms || count > 256 * (size_t)eng->num_sms) {
             const int rc = run_staged(eng, key, d_cts, count, d_err, d_weight, d_pos, s);
             if (rc != CMD_E_BUDGET)

@@ -60,9 +60,6 @@ void budget_give(cmd_engine *eng, size_t bytes);
 // d_pos: with CMD_PATH_AUTO only, positions rows instead of error rows.
 int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t *d_cts, size_t count,
                uint32_t *d_err, uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos = nullptr);
-// The eng->scratch bytes (from its start) CMD_PATH_AUTO would use; 0 for the
-// fused kernel, which it also falls back to when they do not fit.
-size_t auto_scratch_bytes(const cmd_engine *eng, int set, size_t count);
 int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                      uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos = nullptr);
 // The staged kernels over one key's device batch (see engine.cu): err/weight or
@@ -118,10 +115,10 @@ struct cmd_engine {
     cmd::Scratch scratch;          // plain-path intermediates
     cmd::Scratch io;               // device staging for host-buffer calls
     cmd::Scratch fused;            // fused-kernel work lists
-    cmd::Scratch staged;           // staged kernels' intermediates, one part per piece stream
+    cmd::Scratch staged;           // staged kernels' intermediates, one part per piece stream,
+                                   // and CMD_PATH_AUTO's small batches'
     cudaEvent_t staged_fork = nullptr, staged_join[cmd::STAGED_STREAMS] = {};  // created on first use
-    cudaEvent_t staged_done = nullptr;      // recorded after each staged batch, on staged_last
-    cudaStream_t staged_last = nullptr;
+    cudaEvent_t staged_done = nullptr;      // recorded after each use of `staged`
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
     cmd::HostScratch host_scratch; // pinned staging
     uint32_t *tile_counter = nullptr;

@@ -127,3 +127,26 @@ def test_mixed_sizes_match_plain(engine):
     finally:
         for k in keys:
             k.free()
+
+
+def test_small_batches_on_two_streams(engine):
+    """Small batches in flight on two streams at once share the scratch between
+    their kernels' launches in order, beside a larger batch."""
+    s = 460896
+    info, cts = batch(s, 8000)
+    key = cmd.Key(engine, s, golden_sk(s))
+    try:
+        want, want_w = run(engine, key, cts, "plain")
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        jobs = [(first, n) for n in (3000, 100, 8000, 65, 3552) for first in (0, 31) if first + n <= 8000] * 4
+        outs = [(torch.zeros((n, info.err_words), dtype=torch.int32, device="cuda"),
+                 torch.zeros(n, dtype=torch.int16, device="cuda")) for _, n in jobs]
+        torch.cuda.synchronize()
+        for i, ((first, n), (err, w)) in enumerate(zip(jobs, outs)):
+            cmd.decrypt_device(engine, key, cts.data_ptr() + first * info.ct_bytes, n, err.data_ptr(), w.data_ptr(),
+                               streams[i % 2].cuda_stream)
+        torch.cuda.synchronize()
+        for (first, n), (err, w) in zip(jobs, outs):
+            assert torch.equal(err, want[first:first + n]) and torch.equal(w, want_w[first:first + n]), (first, n)
+    finally:
+        key.free()
