@@ -232,11 +232,11 @@ static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t 
     size_t words[NSETS + 1] = {};
     for (int st = 0; st < NSETS; st++)
         words[st + 1] = words[st] + staged_scratch_words(st, 32 * (size_t)(p.tile0[st + 1] - p.tile0[st]));
-    if (eng->fused.reserve(eng, b_order + 2 * b_off + b_blk + b_tile + b_keys) != CMD_OK)
-        return CMD_E_BUDGET;
-    int rc = staged_begin(eng, words[NSETS] * 4, 1, s);  // the lists follow the previous batch's reads, too
+    int rc = eng->staged.reserve(eng, words[NSETS] * 4);
     if (rc)
         return rc;
+    if (eng->fused.begin(eng, b_order + 2 * b_off + b_blk + b_tile + b_keys, s) != CMD_OK)
+        return CMD_E_BUDGET;
     uint8_t *at = static_cast<uint8_t *>(eng->fused.ptr);
     cudaError_t e = cudaSuccess;
     auto put = [&](const void *src, size_t bytes, size_t room) {
@@ -254,11 +254,13 @@ static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t 
     mx.tiles = reinterpret_cast<const StagedPiece *>(put(p.tiles.data(), p.tiles.size() * sizeof(StagedPiece), b_tile));
     mx.keys = reinterpret_cast<const FusedKeyRef *>(put(krefs.data(), nkeys * sizeof(FusedKeyRef), b_keys));
     if (e != cudaSuccess)
-        return staged_end(eng, 1, s, e);
+        return eng->fused.end(s, e);
     // the sets beside one another, as the parts of a single-key batch
     const int ns = STAGED_STREAMS;
-    if ((rc = staged_begin(eng, words[NSETS] * 4, ns, s)))
+    if ((rc = staged_begin(eng, words[NSETS] * 4, ns, s))) {
+        eng->fused.end(s);
         return rc;
+    }
     for (int st = NSETS - 1, i = 0; st >= 0 && e == cudaSuccess; st--) {  // the costlier sets first
         const uint32_t nb = p.block0[st + 1] - p.block0[st], nt = p.tile0[st + 1] - p.tile0[st];
         if (nt == 0)
@@ -270,7 +272,9 @@ static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t 
                                 d_weight, eng->fft[st], eng->num_sms, eng->piece_stream[i++ % ns],
                                 LaunchCounter{&eng->launches});
     }
-    return staged_end(eng, ns, s, e);
+    rc = staged_end(eng, ns, s, e);
+    const int r = eng->fused.end(s);
+    return rc ? rc : r;
 }
 
 // A small mixed batch on the per-ciphertext kernels.  CMD_E_BUDGET as above, also
@@ -383,7 +387,7 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
                  b_keys = nkeys * sizeof(FusedKeyRef);
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
     const size_t need = al(b_order) + 2 * al(b_off) + al(b_tiles) + al(b_keys);
-    if ((rc = eng->fused.reserve(eng, need)))
+    if ((rc = eng->fused.begin(eng, need, s)))
         return rc;
     uint8_t *base = static_cast<uint8_t *>(eng->fused.ptr);
     uint32_t *d_order = reinterpret_cast<uint32_t *>(base);
@@ -398,7 +402,7 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
         (e = cudaMemcpyAsync(d_tiles, tiles.data(), b_tiles, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(d_keys, krefs.data(), b_keys, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemsetAsync(eng->tile_counter, 0, sizeof(uint32_t), s)) != cudaSuccess)
-        return cuda_fail(e, "mixed batch upload");
+        return eng->fused.end(s, e);
     FusedArgs a;
     memset(&a, 0, sizeof a);
     a.tiles = d_tiles;
@@ -421,5 +425,5 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
             smem = std::max(smem, fused_smem(st, wpb));
     const int grid = grid_for(eng, single, wpb, smem, tiles.size());
     e = launch_fused(a, grid, wpb, s, LaunchCounter{&eng->launches});
-    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "fused kernel launch (mixed)");
+    return eng->fused.end(s, e);
 }

@@ -51,6 +51,8 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes)
         return CMD_E_BUDGET;
     }
     if (ptr) {
+        if (done)
+            cudaEventSynchronize(done);
         cudaFree(ptr);
         ptr = nullptr;
     }
@@ -65,12 +67,47 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes)
     return CMD_OK;
 }
 
+static bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess)
+        return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();  // the legacy stream beside a capture
+    return true;
+}
+
+int Scratch::begin(cmd_engine *eng, size_t bytes, cudaStream_t s)
+{
+    const int rc = reserve(eng, bytes);
+    if (rc || !done || capturing(s))
+        return rc;
+    const cudaError_t e = cudaStreamWaitEvent(s, done);
+    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "scratch order");
+}
+
+int Scratch::end(cudaStream_t s, cudaError_t e)
+{
+    if (!capturing(s)) {
+        cudaError_t r = done ? cudaSuccess : cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+        if (r == cudaSuccess)
+            r = cudaEventRecord(done, s);
+        if (e == cudaSuccess)
+            e = r;
+    }
+    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "batch on the engine's scratch");
+}
+
 void Scratch::release(cmd_engine *eng)
 {
+    if (done) {
+        cudaEventSynchronize(done);
+        cudaEventDestroy(done);
+    }
     if (ptr)
         cudaFree(ptr);
     budget_give(eng, cap);
     ptr = nullptr;
+    done = nullptr;
     cap = 0;
 }
 
@@ -206,9 +243,8 @@ void cmd_engine_destroy(cmd_engine *eng)
             cudaStreamSynchronize(eng->piece_stream[i]);
             cudaStreamDestroy(eng->piece_stream[i]);
         }
-    for (cudaEvent_t ev : {eng->staged_fork, eng->staged_done})
-        if (ev)
-            cudaEventDestroy(ev);
+    if (eng->staged_fork)
+        cudaEventDestroy(eng->staged_fork);
     for (cudaEvent_t ev : eng->staged_join)
         if (ev)
             cudaEventDestroy(ev);
@@ -510,26 +546,22 @@ static size_t staged_part(size_t count)
 
 int staged_begin(cmd_engine *eng, size_t bytes, int ns, cudaStream_t s)
 {
-    int rc = eng->staged.reserve(eng, bytes);
-    if (rc || (ns > 1 && (rc = ensure_piece_streams(eng))))
+    int rc = eng->staged.begin(eng, bytes, s);
+    if (rc || ns == 1)
+        return rc;
+    if ((rc = ensure_piece_streams(eng)))
         return rc;
     cudaError_t e = cudaSuccess;
-    if (!eng->staged_done) {
-        auto make = [&](cudaEvent_t *ev) {
-            if (e == cudaSuccess)
-                e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
-        };
-        make(&eng->staged_fork);
-        for (cudaEvent_t &ev : eng->staged_join)
-            make(&ev);
-        make(&eng->staged_done);
-    } else {
-        // the scratch may still be in use by a batch on another stream
-        e = cudaStreamWaitEvent(s, eng->staged_done);
-    }
-    if (e == cudaSuccess && ns > 1)
+    auto make = [&](cudaEvent_t &ev) {
+        if (!ev && e == cudaSuccess)
+            e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    };
+    make(eng->staged_fork);
+    for (cudaEvent_t &ev : eng->staged_join)
+        make(ev);
+    if (e == cudaSuccess)
         e = cudaEventRecord(eng->staged_fork, s);
-    for (int i = 0; i < ns && ns > 1 && e == cudaSuccess; i++)
+    for (int i = 0; i < ns && e == cudaSuccess; i++)
         e = cudaStreamWaitEvent(eng->piece_stream[i], eng->staged_fork);
     return e == cudaSuccess ? CMD_OK : cuda_fail(e, "staged batch");
 }
@@ -543,9 +575,7 @@ int staged_end(cmd_engine *eng, int ns, cudaStream_t s, cudaError_t e)
         if (e == cudaSuccess)
             e = e2;
     }
-    if (e == cudaSuccess)
-        e = cudaEventRecord(eng->staged_done, s);
-    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "staged batch");
+    return eng->staged.end(s, e);
 }
 
 int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
@@ -589,8 +619,7 @@ static int run_auto(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
                     uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
 {
     const int set = key->dev.set;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    if (!capturing(s)) {
         if (takes_small(eng, set, count) && (!d_pos || count <= (size_t)CT_PER_SM * eng->num_sms)) {
             const int rc = run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s, true);
             if (rc != CMD_E_BUDGET)

@@ -19,7 +19,13 @@ namespace cmd {
 struct Scratch {
     void *ptr = nullptr;
     size_t cap = 0;
+    cudaEvent_t done = nullptr;  // after the last use between begin and end
     int reserve(cmd_engine *eng, size_t bytes);
+    // Around work on a caller's stream that uses the buffer: reserves it and orders
+    // s after its last use on any stream; marks this use (also after an error e).
+    // A stream under capture neither waits nor marks.
+    int begin(cmd_engine *eng, size_t bytes, cudaStream_t s);
+    int end(cudaStream_t s, cudaError_t e = cudaSuccess);
     void release(cmd_engine *eng);
 };
 
@@ -118,7 +124,6 @@ struct cmd_engine {
     cmd::Scratch staged;           // staged kernels' intermediates, one part per piece stream,
                                    // and CMD_PATH_AUTO's small batches'
     cudaEvent_t staged_fork = nullptr, staged_join[cmd::STAGED_STREAMS] = {};  // created on first use
-    cudaEvent_t staged_done = nullptr;      // recorded after each use of `staged`
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
     cmd::HostScratch host_scratch; // pinned staging
     uint32_t *tile_counter = nullptr;

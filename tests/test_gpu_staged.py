@@ -150,3 +150,42 @@ def test_small_batches_on_two_streams(engine):
             assert torch.equal(err, want[first:first + n]) and torch.equal(w, want_w[first:first + n]), (first, n)
     finally:
         key.free()
+
+
+def test_mixed_batches_on_two_streams(engine):
+    """Mixed batches in flight on two streams, of the sizes of all three kinds of
+    kernels, each with its own order of the keys, rewrite the work lists in turn."""
+    sets = [348864, 6960119, 460896]
+    keys = [cmd.Key(engine, s, golden_sk(s)) for s in sets]
+    try:
+        pool = [batch(s, 300)[1] for s in sets]
+        want = [run(engine, k, c, "plain") for k, c in zip(keys, pool)]
+        torch.cuda.synchronize()
+        rng = np.random.default_rng(11)
+        jobs = []
+        for n in (20000, 40000, 3000, 40000, 10000, 30000):
+            ki = rng.integers(0, 3, n).astype(np.uint32)
+            at = torch.from_numpy(rng.integers(0, 300, n)).cuda()
+            ct = np.array([k.info.ct_bytes for k in keys], np.uint64)[ki]
+            nw = np.array([k.info.err_words for k in keys], np.uint64)[ki]
+            off, eoff = (np.cumsum(ct) - ct).astype(np.uint64), (np.cumsum(nw) - nw).astype(np.uint64)
+            buf = torch.zeros(int(ct.sum()), dtype=torch.uint8, device="cuda")
+            expect = torch.zeros(int(nw.sum()), dtype=torch.int32, device="cuda")
+            for k in range(3):
+                m = ki == k
+                rows = at[torch.from_numpy(m).cuda()]
+                for dst, src, o in ((buf, pool[k], off), (expect, want[k][0], eoff)):
+                    w = torch.arange(src.shape[1], device="cuda")
+                    dst[(torch.from_numpy(o[m].astype(np.int64)).cuda()[:, None] + w).reshape(-1)] = src[rows].reshape(-1)
+            jobs.append((ki, buf, off, torch.full_like(expect, -1), eoff, expect))
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        torch.cuda.synchronize()
+        for i, (ki, buf, off, err, eoff, _) in enumerate(jobs):
+            cmd.decrypt_mixed_device(engine, keys, ki, buf.data_ptr(), off, err.data_ptr(), eoff, 0,
+                                     streams[i % 2].cuda_stream)
+        torch.cuda.synchronize()
+        for i, job in enumerate(jobs):
+            assert torch.equal(job[3], job[5]), i
+    finally:
+        for k in keys:
+            k.free()
