@@ -36,14 +36,6 @@ void HostScratch::release()
     cap = 0;
 }
 
-int ensure_counter(cmd_engine *eng)
-{
-    if (eng->tile_counter)
-        return CMD_OK;
-    cudaError_t e = cudaMalloc(&eng->tile_counter, 256);
-    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "cudaMalloc(counter)");
-}
-
 // Persistent grid: resident CTAs per SM (occupancy with this smem) x SMs,
 // never more CTAs than rounds.
 static int grid_for(cmd_engine *eng, int single_set, int wpb, size_t smem, uint64_t rounds)
@@ -134,9 +126,6 @@ cudaError_t fused_prepare(cmd_engine *eng, int set)
 int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                      uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos)
 {
-    int rc = ensure_counter(eng);
-    if (rc)
-        return rc;
     return run_fused_counter(eng, key, d_cts, count, d_err, d_weight, s, eng->tile_counter, d_pos, -1);
 }
 
@@ -373,21 +362,13 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
     for (size_t k = 0; k < nkeys; k++)
         krefs[k] = key_ref(keys[k]->dev);
 
-    int rc = 0;
-    if ((rc = [&] {
-            if (eng->tile_counter)
-                return CMD_OK;
-            cudaError_t e = cudaMalloc(&eng->tile_counter, 256);
-            return e == cudaSuccess ? CMD_OK : cuda_fail(e, "cudaMalloc(counter)");
-        }()))
-        return rc;
     // One device block for the work lists; pageable sources, so each copy has
     // consumed its host buffer when cudaMemcpyAsync returns.
     const size_t b_order = count * 4, b_off = count * 8, b_tiles = tiles.size() * sizeof(FusedTile),
                  b_keys = nkeys * sizeof(FusedKeyRef);
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
     const size_t need = al(b_order) + 2 * al(b_off) + al(b_tiles) + al(b_keys);
-    if ((rc = eng->fused.begin(eng, need, s)))
+    if (const int rc = eng->fused.begin(eng, need, s))
         return rc;
     uint8_t *base = static_cast<uint8_t *>(eng->fused.ptr);
     uint32_t *d_order = reinterpret_cast<uint32_t *>(base);

@@ -211,12 +211,20 @@ int cmd_engine_create(int device, size_t hbm_budget_bytes, cmd_engine **out)
         return cuda_fail(e, "cudaStreamCreate");
     }
     snprintf(eng->gpu_name, sizeof eng->gpu_name, "%s", prop.name);
+    // now, since a launch may be captured, when nothing can be allocated
+    if ((e = cudaMalloc(&eng->tile_counter, TILE_COUNTERS * 4)) != cudaSuccess) {
+        cudaStreamDestroy(eng->stream);
+        delete eng;
+        return cuda_fail(e, "cudaMalloc(counters)");
+    }
     if (int rc = noalloc_setup(device)) {
+        cudaFree(eng->tile_counter);
         cudaStreamDestroy(eng->stream);
         delete eng;
         return rc;
     }
     if (int rc = upload_fft_plans(eng)) {
+        cudaFree(eng->tile_counter);
         cudaStreamDestroy(eng->stream);
         delete eng;
         return rc;
@@ -248,8 +256,7 @@ void cmd_engine_destroy(cmd_engine *eng)
     for (cudaEvent_t ev : eng->staged_join)
         if (ev)
             cudaEventDestroy(ev);
-    if (eng->tile_counter)
-        cudaFree(eng->tile_counter);
+    cudaFree(eng->tile_counter);
     cudaStreamDestroy(eng->stream);
     delete eng;
 }
@@ -719,12 +726,8 @@ int cmd_decrypt_batch(cmd_engine *eng, const cmd_key *key, cmd_path path, const 
     // packed rows there directly: the rows cross PCIe while the kernels run,
     // instead of in a copy after the last piece's kernel.
     uint8_t *err_view = pieces ? device_view(h_err, count * (size_t)(si.n / 8)) : nullptr;
-    if (pieces) {
-        if ((rc = ensure_counter(eng)))
-            return rc;
-        if ((rc = ensure_piece_streams(eng)))
-            return rc;
-    }
+    if (pieces && (rc = ensure_piece_streams(eng)))
+        return rc;
     for (size_t c0 = 0; c0 < count; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
         if (pieces) {
@@ -818,12 +821,8 @@ int cmd_decrypt_positions(cmd_engine *eng, const cmd_key *key, const uint8_t *h_
     uint16_t *d_pos = cv.take<uint16_t>(chunk * row);
     cudaStream_t s = eng->stream;
     const bool pieces = chunk >= (size_t)BATCH_STREAMS * 8192;
-    if (pieces) {
-        if ((rc = ensure_counter(eng)))
-            return rc;
-        if ((rc = ensure_piece_streams(eng)))
-            return rc;
-    }
+    if (pieces && (rc = ensure_piece_streams(eng)))
+        return rc;
     for (size_t c0 = 0; c0 < count; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
         if (pieces) {  // as in cmd_decrypt_batch

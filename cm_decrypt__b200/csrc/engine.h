@@ -88,7 +88,7 @@ int run_fused_counter(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts,
 // Ciphertexts per round of one launch over `count` ciphertexts of `set` under
 // the tuned schedule.
 uint32_t fused_round(cmd_engine *eng, int set, size_t count);
-int ensure_counter(cmd_engine *eng);  // eng->tile_counter: 64 u32 work counters
+constexpr int TILE_COUNTERS = 64;     // u32 of cmd_engine::tile_counter
 constexpr int BATCH_STREAMS = 8;      // pieces of a host-buffer batch in flight
 constexpr int STAGED_STREAMS = 4;     // parts of a staged device batch in flight
 int ensure_piece_streams(cmd_engine *eng);
@@ -126,7 +126,7 @@ struct cmd_engine {
     cudaEvent_t staged_fork = nullptr, staged_join[cmd::STAGED_STREAMS] = {};  // created on first use
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
     cmd::HostScratch host_scratch; // pinned staging
-    uint32_t *tile_counter = nullptr;
+    uint32_t *tile_counter = nullptr;  // the fused kernel's work counters
     cudaStream_t piece_stream[cmd::BATCH_STREAMS] = {};  // host-buffer batches, created on first use
     std::atomic<uint64_t> launches{0};
     cmd::FusedConfig fcfg[cmd::NSETS];

@@ -195,11 +195,6 @@ int cmd_tune(cmd_engine *eng, const cmd_key *key, size_t sample_count, int force
         return rc;
     uint8_t *d_cts = static_cast<uint8_t *>(eng->io.ptr);
     uint32_t *d_err = reinterpret_cast<uint32_t *>(d_cts + (sample_count * si.ct + 255) / 256 * 256);
-    if (!eng->tile_counter) {
-        cudaError_t e = cudaMalloc(&eng->tile_counter, 256);
-        if (e != cudaSuccess)
-            return cuda_fail(e, "cudaMalloc(counter)");
-    }
     cudaStream_t s = eng->stream;
     cudaError_t e = cudaMemsetAsync(d_cts, 0xA5, sample_count * si.ct, s);
     if (e != cudaSuccess)

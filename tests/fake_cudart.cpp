@@ -127,7 +127,12 @@ size_t fake_allocated()
         n += b.second;
     return n;
 }
-void fake_clear() { ops.clear(); }
+void fake_clear()
+{
+    ops.clear();
+    for (Stream *s : streams)
+        s->capture = 0;
+}
 const char *fake_ops()
 {
     std::lock_guard<std::recursive_mutex> lk(mu);

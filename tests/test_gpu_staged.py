@@ -189,3 +189,25 @@ def test_mixed_batches_on_two_streams(engine):
     finally:
         for k in keys:
             k.free()
+
+
+@pytest.mark.parametrize("count", [40, 5000])
+def test_capture_after_an_auto_warm_up_only(count):
+    """On an engine of its own, so that no other call has prepared anything."""
+    s = 348864
+    info, cts = batch(s, count)
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, s, golden_sk(s))
+        try:
+            want, _ = run(eng, key, cts, "auto")
+            err = torch.zeros_like(want)
+            torch.cuda.synchronize()
+            graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            with torch.cuda.graph(graph, stream=side):
+                cmd.decrypt_device(eng, key, cts.data_ptr(), count, err.data_ptr(), 0, side.cuda_stream)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(err, want)
+            del graph
+        finally:
+            key.free()

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from conftest import golden_sk
-from fake_cuda import Fake
+from fake_cuda import GLOBAL_CAPTURE, Fake
 
 
 @pytest.fixture(scope="module")
@@ -51,3 +51,17 @@ def test_mixed_lists_are_rewritten_after_their_last_use(fake, first, then):
                 assert all(o.after(k) for k in kernels), (o.name, o.dst)
         for k in keys:
             k.free()
+
+
+@pytest.mark.parametrize("count", [1, 3000, 5000, 30000, 70000])
+def test_auto_is_captured_after_a_warm_up_of_its_own(fake, count):
+    """In the default capture mode, where an allocation would end the capture."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key, s = cmd.Key(eng, 348864, golden_sk(348864)), fake.stream()
+        cmd.decrypt_device(eng, key, 0x1000, count, 0x1000, 0x1000, s)
+        fake.begin_capture(s, GLOBAL_CAPTURE)
+        cmd.decrypt_device(eng, key, 0x1000, count, 0x1000, 0x1000, s)
+        cmd.decrypt_positions_device(eng, key, 0x1000, count, 0x1000, s)
+        assert fake.end_capture(s) == 0
+        key.free()
