@@ -36,6 +36,41 @@ void HostScratch::release()
     cap = 0;
 }
 
+int TileCounter::begin(cmd_engine *eng, cudaStream_t s)
+{
+    cudaError_t e = cudaSuccess;
+    if (capturing(s)) {
+        constexpr unsigned BLOCK = 256;
+        if (eng->graph_counters_left == 0) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // cudaMalloc takes no part in the capture
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            void *p = nullptr;
+            e = cudaMalloc(&p, BLOCK * 4);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess)
+                return cuda_fail(e, "cudaMalloc(counters)");
+            eng->graph_counters.push_back(static_cast<uint32_t *>(p));
+            eng->graph_counters_left = BLOCK;
+        }
+        ptr = eng->graph_counters.back() + --eng->graph_counters_left;
+        return CMD_OK;
+    }
+    const unsigned i = eng->counter_next++ % COUNTER_RING;
+    if (!eng->counter_done[i])
+        e = cudaEventCreateWithFlags(&eng->counter_done[i], cudaEventDisableTiming);
+    else
+        e = cudaStreamWaitEvent(s, eng->counter_done[i]);
+    ptr = eng->tile_counter + COUNTER_RING0 + i;
+    done = eng->counter_done[i];
+    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "work counter");
+}
+
+int TileCounter::end(cudaStream_t s, int rc)
+{
+    const cudaError_t e = done ? cudaEventRecord(done, s) : cudaSuccess;
+    return rc ? rc : e == cudaSuccess ? CMD_OK : cuda_fail(e, "work counter");
+}
+
 // Persistent grid: resident CTAs per SM (occupancy with this smem) x SMs,
 // never more CTAs than rounds.
 static int grid_for(cmd_engine *eng, int single_set, int wpb, size_t smem, uint64_t rounds)
@@ -126,7 +161,9 @@ cudaError_t fused_prepare(cmd_engine *eng, int set)
 int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                      uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos)
 {
-    return run_fused_counter(eng, key, d_cts, count, d_err, d_weight, s, eng->tile_counter, d_pos, -1);
+    TileCounter counter;
+    const int rc = counter.begin(eng, s);
+    return rc ? rc : counter.end(s, run_fused_counter(eng, key, d_cts, count, d_err, d_weight, s, counter.ptr, d_pos, -1));
 }
 
 // Set shared by every ciphertext of a mixed batch, or -1.
@@ -368,7 +405,9 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
                  b_keys = nkeys * sizeof(FusedKeyRef);
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
     const size_t need = al(b_order) + 2 * al(b_off) + al(b_tiles) + al(b_keys);
-    if (const int rc = eng->fused.begin(eng, need, s))
+    TileCounter counter;
+    int rc;
+    if ((rc = counter.begin(eng, s)) || (rc = eng->fused.begin(eng, need, s)))
         return rc;
     uint8_t *base = static_cast<uint8_t *>(eng->fused.ptr);
     uint32_t *d_order = reinterpret_cast<uint32_t *>(base);
@@ -382,8 +421,8 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
         (e = cudaMemcpyAsync(d_err_off, h_err_off, b_off, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(d_tiles, tiles.data(), b_tiles, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
         (e = cudaMemcpyAsync(d_keys, krefs.data(), b_keys, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(eng->tile_counter, 0, sizeof(uint32_t), s)) != cudaSuccess)
-        return eng->fused.end(s, e);
+        (e = cudaMemsetAsync(counter.ptr, 0, sizeof(uint32_t), s)) != cudaSuccess)
+        return counter.end(s, eng->fused.end(s, e));
     FusedArgs a;
     memset(&a, 0, sizeof a);
     a.tiles = d_tiles;
@@ -395,7 +434,7 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
     a.order = d_order;
     a.err = d_err;
     a.weight = d_weight;
-    a.tile_counter = eng->tile_counter;
+    a.tile_counter = counter.ptr;
     a.single_set = single;
     fill_fft(a, eng);
     size_t smem = 0;
@@ -406,5 +445,5 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
             smem = std::max(smem, fused_smem(st, wpb));
     const int grid = grid_for(eng, single, wpb, smem, tiles.size());
     e = launch_fused(a, grid, wpb, s, LaunchCounter{&eng->launches});
-    return eng->fused.end(s, e);
+    return counter.end(s, eng->fused.end(s, e));
 }

@@ -67,7 +67,7 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes)
     return CMD_OK;
 }
 
-static bool capturing(cudaStream_t s)
+bool capturing(cudaStream_t s)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) == cudaSuccess)
@@ -257,6 +257,11 @@ void cmd_engine_destroy(cmd_engine *eng)
         if (ev)
             cudaEventDestroy(ev);
     cudaFree(eng->tile_counter);
+    for (cudaEvent_t ev : eng->counter_done)
+        if (ev)
+            cudaEventDestroy(ev);
+    for (uint32_t *block : eng->graph_counters)
+        cudaFree(block);
     cudaStreamDestroy(eng->stream);
     delete eng;
 }

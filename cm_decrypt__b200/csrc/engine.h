@@ -88,8 +88,21 @@ int run_fused_counter(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts,
 // Ciphertexts per round of one launch over `count` ciphertexts of `set` under
 // the tuned schedule.
 uint32_t fused_round(cmd_engine *eng, int set, size_t count);
-constexpr int TILE_COUNTERS = 64;     // u32 of cmd_engine::tile_counter
 constexpr int BATCH_STREAMS = 8;      // pieces of a host-buffer batch in flight
+// cmd_engine::tile_counter: one u32 for calls that wait for their launches, one a
+// piece of theirs, then a ring for launches on callers' streams.
+constexpr int COUNTER_RING = 16, COUNTER_RING0 = 1 + BATCH_STREAMS, TILE_COUNTERS = COUNTER_RING0 + COUNTER_RING;
+bool capturing(cudaStream_t s);
+// Around a fused launch on a caller's stream: a work counter that no other launch in
+// flight uses, the next of the ring once its last launch has ended.  Under capture
+// the counter stays the captured launch's own, since a graph may be replayed at
+// any time.
+struct TileCounter {
+    uint32_t *ptr = nullptr;
+    cudaEvent_t done = nullptr;  // null under capture
+    int begin(cmd_engine *eng, cudaStream_t s);
+    int end(cudaStream_t s, int rc);  // also after an error rc
+};
 constexpr int STAGED_STREAMS = 4;     // parts of a staged device batch in flight
 int ensure_piece_streams(cmd_engine *eng);
 size_t fused_smem(int set, int wpb);
@@ -127,6 +140,10 @@ struct cmd_engine {
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
     cmd::HostScratch host_scratch; // pinned staging
     uint32_t *tile_counter = nullptr;  // the fused kernel's work counters
+    cudaEvent_t counter_done[cmd::COUNTER_RING] = {};  // created on first use
+    unsigned counter_next = 0;
+    std::vector<uint32_t *> graph_counters;  // blocks of counters of captured launches
+    unsigned graph_counters_left = 0;        // in the last block
     cudaStream_t piece_stream[cmd::BATCH_STREAMS] = {};  // host-buffer batches, created on first use
     std::atomic<uint64_t> launches{0};
     cmd::FusedConfig fcfg[cmd::NSETS];

@@ -211,3 +211,35 @@ def test_capture_after_an_auto_warm_up_only(count):
             del graph
         finally:
             key.free()
+
+
+def test_fused_batches_on_two_streams(engine):
+    """Batches of the sizes that CMD_PATH_AUTO gives to the fused kernel, and a
+    captured one, each with its own work counter."""
+    s = 348864
+    info, cts = batch(s, 60000)
+    key = cmd.Key(engine, s, golden_sk(s))
+    try:
+        want, want_w = run(engine, key, cts, "plain")
+        streams = [torch.cuda.Stream() for _ in range(3)]
+        jobs = [(n, path) for n, path in ((30000, "auto"), (37888, "auto"), (500, "fused"), (60000, "auto"))] * 6
+        outs = [(torch.zeros((n, info.err_words), dtype=torch.int32, device="cuda"),
+                 torch.zeros(n, dtype=torch.int16, device="cuda")) for n, _ in jobs]
+        graph_err = torch.zeros((5000, info.err_words), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[2]):
+            cmd.decrypt_device(engine, key, cts.data_ptr(), 5000, graph_err.data_ptr(), 0, streams[2].cuda_stream)
+        torch.cuda.synchronize()
+        for i, ((n, path), (err, w)) in enumerate(zip(jobs, outs)):
+            cmd.decrypt_device(engine, key, cts.data_ptr(), n, err.data_ptr(), w.data_ptr(), streams[i % 2].cuda_stream,
+                               path)
+            if i % 4 == 0:
+                with torch.cuda.stream(streams[2]):
+                    graph.replay()
+        torch.cuda.synchronize()
+        for (n, path), (err, w) in zip(jobs, outs):
+            assert torch.equal(err, want[:n]) and torch.equal(w, want_w[:n]), (n, path)
+        assert torch.equal(graph_err, want[:5000])
+    finally:
+        key.free()

@@ -65,3 +65,54 @@ def test_auto_is_captured_after_a_warm_up_of_its_own(fake, count):
         cmd.decrypt_positions_device(eng, key, 0x1000, count, 0x1000, s)
         assert fake.end_capture(s) == 0
         key.free()
+
+
+def fused_calls(fake, eng, key, stream):
+    """Every kind of call that may take the fused kernel, one after the other."""
+    cmd = fake.cmd
+    yield lambda: cmd.decrypt_device(eng, key, 0x1000, 30000, 0x1000, 0, stream)
+    yield lambda: cmd.decrypt_device(eng, key, 0x1000, 500, 0x1000, 0, stream, "fused")
+    yield lambda: cmd.decrypt_positions_device(eng, key, 0x1000, 37888, 0x1000, stream)
+    yield lambda: mixed(fake, eng, [key], np.zeros(40000), stream)
+
+
+def test_a_fused_launch_has_its_work_counter_to_itself(fake):
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, 348864, golden_sk(348864))
+        n = 0
+        for i in range(30):
+            for job in fused_calls(fake, eng, key, fake.stream()):
+                fake.call(n := n + 1)
+                job()
+        ops = fake.ops()
+        zeroed = [o for o in ops if o.name == "memset"]
+        kernel = {o.call: o for o in ops if "k_fused" in o.name}
+        assert len(zeroed) == n == len(kernel)
+        for i, m in enumerate(zeroed):
+            for before in zeroed[:i]:
+                assert not m.writes(before) or m.after(kernel[before.call]), (before.call, m.call)
+        # launches on different streams do not wait for one another needlessly
+        assert not zeroed[4].after(kernel[1])
+        key.free()
+
+
+def test_a_captured_launch_keeps_its_work_counter(fake):
+    """A graph zeroes its counter at every replay: no other launch may use it."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, 348864, golden_sk(348864))
+        streams, live = [fake.stream() for _ in range(2)], 0
+        for i in range(2000):
+            s = streams[i % 2]
+            fake.call(i % 2)
+            if i % 2:
+                fake.begin_capture(s, GLOBAL_CAPTURE)
+                cmd.decrypt_device(eng, key, 0x1000, 5000, 0x1000, 0, s)
+                assert fake.end_capture(s) == 0
+            else:
+                cmd.decrypt_device(eng, key, 0x1000, 30000, 0x1000, 0, s)
+        zeroed = [o for o in fake.ops() if o.name == "memset"]
+        captured = {o.dst for o in zeroed if o.call == 1}
+        assert len(captured) == 1000 and not captured & {o.dst for o in zeroed if o.call == 0}
+        key.free()
