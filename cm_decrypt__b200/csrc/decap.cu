@@ -372,16 +372,18 @@ int cmd_kem_decap_device(cmd_engine *eng, cmd_key *key, const uint8_t *d_cts, si
     std::lock_guard<std::mutex> lk(eng->mu);
     cudaStream_t s = stream ? (cudaStream_t)stream : eng->stream;
     const size_t words = count * si.nw;
-    if ((rc = eng->scratch.reserve(eng, words * 4 + count * 2 + 256)))
+    if ((rc = eng->scratch.begin(eng, words * 4 + count * 2 + 256, s)))
         return rc;
     uint32_t *d_err = static_cast<uint32_t *>(eng->scratch.ptr);
     uint16_t *d_w = reinterpret_cast<uint16_t *>(d_err + words);
-    if ((rc = run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)))
-        return rc;
-    const uint8_t *d_s = key->dev.sk + 40 + 2 * si.t + si.cond;
-    cudaError_t e = launch_decap(key->dev.set, d_cts, d_err, d_w, key->pk, d_s, d_keys, d_accept, count, s,
-                                 LaunchCounter{&eng->launches});
-    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "decapsulation kernel");
+    cudaError_t e = cudaSuccess;
+    if ((rc = run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)) == CMD_OK) {
+        const uint8_t *d_s = key->dev.sk + 40 + 2 * si.t + si.cond;
+        e = launch_decap(key->dev.set, d_cts, d_err, d_w, key->pk, d_s, d_keys, d_accept, count, s,
+                         LaunchCounter{&eng->launches});
+    }
+    const int r = eng->scratch.end(s, e);  // the rows are read up to here
+    return rc ? rc : r;
 }
 
 int cmd_kem_decap(cmd_engine *eng, cmd_key *key, const uint8_t *h_cts, size_t count, uint8_t *h_keys,

@@ -13,7 +13,7 @@
 
 namespace cmd {
 static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s, bool ordered = false);
+                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s, Scratch &buf);
 
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
@@ -417,7 +417,8 @@ int cmd_stage_synd_fft(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts
         return CMD_OK;
     cudaSetDevice(eng->device);
     std::lock_guard<std::mutex> lk(eng->mu);
-    return run_tile(eng, key, d_cts, count, nullptr, nullptr, nullptr, d_synd, stream ? (cudaStream_t)stream : eng->stream);
+    return run_tile(eng, key, d_cts, count, nullptr, nullptr, nullptr, d_synd,
+                    stream ? (cudaStream_t)stream : eng->stream, eng->scratch);
 }
 
 int cmd_stage_bm(cmd_engine *eng, cmd_set set, const uint16_t *d_synd, size_t count, uint16_t *d_loc, void *stream)
@@ -473,63 +474,53 @@ static int run_plain(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, 
     const SetInfo si = set_info(key->dev.set);
     const size_t chunk = std::min<size_t>(count, (size_t)1 << 18);
     const size_t need = plain_scratch_bytes(key->dev.set, count);
-    int rc = eng->scratch.reserve(eng, need);
+    int rc = eng->scratch.begin(eng, need, s);
     if (rc)
         return rc;
     Carver cv{static_cast<uint8_t *>(eng->scratch.ptr)};
     uint32_t *synd = cv.take<uint32_t>(chunk * si.t);
     uint16_t *loc = cv.take<uint16_t>(chunk * (si.t + 1));
     LaunchCounter lc{&eng->launches};
-    for (size_t c0 = 0; c0 < count; c0 += chunk) {
+    cudaError_t e = cudaSuccess;
+    for (size_t c0 = 0; c0 < count && e == cudaSuccess; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
-        cudaError_t e;
         if ((e = launch_synd_plain(key->dev, d_cts + c0 * si.ct, n, synd, s, lc)) != cudaSuccess ||
             (e = launch_bm_plain(key->dev.set, reinterpret_cast<uint16_t *>(synd), n, loc, s, lc)) != cudaSuccess ||
             (e = launch_root_plain(key->dev, loc, n, d_err + c0 * si.nw, d_weight ? d_weight + c0 : nullptr, s, lc,
                                    eng->num_sms)) != cudaSuccess)
-            return cuda_fail(e, "plain path launch");
+            break;
     }
-    return CMD_OK;
+    return eng->scratch.end(s, e);
 }
 
 // The serving tile kernels over one key's batch, in chunks whose byte and
 // word offsets fit the tile items' 32-bit fields.  With d_synd: syndromes
-// only.  Scratch: the engine's, or (ordered) that of the staged batches, which is
-// safe with batches in flight on other streams.  Caller holds eng->mu.
+// only.  buf: the engine's scratch, or that of the staged batches.  Caller holds
+// eng->mu.
 static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
-                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s, bool ordered)
+                    uint16_t *d_weight, uint16_t *d_pos, uint16_t *d_synd, cudaStream_t s, Scratch &buf)
 {
     const SetInfo si = set_info(key->dev.set);
     const size_t chunk = std::min<size_t>(count, (size_t)1 << 22);
-    int rc = CMD_OK;
-    if (!d_synd && count <= CT_ONE_LAUNCH)  // everything stays on chip
-        ordered = false;
-    else if (ordered)
-        rc = staged_begin(eng, tile_single_scratch_words(chunk) * 4, 1, s);
-    else
-        rc = eng->scratch.reserve(eng, tile_single_scratch_words(chunk) * 4);
-    if (rc)
-        return rc;
-    uint32_t *scratch = static_cast<uint32_t *>(ordered ? eng->staged.ptr : eng->scratch.ptr);
+    const bool on_chip = !d_synd && count <= CT_ONE_LAUNCH;  // one launch, no scratch
+    if (!on_chip)
+        if (const int rc = buf.begin(eng, tile_single_scratch_words(chunk) * 4, s))
+            return rc;
+    uint32_t *scratch = on_chip ? nullptr : static_cast<uint32_t *>(buf.ptr);
     FftPlans plans;
     for (int st = 0; st < NSETS; st++)
         plans.p[st] = eng->fft[st];
-    for (size_t c0 = 0; c0 < count; c0 += chunk) {
+    cudaError_t e = cudaSuccess;
+    for (size_t c0 = 0; c0 < count && e == cudaSuccess; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
-        const cudaError_t e = launch_tile_single(
+        e = launch_tile_single(
             key->dev, d_cts + c0 * si.ct, n, scratch, d_err ? d_err + c0 * si.nw : nullptr,
             d_weight ? d_weight + c0 : nullptr, d_pos,
             d_synd ? d_synd + c0 * 2 * si.t : nullptr, plans, eng->num_sms, s, LaunchCounter{&eng->launches});
-        if (e != cudaSuccess) {
-            rc = cuda_fail(e, "tile path launch");
-            break;
-        }
     }
-    if (ordered) {  // also after an error
-        const int r = staged_end(eng, 1, s, cudaSuccess);
-        return rc ? rc : r;
-    }
-    return rc;
+    if (!on_chip)
+        return buf.end(s, e);
+    return e == cudaSuccess ? CMD_OK : cuda_fail(e, "tile path launch");
 }
 
 int ensure_piece_streams(cmd_engine *eng)
@@ -633,7 +624,7 @@ static int run_auto(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
     const int set = key->dev.set;
     if (!capturing(s)) {
         if (takes_small(eng, set, count) && (!d_pos || count <= (size_t)CT_PER_SM * eng->num_sms)) {
-            const int rc = run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s, true);
+            const int rc = run_tile(eng, key, d_cts, count, d_err, d_weight, d_pos, nullptr, s, eng->staged);
             if (rc != CMD_E_BUDGET)
                 return rc;
         } else if (count <= 192 * (size_t)eng->num_sms || count > 256 * (size_t)eng->num_sms) {
@@ -654,7 +645,7 @@ int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t
     if (path == CMD_PATH_PLAIN)
         return run_plain(eng, key, d_cts, count, d_err, d_weight, s);
     if (path == CMD_PATH_TILE)
-        return run_tile(eng, key, d_cts, count, d_err, d_weight, nullptr, nullptr, s);
+        return run_tile(eng, key, d_cts, count, d_err, d_weight, nullptr, nullptr, s, eng->scratch);
     if (path == CMD_PATH_AUTO)
         return run_auto(eng, key, d_cts, count, d_err, d_weight, d_pos, s);
     return run_fused_single(eng, key, d_cts, count, d_err, d_weight, s);

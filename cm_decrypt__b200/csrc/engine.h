@@ -131,7 +131,7 @@ struct cmd_engine {
     std::atomic<size_t> used{0};
     cudaStream_t stream = nullptr;
     std::mutex mu;                 // serialises calls that share scratch
-    cmd::Scratch scratch;          // plain-path intermediates
+    cmd::Scratch scratch;          // intermediates of the plain and tile paths, a decapsulation's error rows
     cmd::Scratch io;               // device staging for host-buffer calls
     cmd::Scratch fused;            // fused-kernel work lists
     cmd::Scratch staged;           // staged kernels' intermediates, one part per piece stream,

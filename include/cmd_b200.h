@@ -402,8 +402,8 @@ int cmd_engine_set_fused_config(cmd_engine *eng, cmd_set set, int wpb, int balan
 /* A decrypt over fixed device buffers captured as a CUDA graph and replayed
  * with cmd_graph_launch (asynchronous on `stream`, NULL = engine stream).
  * A fused-path graph owns its work counter; a plain-path graph uses the
- * engine's scratch, so do not replay it concurrently with other plain-path
- * work of the same engine. */
+ * engine's scratch, so do not replay it concurrently with plain-path,
+ * tile-path or decapsulation work of the same engine. */
 typedef struct cmd_graph cmd_graph;
 int cmd_graph_capture(cmd_engine *eng, const cmd_key *key, cmd_path path,
                       const uint8_t *d_cts, size_t count, uint32_t *d_err,

@@ -243,3 +243,34 @@ def test_fused_batches_on_two_streams(engine):
         assert torch.equal(graph_err, want[:5000])
     finally:
         key.free()
+
+
+@pytest.mark.parametrize("s,n", [(348864, 20000), (6688128, 3000)])
+def test_decapsulations_on_two_streams(engine, s, n):
+    """Beside one another and beside tile- and plain-path batches, which use the
+    same scratch; also the 6688128 set at staged sizes."""
+    info, cts = batch(s, 2 * n)
+    key = cmd.Key(engine, s, golden_sk(s))
+    try:
+        want = cmd.kem_decap(engine, key, cts.cpu().numpy())
+        rows, _ = run(engine, key, cts, "fused")
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        outs = [(torch.zeros((n, 32), dtype=torch.uint8, device="cuda"), torch.zeros(n, dtype=torch.uint8, device="cuda"))
+                for _ in range(6)]
+        errs = [torch.zeros((700, info.err_words), dtype=torch.int32, device="cuda") for _ in range(6)]
+        torch.cuda.synchronize()
+        for i in range(6):
+            half = cts[i % 2 * n:]
+            cmd.kem_decap_device(engine, key, half.data_ptr(), n, outs[i][0].data_ptr(), outs[i][1].data_ptr(),
+                                 streams[i % 2].cuda_stream)
+            cmd.decrypt_device(engine, key, half.data_ptr(), 700, errs[i].data_ptr(), 0, streams[i % 2].cuda_stream,
+                               "plain" if i % 3 else "tile")
+        torch.cuda.synchronize()
+        for i, ((k, a), err) in enumerate(zip(outs, errs)):
+            at = i % 2 * n
+            assert np.array_equal(k.cpu().numpy(), want[0][at:at + n]), i
+            assert np.array_equal(a.cpu().numpy(), want[1][at:at + n]), i
+            assert torch.equal(err, rows[at:at + 700]), i
+        assert want[1].any() and not want[1].all()
+    finally:
+        key.free()

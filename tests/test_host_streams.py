@@ -116,3 +116,30 @@ def test_a_captured_launch_keeps_its_work_counter(fake):
         captured = {o.dst for o in zeroed if o.call == 1}
         assert len(captured) == 1000 and not captured & {o.dst for o in zeroed if o.call == 0}
         key.free()
+
+
+@pytest.mark.parametrize("first", ["decap", "plain", "tile", "tile_small", "synd"])
+@pytest.mark.parametrize("then", ["decap", "plain", "tile", "tile_small", "synd"])
+def test_the_engines_scratch_is_reused_after_its_last_use(fake, first, then):
+    """Error rows of a decapsulation, intermediates of the plain and tile paths."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, 348864, golden_sk(348864))
+        cmd.prepare_decap(eng, key)
+        jobs = {"decap": lambda s: cmd.kem_decap_device(eng, key, 0x1000, 20000, 0x1000, 0x1000, s),
+                "plain": lambda s: cmd.decrypt_device(eng, key, 0x1000, 300, 0x1000, 0, s, "plain"),
+                "tile": lambda s: cmd.decrypt_device(eng, key, 0x1000, 5000, 0x1000, 0, s, "tile"),
+                "tile_small": lambda s: cmd.decrypt_device(eng, key, 0x1000, 100, 0x1000, 0, s, "tile"),
+                "synd": lambda s: cmd.lib().cmd_stage_synd_fft(eng.handle, key.handle, 0x1000, 40, 0x1000, s)}
+        a, b = fake.stream(), fake.stream()
+        jobs["tile"](a)  # grown: no call below moves it
+        jobs["decap"](a)
+        fake.call(1)
+        jobs[first](a)
+        fake.call(2)
+        jobs[then](b)
+        ops = fake.ops()
+        one, two = ([o for o in ops if o.call == i] for i in (1, 2))
+        assert one and two
+        assert all(o.after(one[-1]) for o in two)
+        key.free()
