@@ -258,7 +258,7 @@ static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t 
     size_t words[NSETS + 1] = {};
     for (int st = 0; st < NSETS; st++)
         words[st + 1] = words[st] + staged_scratch_words(st, 32 * (size_t)(p.tile0[st + 1] - p.tile0[st]));
-    int rc = eng->staged.reserve(eng, words[NSETS] * 4);
+    int rc = eng->staged.reserve(eng, words[NSETS] * 4, CMD_E_BUDGET);
     if (rc)
         return rc;
     if (eng->fused.begin(eng, b_order + 2 * b_off + b_blk + b_tile + b_keys, s) != CMD_OK)

@@ -41,7 +41,7 @@ bool budget_take(cmd_engine *eng, size_t bytes)
 }
 void budget_give(cmd_engine *eng, size_t bytes) { eng->used.fetch_sub(bytes); }
 
-int Scratch::reserve(cmd_engine *eng, size_t bytes)
+int Scratch::reserve(cmd_engine *eng, size_t bytes, int no_memory)
 {
     if (bytes <= cap)
         return CMD_OK;
@@ -61,7 +61,11 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes)
         budget_give(eng, want - cap);
         budget_give(eng, cap);
         cap = 0;
-        return cuda_fail(e, "cudaMalloc(scratch)");
+        const int rc = cuda_fail(e, "cudaMalloc(scratch)");
+        if (e != cudaErrorMemoryAllocation || no_memory == rc)
+            return rc;
+        cudaGetLastError();
+        return no_memory;
     }
     cap = want;
     return CMD_OK;
@@ -76,9 +80,9 @@ bool capturing(cudaStream_t s)
     return true;
 }
 
-int Scratch::begin(cmd_engine *eng, size_t bytes, cudaStream_t s)
+int Scratch::begin(cmd_engine *eng, size_t bytes, cudaStream_t s, int no_memory)
 {
-    const int rc = reserve(eng, bytes);
+    const int rc = reserve(eng, bytes, no_memory);
     if (rc || !done || capturing(s))
         return rc;
     const cudaError_t e = cudaStreamWaitEvent(s, done);
@@ -504,7 +508,8 @@ static int run_tile(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, s
     const size_t chunk = std::min<size_t>(count, (size_t)1 << 22);
     const bool on_chip = !d_synd && count <= CT_ONE_LAUNCH;  // one launch, no scratch
     if (!on_chip)
-        if (const int rc = buf.begin(eng, tile_single_scratch_words(chunk) * 4, s))
+        if (const int rc = buf.begin(eng, tile_single_scratch_words(chunk) * 4, s,
+                                     &buf == &eng->staged ? CMD_E_BUDGET : CMD_E_CUDA))
             return rc;
     uint32_t *scratch = on_chip ? nullptr : static_cast<uint32_t *>(buf.ptr);
     FftPlans plans;
@@ -549,7 +554,7 @@ static size_t staged_part(size_t count)
 
 int staged_begin(cmd_engine *eng, size_t bytes, int ns, cudaStream_t s)
 {
-    int rc = eng->staged.begin(eng, bytes, s);
+    int rc = eng->staged.begin(eng, bytes, s, CMD_E_BUDGET);
     if (rc || ns == 1)
         return rc;
     if ((rc = ensure_piece_streams(eng)))
@@ -615,9 +620,9 @@ static bool takes_small(const cmd_engine *eng, int set, size_t count)
 // small-batch kernels, else the staged ones.  The fused kernel takes batches of
 // six to eight tiles an SM, one nearly full round of its warps (37,888
 // mceliece6960119 ciphertexts 1,485 us, staged 1,534 us); needing no scratch, it
-// also runs when theirs does not fit the budget, and under stream capture, where
-// nothing may be allocated and a graph would keep the address of scratch that can
-// grow.
+// also runs when theirs does not fit the budget or the device's free memory, and
+// under stream capture, where nothing may be allocated and a graph would keep the
+// address of scratch that can grow.
 static int run_auto(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                     uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s)
 {

@@ -20,11 +20,13 @@ struct Scratch {
     void *ptr = nullptr;
     size_t cap = 0;
     cudaEvent_t done = nullptr;  // after the last use between begin and end
-    int reserve(cmd_engine *eng, size_t bytes);
+    // no_memory: returned when the budget allows the growth but the device's memory
+    // does not (others use it, too); CMD_E_BUDGET from callers that can do without.
+    int reserve(cmd_engine *eng, size_t bytes, int no_memory = CMD_E_CUDA);
     // Around work on a caller's stream that uses the buffer: reserves it and orders
     // s after its last use on any stream; marks this use (also after an error e).
     // A stream under capture neither waits nor marks.
-    int begin(cmd_engine *eng, size_t bytes, cudaStream_t s);
+    int begin(cmd_engine *eng, size_t bytes, cudaStream_t s, int no_memory = CMD_E_CUDA);
     int end(cudaStream_t s, cudaError_t e = cudaSuccess);
     void release(cmd_engine *eng);
 };
@@ -69,7 +71,8 @@ int run_device(cmd_engine *eng, const cmd_key *key, cmd_path path, const uint8_t
 int run_fused_single(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                      uint16_t *d_weight, cudaStream_t s, uint16_t *d_pos = nullptr);
 // The staged kernels over one key's device batch (see engine.cu): err/weight or
-// pos, each or null.  CMD_E_BUDGET when their scratch does not fit.
+// pos, each or null.  CMD_E_BUDGET when their scratch does not fit the budget or
+// the device.
 int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t count, uint32_t *d_err,
                uint16_t *d_weight, uint16_t *d_pos, cudaStream_t s);
 // Around staged launches on s (ns = 1) or on the first ns piece streams: reserves

@@ -130,6 +130,7 @@ size_t fake_allocated()
 void fake_clear()
 {
     ops.clear();
+    last = cudaSuccess;
     for (Stream *s : streams)
         s->capture = 0;
 }

@@ -274,3 +274,36 @@ def test_decapsulations_on_two_streams(engine, s, n):
         assert want[1].any() and not want[1].all()
     finally:
         key.free()
+
+
+def test_budget_without_room_for_scratch(engine):
+    """The staged and small-batch scratch refused: the same results from the fused
+    kernel, within the budget."""
+    s = 6960119
+    info, cts = batch(s, 50000)
+    key = cmd.Key(engine, s, golden_sk(s))
+    want, want_w = run(engine, key, cts, "fused")
+    pos = torch.zeros((50000, info.t + 1), dtype=torch.int16, device="cuda")
+    cmd.decrypt_positions_device(engine, key, cts.data_ptr(), 50000, pos.data_ptr())
+    torch.cuda.synchronize()
+    key.free()
+    with cmd.Engine(0, hbm_budget=3 << 20) as eng:
+        key = cmd.Key(eng, s, golden_sk(s))
+        try:
+            for n in (3000, 5000, 50000):
+                err, w = run(eng, key, cts, "auto", 0, n)
+                got = torch.zeros_like(pos[:n])
+                cmd.decrypt_positions_device(eng, key, cts.data_ptr(), n, got.data_ptr())
+                torch.cuda.synchronize()
+                assert torch.equal(err, want[:n]) and torch.equal(w, want_w[:n]), n
+                assert torch.equal(got, pos[:n]), n
+            for n in (3000, 5000):
+                err = torch.full((n, info.err_words), -1, dtype=torch.int32, device="cuda")
+                step = np.arange(n, dtype=np.uint64)
+                cmd.decrypt_mixed_device(eng, [key], np.zeros(n, np.uint32), cts.data_ptr(), step * info.ct_bytes,
+                                         err.data_ptr(), step * info.err_words)
+                torch.cuda.synchronize()
+                assert torch.equal(err, want[:n]), n
+            assert eng.memory()[0] <= eng.memory()[1]
+        finally:
+            key.free()
