@@ -206,12 +206,19 @@ void plan_mixed(const int *key_set, size_t nkeys, const uint32_t *key_idx, size_
 }
 
 // A mixed batch on the staged kernels, set by set: slots grouped by key, each key's
-// run cut into tiles and syndrome blocks.
+// run cut into tiles and syndrome blocks; passes of at most as many tiles as the
+// parts of a single-key batch in flight, since every key's last tile takes the scratch
+// of a full one (46 KB), however few ciphertexts it has.
+struct StagedSlice {
+    int set, pass;
+    uint32_t block0, nblocks, tile0, ntiles;
+};
 struct StagedPlan {
     std::vector<uint32_t> order;
-    std::vector<StagedPiece> blocks, tiles;  // of all sets, set by set
-    uint32_t block0[NSETS + 1] = {}, tile0[NSETS + 1] = {};
+    std::vector<StagedPiece> blocks, tiles;
+    std::vector<StagedSlice> slices;  // by pass, the costlier sets first
 };
+constexpr uint32_t STAGED_PASS_TILES = STAGED_STREAMS * 65536 / 32;
 
 static void plan_staged(const int *key_set, size_t nkeys, const uint32_t *key_idx, size_t count, StagedPlan &p)
 {
@@ -225,19 +232,29 @@ static void plan_staged(const int *key_set, size_t nkeys, const uint32_t *key_id
     for (size_t c = 0; c < count; c++)
         p.order[fill[key_idx[c]]++] = (uint32_t)c;
     constexpr uint32_t bs = 32 * staged_block_tiles;
-    for (int st = 0; st < NSETS; st++) {
+    uint32_t room = STAGED_PASS_TILES;  // tiles left in the pass
+    int pass = 0;
+    for (int st = NSETS - 1; st >= 0; st--) {
         for (size_t k = 0; k < nkeys; k++) {
             if (key_set[k] != st)
                 continue;
-            for (uint32_t r = cnt[k]; r < cnt[k + 1]; r += 32) {
-                const uint32_t left = cnt[k + 1] - r, tile = (uint32_t)p.tiles.size() - p.tile0[st];
-                if ((r - cnt[k]) % bs == 0)
-                    p.blocks.push_back(StagedPiece{(uint32_t)k, std::min(left, bs), r, tile});
-                p.tiles.push_back(StagedPiece{(uint32_t)k, std::min(left, 32u), r, 0});
+            for (uint32_t r = cnt[k]; r < cnt[k + 1]; r += bs) {
+                const uint32_t n = std::min(cnt[k + 1] - r, bs), nt = (n + 31) / 32;
+                if (nt > room) {
+                    pass++;
+                    room = STAGED_PASS_TILES;
+                }
+                if (p.slices.empty() || p.slices.back().set != st || p.slices.back().pass != pass)
+                    p.slices.push_back(StagedSlice{st, pass, (uint32_t)p.blocks.size(), 0, (uint32_t)p.tiles.size(), 0});
+                StagedSlice &sl = p.slices.back();
+                p.blocks.push_back(StagedPiece{(uint32_t)k, n, r, sl.ntiles});
+                for (uint32_t i = 0; i < n; i += 32)
+                    p.tiles.push_back(StagedPiece{(uint32_t)k, std::min(n - i, 32u), r + i, 0});
+                sl.nblocks++;
+                sl.ntiles += nt;
+                room -= nt;
             }
         }
-        p.block0[st + 1] = (uint32_t)p.blocks.size();
-        p.tile0[st + 1] = (uint32_t)p.tiles.size();
     }
 }
 
@@ -255,10 +272,14 @@ static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t 
         krefs[k] = key_ref(keys[k]->dev);
     const size_t b_order = al256(count * 4), b_off = al256(count * 8), b_blk = al256(p.blocks.size() * sizeof(StagedPiece)),
                  b_tile = al256(p.tiles.size() * sizeof(StagedPiece)), b_keys = al256(nkeys * sizeof(FusedKeyRef));
-    size_t words[NSETS + 1] = {};
-    for (int st = 0; st < NSETS; st++)
-        words[st + 1] = words[st] + staged_scratch_words(st, 32 * (size_t)(p.tile0[st + 1] - p.tile0[st]));
-    int rc = eng->staged.reserve(eng, words[NSETS] * 4, CMD_E_BUDGET);
+    size_t words = 0, at_word = 0;  // of the largest pass; of a pass so far
+    for (size_t i = 0; i < p.slices.size(); i++) {
+        if (i == 0 || p.slices[i].pass != p.slices[i - 1].pass)
+            at_word = 0;
+        at_word += staged_scratch_words(p.slices[i].set, 32 * (size_t)p.slices[i].ntiles);
+        words = std::max(words, at_word);
+    }
+    int rc = eng->staged.reserve(eng, words * 4, CMD_E_BUDGET);
     if (rc)
         return rc;
     if (eng->fused.begin(eng, b_order + 2 * b_off + b_blk + b_tile + b_keys, s) != CMD_OK)
@@ -281,24 +302,24 @@ static int run_mixed_staged(cmd_engine *eng, const cmd_key *const *keys, size_t 
     mx.keys = reinterpret_cast<const FusedKeyRef *>(put(krefs.data(), nkeys * sizeof(FusedKeyRef), b_keys));
     if (e != cudaSuccess)
         return eng->fused.end(s, e);
-    // the sets beside one another, as the parts of a single-key batch
+    // the sets of a pass beside one another, as the parts of a single-key batch
     const int ns = STAGED_STREAMS;
-    if ((rc = staged_begin(eng, words[NSETS] * 4, ns, s))) {
-        eng->fused.end(s);
-        return rc;
+    for (size_t i = 0; i < p.slices.size() && rc == CMD_OK;) {
+        if ((rc = staged_begin(eng, words * 4, ns, s)))
+            break;
+        const int pass = p.slices[i].pass;
+        uint32_t *scratch = static_cast<uint32_t *>(eng->staged.ptr);
+        for (int k = 0; i < p.slices.size() && p.slices[i].pass == pass && e == cudaSuccess; i++, k++) {
+            const StagedSlice &sl = p.slices[i];
+            StagedMixed m = mx;
+            m.blocks += sl.block0;
+            m.tiles += sl.tile0;
+            e = launch_staged_mixed(sl.set, m, sl.nblocks, sl.ntiles, d_cts, scratch, d_err, d_weight, eng->fft[sl.set],
+                                    eng->num_sms, eng->piece_stream[k % ns], LaunchCounter{&eng->launches});
+            scratch += staged_scratch_words(sl.set, 32 * (size_t)sl.ntiles);
+        }
+        rc = staged_end(eng, ns, s, e);
     }
-    for (int st = NSETS - 1, i = 0; st >= 0 && e == cudaSuccess; st--) {  // the costlier sets first
-        const uint32_t nb = p.block0[st + 1] - p.block0[st], nt = p.tile0[st + 1] - p.tile0[st];
-        if (nt == 0)
-            continue;
-        StagedMixed m = mx;
-        m.blocks += p.block0[st];
-        m.tiles += p.tile0[st];
-        e = launch_staged_mixed(st, m, nb, nt, d_cts, static_cast<uint32_t *>(eng->staged.ptr) + words[st], d_err,
-                                d_weight, eng->fft[st], eng->num_sms, eng->piece_stream[i++ % ns],
-                                LaunchCounter{&eng->launches});
-    }
-    rc = staged_end(eng, ns, s, e);
     const int r = eng->fused.end(s);
     return rc ? rc : r;
 }

@@ -307,3 +307,33 @@ def test_budget_without_room_for_scratch(engine):
             assert eng.memory()[0] <= eng.memory()[1]
         finally:
             key.free()
+
+
+def test_mixed_batch_of_many_keys(engine):
+    """A ciphertext or two a key: more tiles than one pass over the scratch holds."""
+    sets = [348864, 6960119, 8192128]
+    keys = [cmd.Key(engine, s, golden_sk(s)) for s in sets]
+    try:
+        pool = [batch(s, 200)[1] for s in sets]
+        want = [run(engine, k, c, "plain") for k, c in zip(keys, pool)]
+        n = 9500
+        many = [keys[i % 3] for i in range(n - 500)]
+        ki = np.arange(n, dtype=np.uint32) % (n - 500)
+        ct = np.array([k.info.ct_bytes for k in many], np.uint64)[ki]
+        nw = np.array([k.info.err_words for k in many], np.uint64)[ki]
+        off, eoff = (np.cumsum(ct) - ct).astype(np.uint64), (np.cumsum(nw) - nw).astype(np.uint64)
+        rows = np.arange(n) // 3 % 200
+        host = [c.cpu().numpy() for c in pool]
+        buf = torch.from_numpy(np.concatenate([host[k % 3][r] for k, r in zip(ki, rows)])).cuda()
+        err = torch.full((int(nw.sum()),), -1, dtype=torch.int32, device="cuda")
+        w = torch.full((n,), -1, dtype=torch.int16, device="cuda")
+        torch.cuda.synchronize()
+        cmd.decrypt_mixed_device(engine, many, ki, buf.data_ptr(), off, err.data_ptr(), eoff, w.data_ptr())
+        torch.cuda.synchronize()
+        e, got_w = [x[0].cpu().numpy() for x in want], w.cpu().numpy()
+        assert np.array_equal(err.cpu().numpy(), np.concatenate([e[k % 3][r] for k, r in zip(ki, rows)]))
+        we = [x[1].cpu().numpy() for x in want]
+        assert np.array_equal(got_w, np.array([we[k % 3][r] for k, r in zip(ki, rows)]))
+    finally:
+        for k in keys:
+            k.free()

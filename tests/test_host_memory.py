@@ -40,3 +40,25 @@ def test_a_full_gpu_leaves_the_fused_kernel(fake, grown):  # noqa: F811
             assert [o.name for o in fake.ops() if "k_fused" in o.name]
             assert eng.memory()[0] <= used
         key.free()
+
+
+def test_a_mixed_batchs_scratch_is_bounded(fake):  # noqa: F811
+    """By that of four parts of a single-key batch, however many keys cut the batch
+    into partly filled tiles; the passes over the scratch follow one another."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        keys = [cmd.Key(eng, s, golden_sk(s)) for s in (348864, 6960119, 8192128)]
+        cmd.decrypt_device(eng, keys[2], 0x1000, 1 << 20, 0x1000)
+        single = eng.memory()[0]
+        n = 20000
+        fake.rt.fake_clear()
+        mixed(fake, eng, [keys[i % 3] for i in range(n)], np.arange(n), 0)  # a key each
+        assert eng.memory()[0] <= single + (4 << 20)  # the work lists
+        synd, nets = ([o for o in fake.ops() if name in o.name] for name in ("k_synd_table", "k_net_rows"))
+        assert len(synd) == len(nets) == 5  # 8192128, 6960119; the rest, 348864; the rest
+        for i, o in enumerate(synd):
+            # ordered after the rows of every earlier pass, beside those of its own
+            done = [j for j, net in enumerate(nets) if o.after(net)]
+            assert done == list(range((0, 0, 2, 2, 4)[i])), i
+        for k in keys:
+            k.free()
