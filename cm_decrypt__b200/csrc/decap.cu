@@ -333,20 +333,13 @@ int cmd_key_prepare_decap(cmd_engine *eng, cmd_key *key)
     const int set = key->dev.set;
     const size_t bytes = decap_pk_words(set) * 4;
     const int rp = dispatch_set(set, [&]<int S>() { return DecapDims<S>::RP; });
-    if (!budget_take(eng, bytes)) {
-        set_last_error("public key does not fit the engine HBM budget");
-        return CMD_E_BUDGET;
-    }
-    cudaSetDevice(eng->device);
     void *p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-        budget_give(eng, bytes);
-        return cuda_fail(e, "public key columns");
-    }
+    int rc = device_alloc(eng, &p, bytes, "public key columns", "public key does not fit the engine HBM budget");
+    if (rc)
+        return rc;
     // the key's parity-check matrix from its device support and Goppa
     // polynomial, reduced on the device
-    const int rc = kg_pubkey_rows(eng, set, key->dev.L, key->dev.g, static_cast<uint32_t *>(p), rp);
+    rc = kg_pubkey_rows(eng, set, key->dev.L, key->dev.g, static_cast<uint32_t *>(p), rp);
     if (rc) {
         cudaFree(p);
         budget_give(eng, bytes);

@@ -41,12 +41,52 @@ bool budget_take(cmd_engine *eng, size_t bytes)
 }
 void budget_give(cmd_engine *eng, size_t bytes) { eng->used.fetch_sub(bytes); }
 
+// Gives the staged scratch back; false if there is none.  Caller holds eng->mu, and
+// reserves its own buffers before it begins on the staged scratch.
+static bool give_back(cmd_engine *eng)
+{
+    if (!eng->staged.ptr)
+        return false;
+    eng->staged.release(eng);
+    return true;
+}
+
+bool budget_take_first(cmd_engine *eng, size_t bytes)
+{
+    if (budget_take(eng, bytes))
+        return true;
+    std::lock_guard<std::mutex> lk(eng->mu);
+    return give_back(eng) && budget_take(eng, bytes);
+}
+
+int device_alloc(cmd_engine *eng, void **p, size_t bytes, const char *what, const char *over)
+{
+    if (!budget_take_first(eng, bytes)) {
+        set_last_error(over);
+        return CMD_E_BUDGET;
+    }
+    cudaSetDevice(eng->device);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        std::lock_guard<std::mutex> lk(eng->mu);
+        if (give_back(eng)) {
+            cudaGetLastError();
+            e = cudaMalloc(p, bytes);
+        }
+    }
+    if (e == cudaSuccess)
+        return CMD_OK;
+    budget_give(eng, bytes);
+    return cuda_fail(e, what);
+}
+
 int Scratch::reserve(cmd_engine *eng, size_t bytes, int no_memory)
 {
     if (bytes <= cap)
         return CMD_OK;
     size_t want = align_up(std::max(bytes, cap + cap / 2), 1 << 20);
-    if (!budget_take(eng, want - cap)) {
+    const bool staged = this == &eng->staged;
+    if (!budget_take(eng, want - cap) && (staged || !give_back(eng) || !budget_take(eng, want - cap))) {
         set_last_error("scratch growth exceeds the engine HBM budget");
         return CMD_E_BUDGET;
     }
@@ -57,6 +97,10 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes, int no_memory)
         ptr = nullptr;
     }
     cudaError_t e = cudaMalloc(&ptr, want);
+    if (e == cudaErrorMemoryAllocation && !staged && give_back(eng)) {
+        cudaGetLastError();
+        e = cudaMalloc(&ptr, want);
+    }
     if (e != cudaSuccess) {
         budget_give(eng, want - cap);
         budget_give(eng, cap);
@@ -300,23 +344,14 @@ int cmd_key_expand(cmd_engine *eng, cmd_set set, const uint8_t *h_sk, size_t sk_
                                      (size_t)si.sb * si.twp() * 4, (size_t)si.sb * si.twd() * 4,
                                      (size_t)si.m * si.nw * 4,
                                      benes_mask_words(si) * 4, fft_weight_words(si) * 4, (size_t)si.sk});
-    if (!budget_take(eng, bytes)) {
-        set_last_error("key does not fit the engine HBM budget");
-        return CMD_E_BUDGET;
-    }
     cmd_key *key = new (std::nothrow) cmd_key();
-    if (!key) {
-        budget_give(eng, bytes);
+    if (!key)
         return CMD_E_NOMEM;
-    }
     key->eng = eng;
     key->bytes = bytes;
-    cudaSetDevice(eng->device);
-    cudaError_t e = cudaMalloc(&key->block, bytes);
-    if (e != cudaSuccess) {
-        budget_give(eng, bytes);
+    if (const int rc = device_alloc(eng, &key->block, bytes, "cudaMalloc(key)", "key does not fit the engine HBM budget")) {
         delete key;
-        return cuda_fail(e, "cudaMalloc(key)");
+        return rc;
     }
     Carver cv{static_cast<uint8_t *>(key->block)};
     key->dev.set = set;
@@ -330,6 +365,7 @@ int cmd_key_expand(cmd_engine *eng, cmd_set set, const uint8_t *h_sk, size_t sk_
     key->dev.wfft = cv.take<uint32_t>(fft_weight_words(si));
     key->dev.sk = cv.take<uint8_t>(si.sk);
     std::lock_guard<std::mutex> lk(eng->mu);
+    cudaError_t e;
     if ((e = cudaMemcpyAsync(key->dev.sk, h_sk, si.sk, cudaMemcpyHostToDevice, eng->stream)) != cudaSuccess ||
         (e = launch_key_expand(key->dev, eng->stream, LaunchCounter{&eng->launches})) != cudaSuccess ||
         (e = cudaStreamSynchronize(eng->stream)) != cudaSuccess) {

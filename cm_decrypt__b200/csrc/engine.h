@@ -60,6 +60,12 @@ int cuda_fail(cudaError_t e, const char *what);
 int kg_pubkey_rows(cmd_engine *eng, int set, const uint16_t *d_L, const uint16_t *d_g, uint32_t *d_rows, int rp);
 bool valid_set(int set);
 bool budget_take(cmd_engine *eng, size_t bytes);
+// The same for what the engine holds longer than a call, which the scratch kept for
+// CMD_PATH_AUTO makes room for when it has to (the calls that it serves can do
+// without); and device memory so charged: CMD_E_BUDGET with the message `over`, or
+// CMD_E_CUDA.  Not with eng->mu held.
+bool budget_take_first(cmd_engine *eng, size_t bytes);
+int device_alloc(cmd_engine *eng, void **p, size_t bytes, const char *what, const char *over);
 // Device address of GPU-mapped host memory [h, h + bytes) (2-byte aligned,
 // one contiguous mapping), or null.
 uint8_t *device_view(uint8_t *h, size_t bytes);

@@ -844,7 +844,7 @@ int cmd_server_create(cmd_engine *eng, const cmd_server_config *cfg, cmd_server 
     const size_t rows = row_cap(B), locbs = tile_cap(B) * (size_t)TILE_SCRATCH_WORDS * 4;
     const size_t dev_per_slot = lay.total + rows * ERR_STRIDE * 4 + rows * 2 + locbs + 4 * 256;
     srv->device_bytes = dev_per_slot * cfg->slots;
-    if (!budget_take(eng, srv->device_bytes)) {
+    if (!budget_take_first(eng, srv->device_bytes)) {
         delete srv;
         set_last_error("server buffers exceed the engine HBM budget");
         return CMD_E_BUDGET;

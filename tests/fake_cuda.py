@@ -61,11 +61,13 @@ class Fake:
         self.rt.fake_ops.restype = ctypes.c_char_p
         self.rt.fake_allocated.restype = ctypes.c_size_t
         self.rt.fake_largest_malloc.argtypes = [ctypes.c_size_t]
+        self.rt.fake_total.argtypes = [ctypes.c_size_t]
         self.rt.fake_elapsed.argtypes = [ctypes.c_float]
         self.reset()
 
     def reset(self):
         self.rt.fake_largest_malloc(2 ** 63)
+        self.rt.fake_total(2 ** 63)
         self.rt.fake_elapsed(1.0)
         self.rt.fake_clear()
         self.rt.fake_call(0)

@@ -66,7 +66,7 @@ std::vector<Op> ops;
 std::vector<Stream *> streams;
 Stream default_stream;
 Clock host;  // what host waits have covered
-size_t largest = ~(size_t)0;
+size_t largest = ~(size_t)0, total = ~(size_t)0, allocated = 0;
 int call_id = 0, next_capture = 0;
 float elapsed_ms = 1;
 std::string json;
@@ -119,14 +119,9 @@ extern "C" {
 // ---- test controls -----------------------------------------------------------
 void fake_call(int id) { call_id = id; }                    // tags the operations that follow
 void fake_largest_malloc(size_t bytes) { largest = bytes; }  // larger ones fail
+void fake_total(size_t bytes) { total = bytes; }             // more than that at once fails
 void fake_elapsed(float ms) { elapsed_ms = ms; }
-size_t fake_allocated()
-{
-    size_t n = 0;
-    for (const auto &b : blocks)
-        n += b.second;
-    return n;
-}
+size_t fake_allocated() { return allocated; }
 void fake_clear()
 {
     ops.clear();
@@ -233,11 +228,12 @@ cudaError_t cudaMalloc(void **p, size_t bytes)
     std::lock_guard<std::recursive_mutex> lk(mu);
     if (unsafe())
         return ret(cudaErrorStreamCaptureUnsupported);
-    if (bytes > largest)
+    if (bytes > largest || allocated + bytes > total)
         return ret(cudaErrorMemoryAllocation);
     *p = aligned_alloc(4096, (bytes + 4095) / 4096 * 4096);
     memset(*p, 0, bytes < (1 << 20) ? bytes : (1 << 20));
     blocks[*p] = bytes;
+    allocated += bytes;
     return cudaSuccess;
 }
 cudaError_t cudaFree(void *p)
@@ -248,6 +244,7 @@ cudaError_t cudaFree(void *p)
     if (unsafe())
         return ret(cudaErrorStreamCaptureUnsupported);
     wait_all();
+    allocated -= blocks[p];
     blocks.erase(p);
     free(p);
     return cudaSuccess;

@@ -62,3 +62,62 @@ def test_a_mixed_batchs_scratch_is_bounded(fake):  # noqa: F811
             assert done == list(range((0, 0, 2, 2, 4)[i])), i
         for k in keys:
             k.free()
+
+
+def keys_that_fit(fake, eng):  # noqa: F811
+    cmd, keys = fake.cmd, []
+    try:
+        while True:
+            keys.append(cmd.Key(eng, 8192128, golden_sk(8192128)))
+    except cmd.CmdError as e:
+        assert e.code == cmd.CMD_E_BUDGET
+    n = len(keys)
+    for k in keys:
+        k.free()
+    return n
+
+
+def test_kept_scratch_is_given_back(fake):  # noqa: F811
+    """To what the budget or the device would otherwise refuse: keys, a server, key
+    generation, decapsulation, the buffers of a host batch."""
+    cmd = fake.cmd
+
+    def engine():
+        eng = cmd.Engine(0, hbm_budget=200 << 20)
+        return eng, cmd.Key(eng, 8192128, golden_sk(8192128))
+
+    def warm(eng, key):  # staged scratch of 100 MB and more
+        mixed(fake, eng, [key], np.zeros(75000), 0)
+        assert eng.memory()[0] > 100 << 20
+
+    eng, key = engine()
+    fits = keys_that_fit(fake, eng)
+    warm(eng, key)
+    assert keys_that_fit(fake, eng) >= fits - 2  # the mixed batch's work lists, 2 MB, stay
+    key.free()
+    eng.close()
+    host = np.zeros((65535, 208), np.uint8)
+    for job in (lambda e, k: cmd.Server(e, max_batch=16384, slots=4).close(),
+                lambda e, k: cmd.lib().cmd_stage_synd_fft(e.handle, k.handle, 0x1000, 250000, 0x1000, None),
+                lambda e, k: cmd.decrypt(e, k, host, path="fused"),
+                lambda e, k: cmd.kem_decap(e, k, host)):
+        eng, key = engine()
+        job(eng, key)  # fits
+        key.free()
+        eng.close()
+        eng, key = engine()
+        warm(eng, key)
+        job(eng, key)
+        assert eng.memory()[0] <= 200 << 20
+        key.free()
+        eng.close()
+    # the device's memory rather than the budget
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, 8192128, golden_sk(8192128))
+        warm(eng, key)
+        fake.rt.fake_total(fake.rt.fake_allocated() + (1 << 20))
+        more = cmd.Key(eng, 8192128, golden_sk(8192128))
+        cmd.prepare_decap(eng, more)
+        assert eng.memory()[0] < 100 << 20
+        key.free()
+        more.free()
