@@ -6,8 +6,8 @@
 // growing batch sizes and records the size from which the staged ones win, below
 // which CMD_PATH_AUTO takes the small-batch kernels.  The decrypt kernels'
 // instruction stream does not depend on the ciphertext contents, so the sample is
-// a constant byte pattern.  Choices are cached per engine and persisted as JSON keyed by (GPU name, set) in
-// $CMD_TUNE_CACHE (default ~/.cache/cmd_b200/tune.json).
+// a constant byte pattern.  Choices are cached per engine and persisted as JSON
+// keyed by (GPU name, set) in $CMD_TUNE_CACHE (default ~/.cache/cmd_b200/tune.json).
 //
 // Graphs: a decrypt over fixed device buffers is captured once and replayed,
 // which removes the per-call host work (argument checks, round sizing,
@@ -38,8 +38,9 @@ static std::string cache_path()
 }
 
 // Minimal reader/writer for
-// {"key": {"wpb": n, "balanced": b, "ns_per_ct": x, "tile_below": c}, ...};
-// an entry without tile_below (an older tuner's) is tuned again.
+// {"key": {"wpb": n, "balanced": b, "ns_per_ct": x, "small_below": c}, ...};
+// an entry without small_below (an older tuner's, whose "tile_below" was the
+// crossover against the fused kernel) is tuned again.
 static std::map<std::string, FusedConfig> load_cache()
 {
     std::map<std::string, FusedConfig> out;
@@ -70,9 +71,9 @@ static std::map<std::string, FusedConfig> load_cache()
         const char *w = strstr(body.c_str(), "\"wpb\":");
         const char *b = strstr(body.c_str(), "\"balanced\":");
         const char *t = strstr(body.c_str(), "\"ns_per_ct\":");
-        const char *tb = strstr(body.c_str(), "\"tile_below\":");
+        const char *tb = strstr(body.c_str(), "\"small_below\":");
         unsigned tbv = 0;
-        if (w && tb && sscanf(tb + 13, "%u", &tbv) == 1 && sscanf(w + 6, "%d", &wpb) == 1 && (wpb == 4 || wpb == 8)) {
+        if (w && tb && sscanf(tb + 14, "%u", &tbv) == 1 && sscanf(w + 6, "%d", &wpb) == 1 && (wpb == 4 || wpb == 8)) {
             c.tile_below = tbv;
             c.wpb = wpb;
             if (b)
@@ -103,7 +104,7 @@ static void save_cache(const std::map<std::string, FusedConfig> &m)
     fprintf(f, "{\n");
     size_t i = 0;
     for (const auto &kv : m) {
-        fprintf(f, "  \"%s\": {\"wpb\": %d, \"balanced\": %d, \"ns_per_ct\": %.3f, \"tile_below\": %u}%s\n",
+        fprintf(f, "  \"%s\": {\"wpb\": %d, \"balanced\": %d, \"ns_per_ct\": %.3f, \"small_below\": %u}%s\n",
                 kv.first.c_str(), kv.second.wpb, kv.second.balanced ? 1 : 0, kv.second.ns_per_ct,
                 kv.second.tile_below, ++i < m.size() ? "," : "");
     }

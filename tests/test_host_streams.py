@@ -143,3 +143,21 @@ def test_the_engines_scratch_is_reused_after_its_last_use(fake, first, then):
         assert one and two
         assert all(o.after(one[-1]) for o in two)
         key.free()
+
+
+def test_an_older_tuners_file_is_tuned_again(fake, tmp_path, monkeypatch):
+    """Its crossover was against the fused kernel; today's is against the staged ones."""
+    cmd = fake.cmd
+    path = tmp_path / "tune.json"
+    path.write_text('{\n  "host test|348864": {"wpb": 4, "balanced": 0, "ns_per_ct": 50.0, "tile_below": 8192}\n}\n')
+    monkeypatch.setenv("CMD_TUNE_CACHE", str(path))
+    for tuned in (False, True):
+        with cmd.Engine(0) as eng:
+            key = cmd.Key(eng, 348864, golden_sk(348864))
+            fake.rt.fake_clear()
+            assert cmd.tune(eng, key)["tile_below"] == 0  # equal times: not faster
+            assert bool(fake.ops()) != tuned  # the second engine reads what the first one wrote
+            fake.rt.fake_clear()
+            cmd.decrypt_device(eng, key, 0x1000, 5000, 0x1000)
+            assert any("k_bm_tile" in o.name for o in fake.ops())
+            key.free()
