@@ -314,6 +314,27 @@ cudaError_t launch_decap(int set, const uint8_t *d_cts, const uint32_t *d_err, u
     });
 }
 
+// A device batch; the key is prepared.  Caller holds eng->mu.
+static int run_decap(cmd_engine *eng, cmd_key *key, const uint8_t *d_cts, size_t count, uint8_t *d_keys,
+                     uint8_t *d_accept, cudaStream_t s)
+{
+    const SetInfo si = set_info(key->dev.set);
+    const size_t words = count * si.nw;
+    int rc = eng->scratch.begin(eng, words * 4 + count * 2 + 256, s);
+    if (rc)
+        return rc;
+    uint32_t *d_err = static_cast<uint32_t *>(eng->scratch.ptr);
+    uint16_t *d_w = reinterpret_cast<uint16_t *>(d_err + words);
+    cudaError_t e = cudaSuccess;
+    if ((rc = run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)) == CMD_OK) {
+        const uint8_t *d_s = key->dev.sk + 40 + 2 * si.t + si.cond;
+        e = launch_decap(key->dev.set, d_cts, d_err, d_w, key->pk, d_s, d_keys, d_accept, count, s,
+                         LaunchCounter{&eng->launches});
+    }
+    const int r = eng->scratch.end(s, e);  // the rows are read up to here
+    return rc ? rc : r;
+}
+
 }  // namespace cmd
 
 using namespace cmd;
@@ -360,23 +381,9 @@ int cmd_kem_decap_device(cmd_engine *eng, cmd_key *key, const uint8_t *d_cts, si
     int rc = cmd_key_prepare_decap(eng, key);
     if (rc)
         return rc;
-    const SetInfo si = set_info(key->dev.set);
     cudaSetDevice(eng->device);
     std::lock_guard<std::mutex> lk(eng->mu);
-    cudaStream_t s = stream ? (cudaStream_t)stream : eng->stream;
-    const size_t words = count * si.nw;
-    if ((rc = eng->scratch.begin(eng, words * 4 + count * 2 + 256, s)))
-        return rc;
-    uint32_t *d_err = static_cast<uint32_t *>(eng->scratch.ptr);
-    uint16_t *d_w = reinterpret_cast<uint16_t *>(d_err + words);
-    cudaError_t e = cudaSuccess;
-    if ((rc = run_device(eng, key, CMD_PATH_AUTO, d_cts, count, d_err, d_w, s)) == CMD_OK) {
-        const uint8_t *d_s = key->dev.sk + 40 + 2 * si.t + si.cond;
-        e = launch_decap(key->dev.set, d_cts, d_err, d_w, key->pk, d_s, d_keys, d_accept, count, s,
-                         LaunchCounter{&eng->launches});
-    }
-    const int r = eng->scratch.end(s, e);  // the rows are read up to here
-    return rc ? rc : r;
+    return run_decap(eng, key, d_cts, count, d_keys, d_accept, stream ? (cudaStream_t)stream : eng->stream);
 }
 
 int cmd_kem_decap(cmd_engine *eng, cmd_key *key, const uint8_t *h_cts, size_t count, uint8_t *h_keys,
@@ -392,23 +399,18 @@ int cmd_kem_decap(cmd_engine *eng, cmd_key *key, const uint8_t *h_cts, size_t co
     const SetInfo si = set_info(key->dev.set);
     cudaSetDevice(eng->device);
     const size_t chunk = std::min<size_t>(count, (size_t)1 << 20);
-    uint8_t *d_cts = nullptr, *d_keys = nullptr, *d_acc = nullptr;
-    {
-        std::lock_guard<std::mutex> lk(eng->mu);
-        if ((rc = eng->io.reserve(eng, chunk * (si.ct + 32 + 1) + 1024)))
-            return rc;
-        uint8_t *base = static_cast<uint8_t *>(eng->io.ptr);
-        d_cts = base;
-        d_keys = base + (chunk * si.ct + 255) / 256 * 256;
-        d_acc = d_keys + chunk * 32;
-    }
+    std::lock_guard<std::mutex> lk(eng->mu);  // up to the last copy: calls share the buffers below
+    if ((rc = eng->io.reserve(eng, chunk * (si.ct + 32 + 1) + 1024)))
+        return rc;
+    uint8_t *d_cts = static_cast<uint8_t *>(eng->io.ptr), *d_keys = d_cts + (chunk * si.ct + 255) / 256 * 256,
+            *d_acc = d_keys + chunk * 32;
     cudaStream_t s = eng->stream;
     for (size_t c0 = 0; c0 < count; c0 += chunk) {
         const size_t n = std::min(chunk, count - c0);
         cudaError_t e = cudaMemcpyAsync(d_cts, h_cts + c0 * si.ct, n * si.ct, cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess)
             return cuda_fail(e, "cudaMemcpyAsync(cts H2D)");
-        if ((rc = cmd_kem_decap_device(eng, key, d_cts, n, d_keys, d_acc, s)))
+        if ((rc = run_decap(eng, key, d_cts, n, d_keys, d_acc, s)))
             return rc;
         e = cudaMemcpyAsync(h_keys + c0 * 32, d_keys, n * 32, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && h_accept)

@@ -4,6 +4,7 @@
 // Allocations can be made to fail, and stream capture refuses what CUDA refuses.
 // Linked with the engine's own objects in place of the CUDA runtime library.
 #include <cuda_runtime_api.h>
+#include <unistd.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -67,7 +68,9 @@ std::vector<Stream *> streams;
 Stream default_stream;
 Clock host;  // what host waits have covered
 size_t largest = ~(size_t)0, total = ~(size_t)0, allocated = 0;
-int call_id = 0, next_capture = 0;
+int next_capture = 0;
+unsigned pause_us = 0;
+thread_local int call_id = 0;
 float elapsed_ms = 1;
 std::string json;
 thread_local cudaError_t last = cudaSuccess;
@@ -117,7 +120,8 @@ void wait_all()
 extern "C" {
 
 // ---- test controls -----------------------------------------------------------
-void fake_call(int id) { call_id = id; }                    // tags the operations that follow
+void fake_call(int id) { call_id = id; }                    // tags the operations of this thread that follow
+void fake_pause(unsigned us) { pause_us = us; }              // after every copy, so that other threads come in
 void fake_largest_malloc(size_t bytes) { largest = bytes; }  // larger ones fail
 void fake_total(size_t bytes) { total = bytes; }             // more than that at once fails
 void fake_elapsed(float ms) { elapsed_ms = ms; }
@@ -265,9 +269,13 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *)
 }
 cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind kind, cudaStream_t s)
 {
-    std::lock_guard<std::recursive_mutex> lk(mu);
-    memcpy(dst, src, n);
-    record(s, kind == cudaMemcpyHostToDevice ? "h2d" : kind == cudaMemcpyDeviceToHost ? "d2h" : "copy", dst, n);
+    {
+        std::lock_guard<std::recursive_mutex> lk(mu);
+        memcpy(dst, src, n);
+        record(s, kind == cudaMemcpyHostToDevice ? "h2d" : kind == cudaMemcpyDeviceToHost ? "d2h" : "copy", dst, n);
+    }
+    if (pause_us)
+        usleep(pause_us);
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy2DAsync(void *dst, size_t dp, const void *src, size_t sp, size_t w, size_t h, cudaMemcpyKind,

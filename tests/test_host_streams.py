@@ -3,6 +3,8 @@ streams share buffers of the engine only in order, whatever the streams' timing
 (tests/fake_cudart.cpp records who waits for whom; no kernel runs)."""
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -161,3 +163,30 @@ def test_an_older_tuners_file_is_tuned_again(fake, tmp_path, monkeypatch):
             cmd.decrypt_device(eng, key, 0x1000, 5000, 0x1000)
             assert any("k_bm_tile" in o.name for o in fake.ops())
             key.free()
+
+
+def test_host_decapsulations_of_two_threads_take_turns(fake):
+    """From the copy of the ciphertexts to that of the keys: both use the same
+    device buffers."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, 348864, golden_sk(348864))
+        cts = np.zeros((100, key.info.ct_bytes), np.uint8)
+        cmd.kem_decap(eng, key, cts)
+        fake.rt.fake_clear()
+        fake.rt.fake_pause(300)
+
+        def work(i):
+            for j in range(20):
+                fake.call(1 + 2 * j + i)
+                cmd.kem_decap(eng, key, cts)
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        calls = [o.call for o in fake.ops()]
+        assert len(set(calls)) == 40
+        assert sum(a != b for a, b in zip(calls, calls[1:])) == 39  # each call's operations in one run
+        key.free()
