@@ -86,24 +86,29 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes, int no_memory)
         return CMD_OK;
     size_t want = align_up(std::max(bytes, cap + cap / 2), 1 << 20);
     const bool staged = this == &eng->staged;
-    if (!budget_take(eng, want - cap) && (staged || !give_back(eng) || !budget_take(eng, want - cap))) {
+    const size_t held = captured ? 0 : cap;  // bytes charged that the new block replaces
+    if (!budget_take(eng, want - held) && (staged || !give_back(eng) || !budget_take(eng, want - held))) {
         set_last_error("scratch growth exceeds the engine HBM budget");
         return CMD_E_BUDGET;
     }
-    if (ptr) {
+    if (captured) {
+        eng->outgrown.push_back(ptr);
+        eng->outgrown_bytes += cap;
+        captured = false;
+    } else if (ptr) {
         if (done)
             cudaEventSynchronize(done);
         cudaFree(ptr);
-        ptr = nullptr;
     }
+    ptr = nullptr;
     cudaError_t e = cudaMalloc(&ptr, want);
     if (e == cudaErrorMemoryAllocation && !staged && give_back(eng)) {
         cudaGetLastError();
         e = cudaMalloc(&ptr, want);
     }
     if (e != cudaSuccess) {
-        budget_give(eng, want - cap);
-        budget_give(eng, cap);
+        budget_give(eng, want);
+        ptr = nullptr;
         cap = 0;
         const int rc = cuda_fail(e, "cudaMalloc(scratch)");
         if (e != cudaErrorMemoryAllocation || no_memory == rc)
@@ -127,8 +132,14 @@ bool capturing(cudaStream_t s)
 int Scratch::begin(cmd_engine *eng, size_t bytes, cudaStream_t s, int no_memory)
 {
     const int rc = reserve(eng, bytes, no_memory);
-    if (rc || !done || capturing(s))
+    if (rc)
         return rc;
+    if (capturing(s)) {
+        captured = ptr != nullptr;
+        return CMD_OK;
+    }
+    if (!done)
+        return CMD_OK;
     const cudaError_t e = cudaStreamWaitEvent(s, done);
     return e == cudaSuccess ? CMD_OK : cuda_fail(e, "scratch order");
 }
@@ -156,6 +167,7 @@ void Scratch::release(cmd_engine *eng)
     budget_give(eng, cap);
     ptr = nullptr;
     done = nullptr;
+    captured = false;
     cap = 0;
 }
 
@@ -292,6 +304,9 @@ void cmd_engine_destroy(cmd_engine *eng)
     eng->fused.release(eng);
     eng->staged.release(eng);
     eng->keygen.release(eng);
+    for (void *p : eng->outgrown)
+        cudaFree(p);
+    budget_give(eng, eng->outgrown_bytes);
     eng->host_scratch.release();
     release_fft_plans(eng);
     for (int i = 0; i < BATCH_STREAMS; i++)

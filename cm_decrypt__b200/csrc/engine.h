@@ -20,12 +20,14 @@ struct Scratch {
     void *ptr = nullptr;
     size_t cap = 0;
     cudaEvent_t done = nullptr;  // after the last use between begin and end
+    bool captured = false;       // in a graph: growing leaves this block to the engine
     // no_memory: returned when the budget allows the growth but the device's memory
     // does not (others use it, too); CMD_E_BUDGET from callers that can do without.
     int reserve(cmd_engine *eng, size_t bytes, int no_memory = CMD_E_CUDA);
     // Around work on a caller's stream that uses the buffer: reserves it and orders
     // s after its last use on any stream; marks this use (also after an error e).
-    // A stream under capture neither waits nor marks.
+    // A stream under capture neither waits nor marks; its graph keeps the address, so
+    // the block stays until the engine goes.
     int begin(cmd_engine *eng, size_t bytes, cudaStream_t s, int no_memory = CMD_E_CUDA);
     int end(cudaStream_t s, cudaError_t e = cudaSuccess);
     void release(cmd_engine *eng);
@@ -147,6 +149,8 @@ struct cmd_engine {
                                    // and CMD_PATH_AUTO's small batches'
     cudaEvent_t staged_fork = nullptr, staged_join[cmd::STAGED_STREAMS] = {};  // created on first use
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
+    std::vector<void *> outgrown;  // scratch that graphs may still use
+    size_t outgrown_bytes = 0;
     cmd::HostScratch host_scratch; // pinned staging
     uint32_t *tile_counter = nullptr;  // the fused kernel's work counters
     cudaEvent_t counter_done[cmd::COUNTER_RING] = {};  // created on first use

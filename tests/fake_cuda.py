@@ -83,6 +83,10 @@ class Fake:
         assert self.rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(nbytes)) == 0
         return p.value
 
+    def blocks(self) -> set[int]:
+        a = (ctypes.c_uint64 * 4096)()
+        return set(a[:self.rt.fake_blocks(a, 4096)])
+
     def call(self, i: int):
         self.rt.fake_call(i)
 

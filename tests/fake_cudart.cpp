@@ -126,6 +126,14 @@ void fake_largest_malloc(size_t bytes) { largest = bytes; }  // larger ones fail
 void fake_total(size_t bytes) { total = bytes; }             // more than that at once fails
 void fake_elapsed(float ms) { elapsed_ms = ms; }
 size_t fake_allocated() { return allocated; }
+int fake_blocks(uint64_t *address, int most)  // of device memory
+{
+    int n = 0;
+    for (const auto &b : blocks)
+        if (n < most)
+            address[n++] = (uint64_t)b.first;
+    return n;
+}
 void fake_clear()
 {
     ops.clear();

@@ -190,3 +190,32 @@ def test_host_decapsulations_of_two_threads_take_turns(fake):
         assert len(set(calls)) == 40
         assert sum(a != b for a, b in zip(calls, calls[1:])) == 39  # each call's operations in one run
         key.free()
+
+
+@pytest.mark.parametrize("job", ["plain", "tile", "synd", "decap", "graph"])
+def test_scratch_in_a_graph_outlives_its_growth(fake, job):
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key, s = cmd.Key(eng, 348864, golden_sk(348864)), fake.stream()
+        cmd.prepare_decap(eng, key)
+        cmd.decrypt_device(eng, key, 0x1000, 1 << 20, 0x1000)  # all the scratch a decapsulation's decrypt takes
+        jobs = {"plain": lambda n: cmd.decrypt_device(eng, key, 0x1000, n, 0x1000, 0, s, "plain"),
+                "tile": lambda n: cmd.decrypt_device(eng, key, 0x1000, n, 0x1000, 0, s, "tile"),
+                "synd": lambda n: cmd.lib().cmd_stage_synd_fft(eng.handle, key.handle, 0x1000, n, 0x1000, s),
+                "decap": lambda n: cmd.kem_decap_device(eng, key, 0x1000, n, 0x1000, 0x1000, s)}
+        if job == "graph":
+            cmd.Graph(eng, key, 0x1000, 5000, 0x1000, path="plain")
+        else:
+            jobs[job](5000)
+            fake.begin_capture(s, GLOBAL_CAPTURE)
+            jobs[job](5000)
+            assert fake.end_capture(s) == 0
+        held = fake.blocks()
+        for n in (200000, 300000):
+            jobs["decap"](n)
+            jobs["plain"](n)
+        later = fake.blocks()
+        assert held <= later  # what the graph may use
+        jobs["decap"](1000000)
+        assert held <= fake.blocks() and not later <= fake.blocks()  # and no more than that
+        key.free()
