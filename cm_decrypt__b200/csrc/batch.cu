@@ -42,11 +42,9 @@ int TileCounter::begin(cmd_engine *eng, cudaStream_t s)
     if (capturing(s)) {
         constexpr unsigned BLOCK = 256;
         if (eng->graph_counters_left == 0) {
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // cudaMalloc takes no part in the capture
-            cudaThreadExchangeStreamCaptureMode(&mode);
+            BesideCapture beside;
             void *p = nullptr;
             e = cudaMalloc(&p, BLOCK * 4);
-            cudaThreadExchangeStreamCaptureMode(&mode);
             if (e != cudaSuccess)
                 return cuda_fail(e, "cudaMalloc(counters)");
             eng->graph_counters.push_back(static_cast<uint32_t *>(p));
@@ -421,28 +419,45 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
         krefs[k] = key_ref(keys[k]->dev);
 
     // One device block for the work lists; pageable sources, so each copy has
-    // consumed its host buffer when cudaMemcpyAsync returns.
-    const size_t b_order = count * 4, b_off = count * 8, b_tiles = tiles.size() * sizeof(FusedTile),
-                 b_keys = nkeys * sizeof(FusedKeyRef);
-    auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t need = al(b_order) + 2 * al(b_off) + al(b_tiles) + al(b_keys);
+    // consumed its host buffer when cudaMemcpyAsync returns.  Under capture the
+    // graph's own block, filled now: a copy in the graph would read these vectors at
+    // every replay.
+    const size_t b_order = al256(count * 4), b_off = al256(count * 8), b_tiles = al256(tiles.size() * sizeof(FusedTile)),
+                 b_keys = al256(nkeys * sizeof(FusedKeyRef)), need = b_order + 2 * b_off + b_tiles + b_keys;
     TileCounter counter;
-    int rc;
-    if ((rc = counter.begin(eng, s)) || (rc = eng->fused.begin(eng, need, s)))
+    int rc = counter.begin(eng, s);
+    if (rc)
         return rc;
-    uint8_t *base = static_cast<uint8_t *>(eng->fused.ptr);
-    uint32_t *d_order = reinterpret_cast<uint32_t *>(base);
-    uint64_t *d_ct_off = reinterpret_cast<uint64_t *>(base + al(b_order));
-    uint64_t *d_err_off = reinterpret_cast<uint64_t *>(base + al(b_order) + al(b_off));
-    FusedTile *d_tiles = reinterpret_cast<FusedTile *>(base + al(b_order) + 2 * al(b_off));
-    FusedKeyRef *d_keys = reinterpret_cast<FusedKeyRef *>(base + al(b_order) + 2 * al(b_off) + al(b_tiles));
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(d_order, order.data(), b_order, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_ct_off, h_ct_off, b_off, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_err_off, h_err_off, b_off, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_tiles, tiles.data(), b_tiles, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d_keys, krefs.data(), b_keys, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemsetAsync(counter.ptr, 0, sizeof(uint32_t), s)) != cudaSuccess)
+    const bool graph = capturing(s);
+    void *block = nullptr;
+    cudaError_t e = cudaSuccess;
+    uint32_t *d_order;
+    uint64_t *d_ct_off, *d_err_off;
+    FusedTile *d_tiles;
+    FusedKeyRef *d_keys;
+    {
+        BesideCapture beside;
+        if ((rc = graph ? graph_alloc(eng, need, &block) : eng->fused.begin(eng, need, s)))
+            return counter.end(s, rc);
+        uint8_t *at = static_cast<uint8_t *>(graph ? block : eng->fused.ptr);
+        cudaStream_t up = graph ? eng->stream : s;
+        auto put = [&]<class T>(T *&dst, const void *src, size_t bytes, size_t room) {
+            dst = reinterpret_cast<T *>(at);
+            at += room;
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, up);
+        };
+        put(d_order, order.data(), count * 4, b_order);
+        put(d_ct_off, h_ct_off, count * 8, b_off);
+        put(d_err_off, h_err_off, count * 8, b_off);
+        put(d_tiles, tiles.data(), tiles.size() * sizeof(FusedTile), b_tiles);
+        put(d_keys, krefs.data(), nkeys * sizeof(FusedKeyRef), b_keys);
+        if (graph && e == cudaSuccess)
+            e = cudaStreamSynchronize(up);
+    }
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(counter.ptr, 0, sizeof(uint32_t), s);
+    if (e != cudaSuccess)
         return counter.end(s, eng->fused.end(s, e));
     FusedArgs a;
     memset(&a, 0, sizeof a);

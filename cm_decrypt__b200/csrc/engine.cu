@@ -92,8 +92,8 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes, int no_memory)
         return CMD_E_BUDGET;
     }
     if (captured) {
-        eng->outgrown.push_back(ptr);
-        eng->outgrown_bytes += cap;
+        eng->graph_blocks.push_back(ptr);
+        eng->graph_block_bytes += cap;
         captured = false;
     } else if (ptr) {
         if (done)
@@ -127,6 +127,22 @@ bool capturing(cudaStream_t s)
         return cap != cudaStreamCaptureStatusNone;
     cudaGetLastError();  // the legacy stream beside a capture
     return true;
+}
+
+int graph_alloc(cmd_engine *eng, size_t bytes, void **p)
+{
+    if (!budget_take(eng, bytes)) {
+        set_last_error("graph's work lists exceed the engine HBM budget");
+        return CMD_E_BUDGET;
+    }
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        budget_give(eng, bytes);
+        return cuda_fail(e, "cudaMalloc(graph)");
+    }
+    eng->graph_blocks.push_back(*p);
+    eng->graph_block_bytes += bytes;
+    return CMD_OK;
 }
 
 int Scratch::begin(cmd_engine *eng, size_t bytes, cudaStream_t s, int no_memory)
@@ -304,9 +320,9 @@ void cmd_engine_destroy(cmd_engine *eng)
     eng->fused.release(eng);
     eng->staged.release(eng);
     eng->keygen.release(eng);
-    for (void *p : eng->outgrown)
+    for (void *p : eng->graph_blocks)
         cudaFree(p);
-    budget_give(eng, eng->outgrown_bytes);
+    budget_give(eng, eng->graph_block_bytes);
     eng->host_scratch.release();
     release_fft_plans(eng);
     for (int i = 0; i < BATCH_STREAMS; i++)

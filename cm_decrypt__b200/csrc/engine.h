@@ -104,6 +104,16 @@ constexpr int BATCH_STREAMS = 8;      // pieces of a host-buffer batch in flight
 // piece of theirs, then a ring for launches on callers' streams.
 constexpr int COUNTER_RING = 16, COUNTER_RING0 = 1 + BATCH_STREAMS, TILE_COUNTERS = COUNTER_RING0 + COUNTER_RING;
 bool capturing(cudaStream_t s);
+// While it lives, calls of this thread that take no part in a capture (allocations, work
+// on other streams) may be made beside one.
+struct BesideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// Device memory for a graph, kept until the engine goes: CMD_E_BUDGET, CMD_E_CUDA.  Beside
+// a capture; with eng->mu held.
+int graph_alloc(cmd_engine *eng, size_t bytes, void **p);
 // Around a fused launch on a caller's stream: a work counter that no other launch in
 // flight uses, the next of the ring once its last launch has ended.  Under capture
 // the counter stays the captured launch's own, since a graph may be replayed at
@@ -149,8 +159,8 @@ struct cmd_engine {
                                    // and CMD_PATH_AUTO's small batches'
     cudaEvent_t staged_fork = nullptr, staged_join[cmd::STAGED_STREAMS] = {};  // created on first use
     cmd::Scratch keygen;           // key-generation workspace (kept between calls)
-    std::vector<void *> outgrown;  // scratch that graphs may still use
-    size_t outgrown_bytes = 0;
+    std::vector<void *> graph_blocks;  // outgrown scratch and work lists that graphs may use
+    size_t graph_block_bytes = 0;
     cmd::HostScratch host_scratch; // pinned staging
     uint32_t *tile_counter = nullptr;  // the fused kernel's work counters
     cudaEvent_t counter_done[cmd::COUNTER_RING] = {};  // created on first use

@@ -327,6 +327,8 @@ cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }  // kept: it
 cudaError_t cudaStreamSynchronize(cudaStream_t s)
 {
     std::lock_guard<std::recursive_mutex> lk(mu);
+    if (unsafe())
+        return ret(cudaErrorStreamCaptureUnsupported);
     join(host, get(s)->seen);
     return cudaSuccess;
 }
@@ -359,6 +361,8 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s)
 cudaError_t cudaEventSynchronize(cudaEvent_t e)
 {
     std::lock_guard<std::recursive_mutex> lk(mu);
+    if (unsafe())
+        return ret(cudaErrorStreamCaptureUnsupported);
     join(host, get(e)->at);
     return cudaSuccess;
 }

@@ -337,3 +337,46 @@ def test_mixed_batch_of_many_keys(engine):
     finally:
         for k in keys:
             k.free()
+
+
+def test_captured_batches_outlive_larger_calls():
+    """A mixed batch, a plain-path batch and a decapsulation captured on an engine of
+    their own, replayed after larger calls have replaced its buffers."""
+    sets = [348864, 460896]
+    with cmd.Engine(0) as eng:
+        keys = [cmd.Key(eng, s, golden_sk(s)) for s in sets]
+        try:
+            pool = [batch(s, 40000)[1] for s in sets]
+            info, n = keys[0].info, 600
+            cmd.prepare_decap(eng, keys[0])
+            want = [run(eng, k, c, "plain", 0, n)[0] for k, c in zip(keys, pool)]
+            session, accept = cmd.kem_decap(eng, keys[0], pool[0][:n].cpu().numpy())
+            buf = torch.cat([c[:n].reshape(-1) for c in pool])
+            err = torch.zeros(n * sum(k.info.err_words for k in keys), dtype=torch.int32, device="cuda")
+            plain = torch.zeros((n, info.err_words), dtype=torch.int32, device="cuda")
+            k32, acc = (torch.zeros((n, m), dtype=torch.uint8, device="cuda") for m in (32, 1))
+            torch.cuda.synchronize()
+            graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            with torch.cuda.graph(graph, stream=side):
+                ki = np.repeat(np.arange(2, dtype=np.uint32), n)
+                ct = np.array([k.info.ct_bytes for k in keys], np.uint64)[ki]
+                nw = np.array([k.info.err_words for k in keys], np.uint64)[ki]
+                off, eoff = (np.cumsum(ct) - ct).astype(np.uint64), (np.cumsum(nw) - nw).astype(np.uint64)
+                cmd.decrypt_mixed_device(eng, keys, ki, buf.data_ptr(), off, err.data_ptr(), eoff, 0, side.cuda_stream)
+                cmd.decrypt_device(eng, keys[0], pool[0].data_ptr(), n, plain.data_ptr(), 0, side.cuda_stream, "plain")
+                cmd.kem_decap_device(eng, keys[0], pool[0].data_ptr(), n, k32.data_ptr(), acc.data_ptr(), side.cuda_stream)
+            for x in (ki, ct, nw, off, eoff):
+                x.fill(2 ** 31)
+            big = cmd.kem_decap(eng, keys[0], pool[0].cpu().numpy())
+            assert np.array_equal(big[0][:n], session)
+            run(eng, keys[1], pool[1], "plain")
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(err, torch.cat([w.reshape(-1) for w in want]))
+            assert torch.equal(plain, want[0])
+            assert np.array_equal(k32.cpu().numpy(), session) and np.array_equal(acc.cpu().numpy()[:, 0], accept)
+            del graph
+        finally:
+            for k in keys:
+                k.free()

@@ -219,3 +219,28 @@ def test_scratch_in_a_graph_outlives_its_growth(fake, job):
         jobs["decap"](1000000)
         assert held <= fake.blocks() and not later <= fake.blocks()  # and no more than that
         key.free()
+
+
+def test_a_captured_mixed_batch_keeps_its_work_lists(fake):
+    """On the device: a copy in the graph would read the call's host vectors at every
+    replay, and the engine's own lists are rewritten by the next batch."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        keys, s = [cmd.Key(eng, x, golden_sk(x)) for x in (348864, 6960119)], fake.stream()
+        for warm in (False, True):
+            fake.rt.fake_clear()
+            fake.begin_capture(s, GLOBAL_CAPTURE)
+            mixed(fake, eng, keys, np.arange(1000) % 2, s)
+            assert fake.end_capture(s) == 0
+            ops = fake.ops()
+            kernel = next(o for o in ops if "k_fused" in o.name)
+            lists = [o for o in ops if o.name == "h2d"]
+            assert lists and not [o for o in lists if o.stream == kernel.stream]
+            assert any(o.dst == kernel.arg[0] for o in lists)  # FusedArgs::tiles
+            held = fake.blocks()
+            fake.rt.fake_clear()
+            mixed(fake, eng, keys, np.arange(47000) % 2, s)
+            assert not [o for o in fake.ops() if any(o.writes(x) for x in lists)]
+            assert held <= fake.blocks()
+        for k in keys:
+            k.free()
