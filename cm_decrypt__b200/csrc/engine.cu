@@ -666,7 +666,7 @@ int run_staged(cmd_engine *eng, const cmd_key *key, const uint8_t *d_cts, size_t
         const size_t c0 = p * part, n = std::min(part, count - c0), i = p % ns;
         e = launch_staged(key->dev, d_cts + c0 * si.ct, (uint32_t)n,
                           static_cast<uint32_t *>(eng->staged.ptr) + i * words, d_err ? d_err + c0 * si.nw : nullptr,
-                          d_weight ? d_weight + c0 : nullptr, d_pos ? d_pos + c0 * (si.t + 1) : nullptr, nullptr,
+                          d_weight ? d_weight + c0 : nullptr, d_pos ? d_pos + c0 * (si.t + 1) : nullptr,
                           eng->fft[key->dev.set], eng->num_sms, nparts > 2, ns > 1 ? eng->piece_stream[i] : s,
                           LaunchCounter{&eng->launches});
     }

@@ -164,16 +164,15 @@ __device__ __forceinline__ void fft_convert_t(uint32_t *cv, const uint16_t *__re
     }
 }
 
-// Barrier of the WPC warps that share one ciphertext: the warp's own, or named
-// barrier 1 + g of group g of the block.
+// Barrier of the WPC warps that share one ciphertext: the warp's own, or that of a
+// block of four (named barrier 1).
 template <int WPC> __device__ __forceinline__ void group_sync()
 {
+    static_assert(WPC == 1 || WPC == 4, "a warp, or the block's only group");
     if constexpr (WPC == 1)
         __syncwarp();
-    else if constexpr (WPC == 4)  // the block's only group
-        asm volatile("bar.sync 1, 128;" ::: "memory");
     else
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / (32 * WPC)), "n"(32 * WPC) : "memory");
+        asm volatile("bar.sync 1, 128;" ::: "memory");
 }
 
 // Layer l of the key's support network over a 2^m-bit array held by WPC warps

@@ -120,12 +120,12 @@ cudaError_t launch_fused(const FusedArgs &a, int grid, int warps_per_block, cuda
                          LaunchCounter lc);
 
 // One key's batch in four kernels (staged.cu): error rows at the set's nw stride,
-// weights, positions rows (FusedArgs::pos), packed rows (FusedArgs::err_packed),
-// each or null.  d_scratch: staged_scratch_words(set, count) words.  many_parts:
-// one of more than two parts of a batch, on several streams.
+// weights, positions rows (FusedArgs::pos), each or null.  d_scratch:
+// staged_scratch_words(set, count) words.  many_parts: one of more than two parts of
+// a batch, on several streams.
 cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count, uint32_t *d_scratch, uint32_t *d_err,
-                          uint16_t *d_weight, uint16_t *d_pos, uint8_t *err_packed, const FftPlanDev &plan,
-                          int num_sms, bool many_parts, cudaStream_t s, LaunchCounter lc);
+                          uint16_t *d_weight, uint16_t *d_pos, const FftPlanDev &plan, int num_sms, bool many_parts,
+                          cudaStream_t s, LaunchCounter lc);
 size_t staged_scratch_words(int set, size_t count);
 // The same for the ciphertexts of one set in a mixed batch: `blocks` and `tiles`
 // cut the slots of `order` (a key's slots contiguous) into syndrome blocks of up

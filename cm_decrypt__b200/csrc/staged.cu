@@ -332,7 +332,6 @@ struct NetArgs {
     uint32_t *err;        // rows of nw words, or null
     uint16_t *weight;     // or null
     uint16_t *pos;        // rows of t + 1, or null
-    uint8_t *err_packed;  // rows of n/8 bytes, or null
     StagedMixed mx;       // MIX: count is 32 * tiles, err / weight by ciphertext
 };
 
@@ -341,7 +340,7 @@ struct NetArgs {
 template <int S, int NC, bool MIX = false> __global__ void __launch_bounds__(NET_WARPS * 32) k_net_rows(NetArgs a)
 {
     using F = FftDims<S>;
-    constexpr int M = F::M, NWD = F::NWD, R = F::R;
+    constexpr int NWD = F::NWD, R = F::R;
     __shared__ uint32_t rows[NET_WARPS][NC * NWD];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t c0 = ((uint64_t)blockIdx.x * NET_WARPS + warp) * NC;
@@ -378,12 +377,10 @@ template <int S, int NC, bool MIX = false> __global__ void __launch_bounds__(NET
             v[j] = rows[warp][i * NWD + lane + 32 * j];  // this lane's own words
         const uint64_t c = MIX ? order[i] : c0 + i;
         const int cnt = root_output<S>(v, a.err ? a.err + (MIX ? a.mx.err_off[c] : c * F::NW) : nullptr,
-                                       a.pos ? a.pos + c * (F::T + 1) : nullptr,
-                                       a.err_packed ? a.err_packed + c * (F::N / 8) : nullptr, lane);
+                                       a.pos ? a.pos + c * (F::T + 1) : nullptr, nullptr, lane);
         if (lane == 0 && a.weight)
             a.weight[c] = (uint16_t)cnt;
     }
-    (void)M;
 }
 
 // Raises kernel `f`'s shared-memory limit once per device.
@@ -410,8 +407,8 @@ size_t staged_scratch_words(int set, size_t count)
 }
 
 cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count, uint32_t *d_scratch, uint32_t *d_err,
-                          uint16_t *d_weight, uint16_t *d_pos, uint8_t *err_packed, const FftPlanDev &plan,
-                          int num_sms, bool many_parts, cudaStream_t s, LaunchCounter lc)
+                          uint16_t *d_weight, uint16_t *d_pos, const FftPlanDev &plan, int num_sms,
+                          bool many_parts, cudaStream_t s, LaunchCounter lc)
 {
     if (count == 0)
         return cudaSuccess;
@@ -472,7 +469,7 @@ cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count,
         while (parts < 32 / FFT_WARPS && ntiles * parts < 3 * sms)
             parts *= 2;
         k_fft_tile<S><<<dim3(ntiles, parts), FFT_WARPS * 32, fft_smem, s>>>(tiles, count, plan.tw, flags, nullptr);
-        const NetArgs na{flags, k.bctl, count, d_err, d_weight, d_pos, err_packed, {}};
+        const NetArgs na{flags, k.bctl, count, d_err, d_weight, d_pos, {}};
         const uint32_t nc = count <= 64 * sms ? 1 : 4, per = NET_WARPS * nc;
         if (nc == 1)
             k_net_rows<S, 1><<<(count + per - 1) / per, NET_WARPS * 32, 0, s>>>(na);
@@ -513,7 +510,7 @@ cudaError_t launch_staged_mixed(int set, const StagedMixed &mx, uint32_t nblocks
         while (parts < 32 / FFT_WARPS && ntiles * parts < 3 * sms)
             parts *= 2;
         k_fft_tile<S><<<dim3(ntiles, parts), FFT_WARPS * 32, fft_smem, s>>>(tiles, 0, plan.tw, flags, mx.tiles);
-        const NetArgs na{flags, nullptr, 32 * ntiles, d_err, d_weight, nullptr, nullptr, mx};
+        const NetArgs na{flags, nullptr, 32 * ntiles, d_err, d_weight, nullptr, mx};
         k_net_rows<S, 4, true><<<(ntiles + NET_WARPS / 8 - 1) / (NET_WARPS / 8), NET_WARPS * 32, 0, s>>>(na);
         lc.bump(4);
         return cudaGetLastError();
