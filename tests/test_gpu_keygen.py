@@ -84,3 +84,19 @@ def test_keypair_batch_repeatable_and_matches_oracle(oracle_mod, engine):
     for i in range(seeds.shape[0]):
         pk_o, sk_o, a_o = o.keypair(seeds[i].tobytes())
         assert (int(att[i]), sks[i].tobytes(), pks[i].tobytes()) == (a_o, sk_o, pk_o), i
+
+
+@pytest.mark.parametrize("s,count", [(348864, 74), (348864, 75), (348864, 300), (6960119, 75)])
+def test_keypair_batches_by_number_of_chains(oracle_mod, engine, s, count):
+    """Two sets of seed chains up to 74 keys (a quarter of the 296 slots), one set
+    above, in several chunks above 296: the key pairs of batches of 25."""
+    seeds = np.frombuffer(rng(77 + count).bytes(32 * count), np.uint8).reshape(count, 32)
+    whole = cmd.kem_keypair_batch(engine, s, seeds)
+    for i in range(0, count, 25):
+        for a, b in zip(whole, cmd.kem_keypair_batch(engine, s, seeds[i:i + 25])):
+            assert np.array_equal(a[i:i + 25], b), i
+    o = oracle_mod.Oracle(s)
+    for i in (0, count - 1):
+        assert (int(whole[2][i]), whole[1][i].tobytes(), whole[0][i].tobytes()) == \
+            tuple(o.keypair(seeds[i].tobytes())[j] for j in (2, 1, 0)), i
+    assert len(set(whole[2].tolist())) > 1

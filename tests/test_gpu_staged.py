@@ -380,3 +380,18 @@ def test_captured_batches_outlive_larger_calls():
         finally:
             for k in keys:
                 k.free()
+
+
+def test_staged_edges_of_the_largest_t(engine):
+    """6688128 (t = 128 at n < 2^13) at the sizes where the launches change shape."""
+    s = 6688128
+    info, cts = batch(s, max(EDGES))
+    key = cmd.Key(engine, s, golden_sk(s))
+    try:
+        want, want_w = run(engine, key, cts, "fused")
+        for count in EDGES:
+            err, w = run(engine, key, cts, "auto", 0, count)
+            torch.cuda.synchronize()
+            assert torch.equal(err, want[:count]) and torch.equal(w, want_w[:count]), count
+    finally:
+        key.free()
