@@ -97,6 +97,6 @@ def test_keypair_batches_by_number_of_chains(oracle_mod, engine, s, count):
             assert np.array_equal(a[i:i + 25], b), i
     o = oracle_mod.Oracle(s)
     for i in (0, count - 1):
-        assert (int(whole[2][i]), whole[1][i].tobytes(), whole[0][i].tobytes()) == \
-            tuple(o.keypair(seeds[i].tobytes())[j] for j in (2, 1, 0)), i
+        pk_o, sk_o, a_o = o.keypair(seeds[i].tobytes())
+        assert (int(whole[2][i]), whole[1][i].tobytes(), whole[0][i].tobytes()) == (a_o, sk_o, pk_o), i
     assert len(set(whole[2].tolist())) > 1
