@@ -616,7 +616,7 @@ cudaError_t launch_tile_single(const KeyDev &k, const uint8_t *d_cts, size_t cou
                    ? launch_ct_items(items, d_cts, ntiles * 32, (uint32_t)count, reinterpret_cast<uint16_t *>(tiles),
                                      d_err, d_weight, d_pos, plans, num_sms, s, lc)
                    : cudaErrorInvalidValue;
-    return launch_tile_path(items, d_cts, ntiles, (uint32_t)count, tiles, d_err, d_weight, plans, num_sms, s, lc);
+    return launch_tile_path(items, d_cts, ntiles, (uint32_t)count, 0, tiles, d_err, d_weight, plans, num_sms, s, lc);
 }
 
 size_t tile_single_scratch_words(size_t count)
@@ -653,12 +653,12 @@ cudaError_t tile_prepare(int dev, size_t smem, size_t ts_smem, size_t root_smem)
 
 // ntiles tiles of 32 item slots; weights are indexed by item slot.
 cudaError_t launch_tile_path(const void *d_items, const uint8_t *d_cts, uint32_t ntiles, uint32_t live,
-                             uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight, const FftPlans &plans,
-                             int num_sms, cudaStream_t s, LaunchCounter lc)
+                             uint32_t beside, uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight,
+                             const FftPlans &plans, int num_sms, cudaStream_t s, LaunchCounter lc)
 {
     if (ntiles == 0)
         return cudaSuccess;
-    if (live <= CT_PER_SM * (uint32_t)num_sms)
+    if (live <= CT_PER_SM * (uint32_t)num_sms && live + beside <= CT_IN_FLIGHT_PER_SM * (uint32_t)num_sms)
         return launch_ct_items(static_cast<const LatItem *>(d_items), d_cts, ntiles * 32, live,
                                reinterpret_cast<uint16_t *>(d_scratch), d_err, d_weight, nullptr, plans, num_sms, s, lc);
     int dev = 0;

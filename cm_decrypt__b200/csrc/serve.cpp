@@ -15,17 +15,18 @@
 //    when the engine's HBM budget is full (admission by budget).  Every batch
 //    stamps the keys it made resident with its generation; a key is in use
 //    while a batch of that generation or later is in flight.
-//  * Small batches run the latency kernels of latency.cu (any mix of keys and
-//    sets in three launches, a short pass per ciphertext); batches of
-//    fused_threshold or more run the fused kernel (highest throughput).
+//  * Batches of up to CT_PER_SM requests an SM run the per-ciphertext kernels of
+//    single.cu (up to CT_ONE_LAUNCH in one launch, else three) while no more than
+//    CT_IN_FLIGHT_PER_SM are in flight, others the tile kernels of latency.cu (three
+//    launches), either for any mix of keys and sets; batches of fused_threshold or more run the fused kernel.
 //  * A completer thread watches the batches in flight without the queue lock
 //    (each batch's stream copies its sequence number to a pinned word after
 //    the results, so the watch is plain loads, not CUDA calls), takes
 //    whichever finishes first, copies each result to its request's
 //    buffer (large batches split across a few copy threads) and records
 //    arrival-to-completion latency for the p50/p99 statistics.  A buffer in
-//    memory registered with cmd_server_register_rows needs no copy: the tile
-//    path's root kernel stores the row there itself.
+//    memory registered with cmd_server_register_rows needs no copy: the root
+//    kernel of either kind stores the row there itself.
 //  * Host work per request is O(1): the queue is a vector whose buffers
 //    circulate between the queue and the slots (no allocation per request),
 //    keys are marked once per batch by generation stamp, and the tile path
@@ -296,6 +297,7 @@ struct cmd_server {
     std::vector<Slot> slots;
     std::deque<int> free_slots;
     std::atomic<uint32_t> inflight{0};  // bit s: slot s has a batch on the GPU (set under mu)
+    std::atomic<uint32_t> inflight_cts{0};  // their ciphertexts
     // done_seq[s]: pinned host word that slot s's stream overwrites with the
     // batch's sequence number after its result copies (a stream-ordered
     // 8-byte copy), so the completer sees a finished batch with plain loads
@@ -521,8 +523,8 @@ int cmd_server::launch(Slot &sl)
         FftPlans plans;
         for (int st = 0; st < NSETS; st++)
             plans.p[st] = eng->fft[st];
-        e = launch_tile_path(sl.d_in + lay.items, sl.d_in + lay.cts, ntiles, (uint32_t)B, sl.d_locbs, sl.d_err, sl.d_w,
-                             plans, eng->num_sms, s, lc);
+        e = launch_tile_path(sl.d_in + lay.items, sl.d_in + lay.cts, ntiles, (uint32_t)B, inflight_cts.load(),
+                             sl.d_locbs, sl.d_err, sl.d_w, plans, eng->num_sms, s, lc);
         if (e != cudaSuccess)
             return cuda_fail(e, "server tile-path launch");
     } else {
@@ -659,6 +661,7 @@ void cmd_server::dispatch_loop()
         batches++;
         fused_batches += sl.fused ? 1 : 0;
         batched_cts += sl.reqs.size();
+        inflight_cts.fetch_add((uint32_t)sl.reqs.size());  // before the completer can take the batch
         inflight.fetch_or(1u << si);
         inflight_sum += __builtin_popcount(inflight.load());
         cv_complete.notify_one();
@@ -769,6 +772,7 @@ void cmd_server::complete_loop()
         t_last = t;
         complete_ns += t_done - t;
         sl.reqs.clear();
+        inflight_cts.fetch_sub((uint32_t)B);
         inflight.fetch_and(~(1u << si));
         free_slots.push_back(si);
         completions_gen++;

@@ -70,6 +70,7 @@ class Fake:
         self.rt.fake_total(2 ** 63)
         self.rt.fake_elapsed(1.0)
         self.rt.fake_pause(0)
+        self.rt.fake_hold(0)
         self.rt.fake_clear()
         self.rt.fake_call(0)
 

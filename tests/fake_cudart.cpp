@@ -70,6 +70,8 @@ Clock host;  // what host waits have covered
 size_t largest = ~(size_t)0, total = ~(size_t)0, allocated = 0;
 int next_capture = 0;
 unsigned pause_us = 0;
+bool hold = false;
+std::vector<std::pair<void *, uint64_t>> held;
 thread_local int call_id = 0;
 float elapsed_ms = 1;
 std::string json;
@@ -122,6 +124,16 @@ extern "C" {
 // ---- test controls -----------------------------------------------------------
 void fake_call(int id) { call_id = id; }                    // tags the operations of this thread that follow
 void fake_pause(unsigned us) { pause_us = us; }              // after every copy, so that other threads come in
+void fake_hold(int on)  // keeps 8-byte results from the host, as of work that has not ended, until let go
+{
+    std::lock_guard<std::recursive_mutex> lk(mu);
+    hold = on != 0;
+    for (const auto &[dst, word] : held)
+        if (!hold)
+            memcpy(dst, &word, 8);
+    if (!hold)
+        held.clear();
+}
 void fake_largest_malloc(size_t bytes) { largest = bytes; }  // larger ones fail
 void fake_total(size_t bytes) { total = bytes; }             // more than that at once fails
 void fake_elapsed(float ms) { elapsed_ms = ms; }
@@ -279,7 +291,12 @@ cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind
 {
     {
         std::lock_guard<std::recursive_mutex> lk(mu);
-        memcpy(dst, src, n);
+        if (hold && kind == cudaMemcpyDeviceToHost && n == 8) {
+            held.push_back({dst, 0});
+            memcpy(&held.back().second, src, 8);
+        } else {
+            memcpy(dst, src, n);
+        }
         record(s, kind == cudaMemcpyHostToDevice ? "h2d" : kind == cudaMemcpyDeviceToHost ? "d2h" : "copy", dst, n);
     }
     if (pause_us)

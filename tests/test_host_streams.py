@@ -4,6 +4,7 @@ streams share buffers of the engine only in order, whatever the streams' timing
 from __future__ import annotations
 
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -244,3 +245,35 @@ def test_a_captured_mixed_batch_keeps_its_work_lists(fake):
             assert held <= fake.blocks()
         for k in keys:
             k.free()
+
+
+def test_server_batches_take_their_kernels_by_what_is_in_flight(fake):
+    """The per-ciphertext kernels do more work for a ciphertext than the tile kernels:
+    they are for a GPU with few ciphertexts on it, not for one batch of many."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng, cmd.Server(eng, max_batch=2000, slots=16, max_wait_us=0) as srv:
+        kid = srv.add_key(348864, golden_sk(348864))
+        cts, rows = np.zeros((2000, 208), np.uint8), np.zeros((2000, 1024), np.uint8)
+
+        def batch():
+            fake.rt.fake_clear()
+            before = srv.stats()["batches"]
+            srv.submit_many(np.full(2000, kid, np.uint32), cts, rows)
+            until = time.monotonic() + 20
+            while srv.stats()["batches"] == before and time.monotonic() < until:
+                time.sleep(0.001)
+            names = [o.name for o in fake.ops() if "k_" in o.name]
+            assert any("k_ct" in n for n in names) != any("k_tile_bm" in n for n in names)
+            return any("k_ct" in n for n in names)
+
+        assert batch()  # (expands the key)
+        srv.drain()
+        fake.rt.fake_hold(1)
+        try:
+            kinds = [batch() for _ in range(10)]
+        finally:
+            fake.rt.fake_hold(0)
+        assert kinds[0] and not kinds[-1] and kinds == sorted(kinds, reverse=True)
+        srv.drain()
+        assert batch()
+        srv.drain()
