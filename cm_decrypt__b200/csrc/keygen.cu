@@ -1170,10 +1170,14 @@ int cmd_kem_keypair_batch(cmd_engine *eng, cmd_set set, const uint8_t *h_seeds, 
     const size_t fixed = 2048 + chain_bytes;
     // per slot: workspace, seed, collect record, list entry, one pk and sk
     auto need = [&](size_t c) { return fixed + c * (d.stride + 32 + 36 + 4 + pk_bytes + d.sk); };
-    // Few keys (every round takes all SPEC attempts of each): two sets of chains,
-    // so that the expansions, the longest serial part, never wait for a round: a
-    // chain takes 2.5 ms and its polynomials 0.9 ms, a round of 32 slots 2.2 ms.
-    const bool ahead = count * SPEC <= cap && eng->keygen.reserve(eng, need(cap) + 512 + chain_bytes) == CMD_OK;
+    // Few keys: two sets of chains, so that the expansions, the longest serial part,
+    // never wait for a round: a chain takes 2.5 ms and its polynomials 0.9 ms, a round
+    // of 32 slots 2.2 ms.  Up to three fifths of the slots (44 keys on a B200): with
+    // more, the rounds fill the GPU and what is expanded ahead in vain takes from them.
+    // One set against two, mean of the same 14 to 24 calls: mceliece6960119 8 keys 11.1
+    // and 10.6 ms, 24 15.1 and 14.2, 44 20.4 and 19.9, 50 22.0 and 22.7, 74 28.2 and 30.0;
+    // 348864 16 5.6 and 5.1, 44 8.8 and 8.0, 56 8.5 and 8.9, 74 9.1 and 9.8.
+    const bool ahead = count * SPEC * 5 <= cap * 3 && eng->keygen.reserve(eng, need(cap) + 512 + chain_bytes) == CMD_OK;
     while (!ahead && cap > 1 && eng->keygen.reserve(eng, need(cap)) != CMD_OK)
         cap /= 2;
     if (!ahead && cap == 1 && eng->keygen.reserve(eng, need(1)) != CMD_OK)

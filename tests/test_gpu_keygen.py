@@ -86,9 +86,9 @@ def test_keypair_batch_repeatable_and_matches_oracle(oracle_mod, engine):
         assert (int(att[i]), sks[i].tobytes(), pks[i].tobytes()) == (a_o, sk_o, pk_o), i
 
 
-@pytest.mark.parametrize("s,count", [(348864, 74), (348864, 75), (348864, 300), (6960119, 75)])
+@pytest.mark.parametrize("s,count", [(348864, 44), (348864, 45), (348864, 300), (6960119, 45)])
 def test_keypair_batches_by_number_of_chains(oracle_mod, engine, s, count):
-    """Two sets of seed chains up to 74 keys (a quarter of the 296 slots), one set
+    """Two sets of seed chains up to 44 keys (three fifths of the 296 slots), one set
     above, in several chunks above 296: the key pairs of batches of 25."""
     seeds = np.frombuffer(rng(77 + count).bytes(32 * count), np.uint8).reshape(count, 32)
     whole = cmd.kem_keypair_batch(engine, s, seeds)

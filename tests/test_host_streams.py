@@ -277,3 +277,14 @@ def test_server_batches_take_their_kernels_by_what_is_in_flight(fake):
         srv.drain()
         assert batch()
         srv.drain()
+
+
+@pytest.mark.parametrize("count,sets", [(1, 2), (44, 2), (45, 1), (74, 1), (300, 1)])
+def test_seed_chains_of_a_key_generation(fake, count, sets):
+    """A second set of chains ahead of the rounds, while their slots leave the GPU room."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        cmd.kem_keypair_batch(eng, 348864, np.zeros((count, 32), np.uint8))
+        names = [o.name for o in fake.ops()]
+        first = next(i for i, n in enumerate(names) if "k_kg_fill" in n)
+        assert sum("k_kg_expand" in n for n in names[:first]) == sets
