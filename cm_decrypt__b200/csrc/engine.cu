@@ -84,6 +84,7 @@ int Scratch::reserve(cmd_engine *eng, size_t bytes, int no_memory)
 {
     if (bytes <= cap)
         return CMD_OK;
+    BesideCapture beside;
     size_t want = align_up(std::max(bytes, cap + cap / 2), 1 << 20);
     const bool staged = this == &eng->staged;
     const size_t held = captured ? 0 : cap;  // bytes charged that the new block replaces

@@ -395,3 +395,27 @@ def test_staged_edges_of_the_largest_t(engine):
             assert torch.equal(err, want[:count]) and torch.equal(w, want_w[:count]), count
     finally:
         key.free()
+
+
+def test_growth_beside_another_streams_capture():
+    """A larger batch on one stream, for which the scratch grows, while another
+    stream is captured in the default mode."""
+    s = 348864
+    info, cts = batch(s, 100000)
+    with cmd.Engine(0) as eng:
+        key = cmd.Key(eng, s, golden_sk(s))
+        try:
+            want, _ = run(eng, key, cts, "fused")
+            run(eng, key, cts, "auto", 0, 4000)
+            err, small = torch.zeros_like(want), torch.zeros((5000, info.err_words), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            graph, side, other = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.cuda.Stream()
+            with torch.cuda.graph(graph, stream=side):
+                cmd.decrypt_device(eng, key, cts.data_ptr(), 5000, small.data_ptr(), 0, side.cuda_stream)
+                cmd.decrypt_device(eng, key, cts.data_ptr(), 100000, err.data_ptr(), 0, other.cuda_stream)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(err, want) and torch.equal(small, want[:5000])
+            del graph
+        finally:
+            key.free()

@@ -288,3 +288,18 @@ def test_seed_chains_of_a_key_generation(fake, count, sets):
         names = [o.name for o in fake.ops()]
         first = next(i for i, n in enumerate(names) if "k_kg_fill" in n)
         assert sum("k_kg_expand" in n for n in names[:first]) == sets
+
+
+def test_scratch_grows_beside_another_streams_capture(fake):
+    """In the default mode an allocation by any thread would end that capture."""
+    cmd = fake.cmd
+    with cmd.Engine(0) as eng:
+        key, a, b = cmd.Key(eng, 348864, golden_sk(348864)), fake.stream(), fake.stream()
+        cmd.decrypt_device(eng, key, 0x1000, 30000, 0x1000, 0, b)
+        fake.begin_capture(a, GLOBAL_CAPTURE)
+        for n in (3000, 5000, 100000):
+            cmd.decrypt_device(eng, key, 0x1000, n, 0x1000, 0, b)
+            cmd.decrypt_positions_device(eng, key, 0x1000, n, 0x1000, b)
+            mixed(fake, eng, [key], np.zeros(n), b)
+        assert fake.end_capture(a) == 0
+        key.free()
