@@ -395,7 +395,10 @@ extern "C" int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *k
     // does not fit and under stream capture.  64 keys on a B200, fused -> taken:
     // 300 ciphertexts 985 -> 145 us, 1,000 1,271 -> 231 us, 10,000 1,797 -> 1,272 us,
     // 20,000 1,843 -> 1,653 us, 100,000 4,088 -> 3,829 us; 40,000 1,910 us (staged
-    // 2,023 us).
+    // 2,023 us).  The staged kernels' cost is by tile and syndrome block, the fused
+    // kernel's by round, a key has at least one of each, and a round costs more: 5,000
+    // ciphertexts of 3,000 keys 11,557 -> 4,538 us, of as many keys 23,485 -> 8,491 us,
+    // 28,000 of 1,000 keys 7,471 -> 2,996 us, 100,000 of 6,000 37,635 -> 11,691 us.
     std::lock_guard<std::mutex> lk(eng->mu);
     const size_t sms = (size_t)eng->num_sms;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

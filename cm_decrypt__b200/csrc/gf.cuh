@@ -18,7 +18,10 @@ namespace cmd {
 
 // Folds a carry-less product of two field elements back below x^M.  Each
 // fold replaces x^M by the low terms of the modulus; two folds suffice for
-// products of degree <= 2M-2.
+// products of degree <= 2M-2.  For M = 13 the four low terms as a product of two
+// sums: one operation less and one longer in the chain than four shifts, 2 to 5 %
+// faster on the plain path from 33 ciphertexts on (6960119 4,096: 2,603 -> 2,539 us),
+// 2 % slower for a single one, whose warps run alone (390 -> 398 us).
 template <int M> __device__ __forceinline__ uint32_t gf_reduce(uint32_t p)
 {
     if constexpr (M == 13) {

@@ -173,10 +173,11 @@ struct FftPlans {
 // flight stays within CT_IN_FLIGHT_PER_SM an SM: they finish sooner on a GPU with room,
 // but do more work for a ciphertext than the tile kernels.  Without that bound the
 // server, 1,024 keys, kept a queue once it had one: at 8 M requests/s p50 1.4 instead
-// of 0.42 ms in some runs, at 9 M 2.2 ms in all.  At 36 an SM p50 / p99 0.42 / 0.55 at 8 M (0.77 / 1.0), 0.46 / 0.60 at 8.5 M (0.79 / 1.03),
-// 0.76 / 1.01 at 9 M (0.83 / 1.07), 0.80 / 1.05 at 9.5 M (0.88 / 1.11), 0.84 / 1.09 at
-// 10 M (0.95 / 1.17), in brackets the tile kernels alone; 24 lets 7 M go to them (0.69
-// against 0.37), 44 raises p99 at 9 M to 1.17 ms.
+// of 0.42 ms in some runs, at 9 M 2.2 ms in all.  At 36 an SM p50 / p99 0.42 / 0.55 at
+// 8 M (0.77 / 1.0), 0.46 / 0.60 at 8.5 M (0.79 / 1.03), 0.76 / 1.01 at 9 M (0.83 /
+// 1.07), 0.80 / 1.05 at 9.5 M (0.88 / 1.11), 0.84 / 1.09 at 10 M (0.95 / 1.17), in
+// brackets the tile kernels alone; 24 lets 7 M go to them (0.69 against 0.37), 44
+// raises p99 at 9 M to 1.17 ms.
 cudaError_t launch_tile_path(const void *d_items, const uint8_t *d_cts, uint32_t ntiles, uint32_t live,
                              uint32_t beside, uint32_t *d_scratch, uint32_t *d_err, uint16_t *d_weight,
                              const FftPlans &plans, int num_sms, cudaStream_t s, LaunchCounter lc);

@@ -438,11 +438,13 @@ cudaError_t launch_staged(const KeyDev &k, const uint8_t *d_cts, uint32_t count,
             k_synd_table<S, 4><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles, {});
         else
             k_synd_table<S, 1><<<blocks, threads, synd_smem, s>>>(k.tabd, d_cts, count, tiles, {});
-        // Warps a tile, by tiles an SM: enough that every scheduler has a warp (one
-        // tile: four warps 255 us, one 467 us for t = 119), and two to even out the
-        // schedulers when they would hold one or two (25,000 ciphertexts in all:
-        // 1,344 against 1,414 us); otherwise one, which passes no barriers (18,944:
-        // 878 against 953 us, 37,888: 1,534 against 1,693 us).
+        // Warps a tile, by tiles an SM: enough that every scheduler has a warp, and two
+        // to even out the schedulers when they would hold one or two; otherwise one,
+        // which passes no barriers.  Whole call, t = 119, one / two / four warps: one
+        // tile an SM 659 / 524 / 443 us, two 736 / 601 / 681, 2.5 769 / 852 / 886,
+        // three 802 / 882 / 917, four 882 / 960 / 1,165, five 1,359 / 1,293 / 1,475; the
+        // other sets alike (t = 64 at five 505 / 497 / 669).  37,888 ciphertexts, eight
+        // an SM: 1,534 with one, 1,693 with two.
         const int bw = ntiles <= sms ? 4 : ntiles <= 2 * sms ? 2 : ntiles <= 4 * sms ? 1 : ntiles <= 6 * sms ? 2 : 1;
         const size_t bm_smem = 4 * (size_t)(Z::BM_WORDS + 2 * bw * 16);
         // Two tiles a warp where the SM holds at least two such warps a scheduler

@@ -245,7 +245,9 @@ int cmd_tune(cmd_engine *eng, const cmd_key *key, size_t sample_count, int force
     }
     eng->fcfg[set] = best;
     // The staged kernels, which CMD_PATH_AUTO runs otherwise, against the
-    // small-batch kernels at growing batch sizes.
+    // small-batch kernels at growing batch sizes.  (The first two sizes only place
+    // the recorded crossover: AUTO takes the small-batch kernels up to CT_PER_SM
+    // ciphertexts an SM, 3,552 on a B200, at any value.)
     best.tile_below = 0;
     const size_t sizes[] = {256, 1024, 4096, 16384, 65536};
     for (size_t n : sizes) {

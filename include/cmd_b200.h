@@ -107,10 +107,15 @@ int cmd_key_synd_table(const cmd_key *key, uint16_t *h_tab, size_t entries);
  * for Berlekamp-Massey, a warp per ciphertext for the root search);
  * CMD_PATH_AUTO takes the latency kernels for small batches (up to 24 an SM,
  * or below the tuned size), the staged kernels (one per phase, with scratch of
- * about 1.4 KB a ciphertext charged to the engine's budget and kept by the
- * engine) for larger ones, and the fused kernel for about one round of its
- * warps (192 to 256 ciphertexts an SM), when the scratch does not fit and
- * under stream capture.  Graph capture takes AUTO, PLAIN and FUSED. */
+ * about 1.4 KB a ciphertext in flight, charged to the engine's budget, and kept
+ * until keys, a server or other buffers need the room) for larger ones, and the
+ * fused kernel for about one round of its warps (192 to 256 ciphertexts an SM),
+ * when the budget or the device's free memory refuses the scratch and under
+ * stream capture.  Graph capture takes AUTO, PLAIN and FUSED.
+ *
+ * Calls may be in flight on several streams and from several threads: those that
+ * share a buffer of the engine are ordered by events, and run one after the other
+ * on the device. */
 typedef enum { CMD_PATH_AUTO = 0, CMD_PATH_PLAIN = 1, CMD_PATH_FUSED = 2, CMD_PATH_TILE = 3 } cmd_path;
 
 /* Replaces the per-ciphertext loop memcpy -> synd -> bm -> root ->
@@ -137,7 +142,8 @@ int cmd_decrypt_device(cmd_engine *eng, const cmd_key *key, cmd_path path,
 /* Mixed batch in one call: ciphertext c belongs to keys[h_key_idx[c]]; its
  * bytes start at d_cts + h_ct_off[c] and its error row at
  * d_err + h_err_off[c] (in 32-bit words).  Keys may be of different sets.
- * Asynchronous on `stream`. */
+ * Asynchronous on `stream`.  Under stream capture the work lists are uploaded
+ * during the call, and stay on the device as long as the engine. */
 int cmd_decrypt_mixed_device(cmd_engine *eng, const cmd_key *const *keys,
                              size_t nkeys, const uint32_t *h_key_idx,
                              const uint8_t *d_cts, const uint64_t *h_ct_off,
